@@ -35,8 +35,11 @@ struct fs_handle {
   bool dirty = true;
   // compat
   fsd::CompatDev cd{};
-  uint32_t *mt_state = nullptr, *mt_pos = nullptr, *draws = nullptr;
-  uint64_t draws_cap = 0;
+  uint32_t *mt_state = nullptr, *mt_pos = nullptr, *draws = nullptr;  // draws: a ring
+  unsigned int *cbar = nullptr;  // grid barrier of k_compat
+  std::vector<uint32_t> tile_post;
+  uint32_t *dtile_post = nullptr, cblocks = 0;
+  uint32_t gpar = 0;             // parity of the group gates' next buffer (kept across resets, like the gates)
   uint32_t *drawoff = nullptr, *injoff = nullptr;
   uint32_t jcong = 0;
   // batch buffers
@@ -193,6 +196,55 @@ int upload_params(fs_handle *h) {
   return FS_OK;
 }
 
+// Tiles of k_compat: posts cut where their synaptic items (plus a constant for
+// the neuron's own step) balance, one tile per resident block while tiles of
+// 4 to kCompatTile posts allow it, else a whole number per block.
+int compat_tiles(fs_handle *h, const fs_net_desc *d) {
+  const uint32_t n = h->n, W = fsd::kCompatTile;
+  uint32_t res = 0;
+  CK(fsd::compat_blocks(h->sm_count, &res));
+  uint32_t T = std::min(res, (n + 3) / 4);
+  if ((uint64_t)T * W < n) T = ((n + W - 1) / W + res - 1) / res * res;
+  std::vector<double> cost(n + 1, 0.0);
+  for (uint32_t i = 0; i < n; i++) {
+    double c = 32.0;
+    for (int r = 0; r < FS_NREC; r++) {
+      const fs_rec_layout &L = d->compat->rec[r];
+      if (h->cd.R[r].grow) c += (double)(L.gather_rowptr[i + 1] - L.gather_rowptr[i]);
+      if (h->cd.R[r].rrow) c += (r == FS_NMDA ? 1.5 : 1.0) * (double)(L.rec_rowptr[i + 1] - L.rec_rowptr[i]);
+    }
+    cost[i + 1] = cost[i] + c;
+  }
+  std::vector<uint32_t> &cut = h->tile_post;
+  cut.assign(T + 1, n);
+  cut[0] = 0;
+  for (uint32_t b = 1; b < T; b++) {
+    uint32_t c = (uint32_t)(std::lower_bound(cost.begin(), cost.end(), cost[n] * b / T) - cost.begin());
+    c = std::min(std::max(c, cut[b - 1] + 1), cut[b - 1] + W);
+    if ((uint64_t)W * (T - b) < n) c = std::max(c, n - W * (T - b));
+    cut[b] = std::min(c, n - (T - b));
+  }
+  int rc = upload(h, &h->dtile_post, cut.data(), cut.size());
+  if (rc) return rc;
+  h->cblocks = std::min(res, T);
+  // a record's post, counted from its tile's first
+  std::vector<uint8_t> in_tile(n), loc;
+  for (uint32_t t = 0; t < T; t++)
+    for (uint32_t i = cut[t]; i < cut[t + 1]; i++) in_tile[i] = (uint8_t)(i - cut[t]);
+  for (int r = 0; r < FS_NREC; r++) {
+    const fs_rec_layout &L = d->compat->rec[r];
+    fsd::RecDev &R = h->cd.R[r];
+    R.rloc = nullptr;
+    if (!R.rrow) continue;
+    loc.assign(L.n_recs, 0);
+    for (uint32_t i = 0; i < n; i++)
+      std::fill(loc.begin() + L.rec_rowptr[i], loc.begin() + L.rec_rowptr[i + 1], in_tile[i]);
+    if ((rc = upload(h, (uint8_t **)&R.rloc, loc.data(), loc.size()))) return rc;
+  }
+  CK(cudaStreamSynchronize(h->st));
+  return FS_OK;
+}
+
 int create_compat(fs_handle *h, const fs_net_desc *d) {
   const fs_neurons &v = d->neurons;
   const uint32_t n = v.n;
@@ -233,7 +285,7 @@ int create_compat(fs_handle *h, const fs_net_desc *d) {
     if ((rc = upload(h, (uint32_t **)&R.gate_pre, L.gate_pre, L.n_gates)) ||
         (rc = upload(h, (uint32_t **)&R.gate_post0, L.gate_post0, L.n_gates)) ||
         (rc = upload(h, (float **)&R.gate_g, L.gate_g, L.n_gates)) ||
-        (rc = zeros(h, &R.gate_st, L.n_gates)) || (rc = zeros(h, &R.gate_xt, L.n_gates)))
+        (rc = zeros(h, &R.gate_st, (size_t)2 * L.n_gates)) || (rc = zeros(h, &R.gate_xt, L.n_gates)))
       return rc;
     R.grow = nullptr;
     R.ggate = nullptr;
@@ -250,14 +302,16 @@ int create_compat(fs_handle *h, const fs_net_desc *d) {
     for (uint32_t k = 0; k < L.n_gates; k++)
       if (L.gate_pre[k] >= n || L.gate_post0[k] >= n) return set_err(h, FS_ERR_ARG, "gate neuron index out of range");
     R.rrow = nullptr;
+    R.rloc = nullptr;
     if ((rc = upload(h, (uint32_t **)&R.rpre, L.rec_pre, L.n_recs)) ||
         (rc = upload(h, (uint32_t **)&R.rpost, L.rec_post, L.n_recs)) ||
         (rc = upload(h, &R.rg, L.rec_g, L.n_recs)) || (rc = zeros(h, &R.rst, L.n_recs)) ||
         (rc = zeros(h, &R.rxt, L.n_recs)))
       return rc;
     if (L.n_recs) {
-      if (!L.rec_rowptr || L.rec_rowptr[n] != L.n_recs)
-        return set_err(h, FS_ERR_ARG, "rec_rowptr missing or inconsistent");
+      bool ok = L.rec_rowptr && L.rec_rowptr[n] == L.n_recs;
+      for (uint32_t i = 0; ok && i < n; i++) ok = L.rec_rowptr[i] <= L.rec_rowptr[i + 1];
+      if (!ok) return set_err(h, FS_ERR_ARG, "rec_rowptr missing or inconsistent");
       if ((rc = upload(h, (uint32_t **)&R.rrow, L.rec_rowptr, (size_t)n + 1))) return rc;
       for (uint32_t e = 0; e < L.n_recs; e++)
         if (L.rec_pre[e] >= n || L.rec_post[e] >= n) return set_err(h, FS_ERR_ARG, "record neuron index out of range");
@@ -275,10 +329,44 @@ int create_compat(fs_handle *h, const fs_net_desc *d) {
         (rc = upload(h, (float **)&c.gap_g, d->compat->gap_g, ne)))
       return rc;
   }
+  if ((rc = compat_tiles(h, d))) return rc;
+  // gates by presynaptic neuron, and the by-parity copies
+  std::vector<uint32_t> grow(n + 1, 0);
+  for (int r = 0; r < FS_NREC; r++)
+    for (uint32_t k = 0; k < c.R[r].n_gates; k++) grow[d->compat->rec[r].gate_pre[k] + 1]++;
+  for (uint32_t i = 0; i < n; i++) grow[i + 1] += grow[i];
+  std::vector<uint32_t> gent(grow[n]);
+  c.gby_row = c.gby_ent = nullptr;
+  if (grow[n]) {
+    std::vector<uint32_t> fill(grow.begin(), grow.end() - 1);
+    for (int r = 0; r < FS_NREC; r++)
+      for (uint32_t k = 0; k < c.R[r].n_gates; k++) gent[fill[d->compat->rec[r].gate_pre[k]]++] = c.gate_off[r] + k;
+    if ((rc = upload(h, (uint32_t **)&c.gby_row, grow.data(), grow.size())) ||
+        (rc = upload(h, (uint32_t **)&c.gby_ent, gent.data(), gent.size())))
+      return rc;
+  }
+  c.LP2 = c.V2 = c.inc2 = nullptr;
+  if (((c.glob & FS_ACT_LTP) && (rc = zeros(h, &c.LP2, (size_t)2 * n))) ||
+      (c.gap_row && (rc = zeros(h, &c.V2, (size_t)2 * n))) ||
+      ((c.glob & (FS_ACT_STP | FS_ACT_STD)) && (rc = zeros(h, &c.inc2, (size_t)2 * n))))
+    return rc;
+  if ((rc = zeros(h, &h->draws, fsd::draws_ring_words((size_t)FS_NREC * n))) || (rc = zeros(h, &h->cbar, 64))) return rc;
   // random streams
   if ((rc = zeros(h, &h->drawoff, n)) || (rc = zeros(h, &h->injoff, n))) return rc;
   c.drawoff = h->drawoff;
   c.injoff = h->injoff;
+  {  // the tile's words (CP_*, CS_*)
+    const void *par[] = {c.act, c.Vrev, nullptr, nullptr, nullptr, nullptr, c.dfst, nullptr, nullptr, nullptr, nullptr,
+                         c.ext_g, nullptr, nullptr, nullptr, nullptr, c.pb, nullptr, nullptr, nullptr, nullptr,
+                         c.nmda_dfxt, c.nmda_efst, c.nmda_as, c.nmda_mg, c.gl, c.El, c.Cm, c.Vreset, c.df, c.ef,
+                         c.dVmax, c.Vth, c.RfPed, c.SpiDy, c.inj_mean, c.inj_std, c.drawoff, c.injoff, c.ltp_dfLP,
+                         c.ltp_SpiLPDy};
+    const void *st[] = {c.V, c.Count, c.NS, c.Isyn, c.G, nullptr, nullptr, nullptr, nullptr, c.ext_st, nullptr, nullptr,
+                        nullptr, c.ext_xt_n, c.ext_st_n, c.Irep, nullptr, nullptr, nullptr, nullptr, c.LP, c.CountLP};
+    static_assert(sizeof par / sizeof *par == fsd::CP_N && sizeof st / sizeof *st == fsd::CS_N, "tile words");
+    for (int k = 0; k < fsd::CP_N; k++) c.npar[k] = par[k] ? (const uint32_t *)par[k] : c.npar[k - 1] + n;
+    for (int k = 0; k < fsd::CS_N; k++) c.nst[k] = st[k] ? (uint32_t *)st[k] : c.nst[k - 1] + n;
+  }
   if ((rc = zeros(h, &h->mt_state, 624)) || (rc = zeros(h, &h->mt_pos, 1))) return rc;
   // exception tables
   std::vector<uint32_t> ek, lk;
@@ -286,13 +374,20 @@ int create_compat(fs_handle *h, const fs_net_desc *d) {
   const std::string dir = lib_dir();
   if (!fsh::read_table(dir + "/expf_glibc.bin", ek, ev) || !fsh::read_table(dir + "/logf_glibc.bin", lk, lv))
     return set_err(h, FS_ERR_IO, "missing " + dir + "/expf_glibc.bin or logf_glibc.bin (run the build)");
-  if ((rc = upload(h, (uint32_t **)&c.expf_keys, ek.data(), ek.size())) ||
-      (rc = upload(h, (float **)&c.expf_vals, ev.data(), ev.size())) ||
-      (rc = upload(h, (uint32_t **)&c.logf_keys, lk.data(), lk.size())) ||
-      (rc = upload(h, (float **)&c.logf_vals, lv.data(), lv.size())))
-    return rc;
-  c.expf_n = (uint32_t)ek.size();
-  c.logf_n = (uint32_t)lk.size();
+  {
+    uint32_t *dk = nullptr;
+    float *dv = nullptr;
+    for (int f = 0; f < 2; f++) {
+      const std::vector<uint32_t> &keys = f ? lk : ek;
+      const std::vector<float> &vals = f ? lv : ev;
+      uint4 *tab = nullptr;
+      if ((rc = upload(h, &dk, keys.data(), keys.size())) || (rc = upload(h, &dv, vals.data(), vals.size())) ||
+          (rc = dalloc(h, &tab, fsd::kHashBytes / sizeof(uint4))))
+        return rc;
+      CK(fsd::hash_fill(dk, dv, (uint32_t)keys.size(), tab, h->st));
+      (f ? c.logf_tab : c.expf_tab) = tab;
+    }
+  }
   uint32_t kn[128], ja[32], jc[32];
   float fn[128], wn[128];
   host_tables(kn, fn, wn, ja, jc);
@@ -309,15 +404,6 @@ int compat_batch(fs_handle *h, uint32_t nsteps, fs_step_out *out, uint64_t *writ
   const uint32_t n = h->n, words = (n + 31) / 32;
   int rc;
   if ((rc = ensure_batch(h, nsteps))) return rc;
-  // draw buffer
-  const uint64_t need = (uint64_t)nsteps * c.draws_per_step;
-  if (need > h->draws_cap) {
-    if ((rc = dalloc(h, &h->draws, (size_t)need))) return rc;
-    h->draws_cap = need;
-  }
-  CK(fsd::mt_generate(h->mt_state, h->mt_pos, h->draws, need, h->st));
-  h->launches += need ? 1 : 0;
-  c.draws = h->draws;
   c.jcong_base = h->jcong;
   c.spikebits = h->spikebits;
   c.words = words;
@@ -353,7 +439,10 @@ int compat_batch(fs_handle *h, uint32_t nsteps, fs_step_out *out, uint64_t *writ
     c.gv_st = h->gv_st;
     c.gv_xt = h->gv_xt;
   }
-  for (uint32_t s = 0; s < nsteps; s++) CK(fsd::compat_step(c, s, h->sm_count, h->st, &h->launches));
+  CK(fsd::compat_steps(c, fsd::CompatRun{nsteps, h->gpar, h->cblocks, (uint32_t)h->tile_post.size() - 1, h->dtile_post,
+                                          h->mt_state, h->mt_pos, h->draws, 0, h->cbar},
+                       h->st, &h->launches));
+  h->gpar = (h->gpar + nsteps) & 1u;
   CK(fsd::spikes_compact(h->spikebits, nsteps, words, h->counts, h->offsets, h->idx, h->st, &h->launches));
   h->jcong = jcong_advance(h->jcong, (uint64_t)nsteps * c.inj_per_step);
   uint32_t total = 0;
@@ -363,6 +452,7 @@ int compat_batch(fs_handle *h, uint32_t nsteps, fs_step_out *out, uint64_t *writ
   CK(cudaStreamSynchronize(h->st));
   int derr = 0;
   CK(cudaMemcpy(&derr, h->derr, 4, cudaMemcpyDeviceToHost));
+  if (derr & 2) return set_err(h, FS_ERR_TIMEOUT, "grid barrier wait gave up (device error word set)");
   if (derr) return set_err(h, FS_ERR_TIMEOUT, "ziggurat rejection loop exceeded its bound");
   h->spikes_total += total;
   if (out && out->spike_idx) {
@@ -384,13 +474,9 @@ int compat_batch(fs_handle *h, uint32_t nsteps, fs_step_out *out, uint64_t *writ
   return FS_OK;
 }
 
-// steps per batch for compat: bounded by the draw buffer (<= 256 MB) and the
-// spike buffers
+// steps per batch for compat: bounded by the spike buffers
 uint32_t compat_batch_steps(fs_handle *h, uint32_t left) {
-  uint64_t lim = h->chunk;
-  const uint64_t D = std::max<uint32_t>(1, h->cd.draws_per_step);
-  lim = std::min<uint64_t>(lim, std::max<uint64_t>(1, (64ull << 20) / D));
-  lim = std::min<uint64_t>(lim, std::max<uint64_t>(1, (64ull << 20) / std::max<uint32_t>(1, h->n)));
+  const uint64_t lim = std::min<uint64_t>(h->chunk, std::max<uint64_t>(1, (64ull << 20) / std::max<uint32_t>(1, h->n)));
   return (uint32_t)std::min<uint64_t>(lim, left);
 }
 
@@ -882,11 +968,13 @@ int fs_debug_expf(const float *x, float *y, uint64_t k) {
   struct Bufs {
     float *dx = nullptr, *dy = nullptr, *dv = nullptr;
     uint32_t *dk = nullptr;
+    uint4 *tab = nullptr;
     ~Bufs() {
       if (dx) cudaFree(dx);
       if (dy) cudaFree(dy);
       if (dk) cudaFree(dk);
       if (dv) cudaFree(dv);
+      if (tab) cudaFree(tab);
     }
   } b;
   fs_handle tmp;
@@ -895,10 +983,12 @@ int fs_debug_expf(const float *x, float *y, uint64_t k) {
   CK(cudaMalloc(&b.dy, k * 4));
   CK(cudaMalloc(&b.dk, ek.size() * 4));
   CK(cudaMalloc(&b.dv, ev.size() * 4));
+  CK(cudaMalloc(&b.tab, fsd::kHashBytes));
   CK(cudaMemcpy(b.dx, x, k * 4, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(b.dk, ek.data(), ek.size() * 4, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(b.dv, ev.data(), ev.size() * 4, cudaMemcpyHostToDevice));
-  CK(fsd::expf_ref_eval(b.dx, b.dy, k, b.dk, b.dv, (uint32_t)ek.size(), nullptr));
+  CK(fsd::hash_fill(b.dk, b.dv, (uint32_t)ek.size(), b.tab, nullptr));
+  CK(fsd::expf_ref_eval(b.dx, b.dy, k, b.dk, b.dv, (uint32_t)ek.size(), b.tab, nullptr));
   CK(cudaMemcpy(y, b.dy, k * 4, cudaMemcpyDeviceToHost));
   return FS_OK;
 }
@@ -980,7 +1070,7 @@ extern "C" int fs_debug_expf_noalloc(const float *x, float *y, uint64_t k) {
   float *dy = dx + kNaMaxK;
   cudaStream_t st = cudaStreamPerThread;
   CK(cudaMemcpyAsync(dx, x, k * 4, cudaMemcpyHostToDevice, st));
-  CK(fsd::expf_ref_eval(dx, dy, k, dk, dv, s.nk, st));
+  CK(fsd::expf_ref_eval(dx, dy, k, dk, dv, s.nk, nullptr, st));
   CK(cudaMemcpyAsync(y, dy, k * 4, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
   return FS_OK;
