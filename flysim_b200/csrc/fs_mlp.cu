@@ -14,10 +14,10 @@
 // (tcgen05.ld 32x32b) for a fused epilogue: bias, ReLU, the ReLU mask of the
 // backward pass, FP32 / BF16 / transposed-BF16 outputs.
 //
-// Training: one Adam step over a batch of 256 rows is 4 forward GEMMs, the
-// loss kernel, 4 weight-gradient and 3 input-gradient GEMMs, bias sums and
-// the Adam updates; the step is captured once into a CUDA graph (batch
-// index and Adam step count live in device counters) and replayed.
+// Training: an epoch is one persistent launch, k_train (networks of up to
+// about nine layers of 256); deeper networks replay a CUDA graph of one Adam
+// step (forward GEMMs, loss, gradient GEMMs, bias sums, Adam updates; batch
+// index and Adam step count live in device counters).
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -30,6 +30,7 @@
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include "flysim_b200.h"
+#include "fs_barrier.cuh"
 
 namespace fsm {
 
@@ -94,6 +95,13 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
       : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
         "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
       : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+}
+
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(taddr));
   asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 }
 
@@ -532,6 +540,20 @@ __global__ void k_stage_t(const float *t, int rows, int cols, int pcols, const i
   T[i] = c < cols ? t[src * cols + c] : 0.0f;
 }
 
+// One output's loss and gradient: column c of nr regressions and a logit.
+__device__ __forceinline__ void loss_element(float y, float t, int c, int nr, int rows, float &l, float &d) {
+  l = d = 0.0f;
+  if (c < nr) {
+    const float e = y - t;
+    d = 2.0f * e / (float)(nr * rows);
+    l = e * e / (float)(nr * rows);
+  } else if (c == nr) {
+    const float p = 1.0f / (1.0f + expf(-y));
+    d = (p - t) / (float)rows;
+    l = (fmaxf(y, 0.0f) - y * t + log1pf(expf(-fabsf(y)))) / (float)rows;
+  }
+}
+
 // Loss and output-layer gradient.  Columns [0, nr) regress log-rates (mean
 // squared error averaged over nr columns and the rows), column nr is the
 // hyperactivity logit (binary cross-entropy averaged over the rows); padded
@@ -542,17 +564,8 @@ __global__ void k_loss(const float *Z, const float *T, int rows, int pcols, int 
   float l = 0.0f;
   if (i < rows * pcols) {
     const int r = i / pcols, c = i - r * pcols;
-    const float y = Z[i], t = T[i];
-    float d = 0.0f;
-    if (c < nr) {
-      const float e = y - t;
-      d = 2.0f * e / (float)(nr * rows);
-      l = e * e / (float)(nr * rows);
-    } else if (c == nr) {
-      const float p = 1.0f / (1.0f + expf(-y));
-      d = (p - t) / (float)rows;
-      l = (fmaxf(y, 0.0f) - y * t + log1pf(expf(-fabsf(y)))) / (float)rows;
-    }
+    float d;
+    loss_element(Z[i], T[i], c, nr, rows, l, d);
     const bf16 b = __float2bfloat16_rn(d);
     dZ[i] = b;
     dZT[(size_t)c * ldt + r] = b;
@@ -571,21 +584,32 @@ __global__ void k_bias_grad(const bf16 *dZT, int ldt, int rows, int n, float *gb
   if (lane == 0) gb[c] = s;
 }
 
+// One weight's Adam update; c1, c2: the bias corrections of this step.
+__device__ __forceinline__ void adam_update(float &w, float &m, float &v, float gi, float lr, float c1, float c2) {
+  const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+  m = __fmaf_rn(1.0f - b1, gi, __fmul_rn(b1, m));  // one contraction in every kernel
+  v = __fmaf_rn(__fmul_rn(1.0f - b2, gi), gi, __fmul_rn(b2, v));
+  // (a weight that never had a gradient: the step is exactly 0, and its
+  // zero operands would take the divisions' slow path)
+  if (m != 0.0f || v != 0.0f) w = w - lr * (m / c1) / (sqrtf(v / c2) + eps);
+}
+__device__ __forceinline__ void adam_corrections(int step, float &c1, float &c2) {
+  const float t = (float)(step + 1);
+  c1 = 1.0f - powf(0.9f, t);
+  c2 = 1.0f - powf(0.999f, t);
+}
+
 // Adam on the FP32 master copy (step count from the device counter), then the
 // BF16 copies W and W^T.
 __global__ void k_adam(float *w, float *m, float *v, const float *g, int n, int rows, int cols, float lr,
                        const int *ctr, bf16 *Wb, bf16 *Wt) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-  const float t = (float)(ctr[1] + 1);
-  const float c1 = 1.0f - powf(b1, t), c2 = 1.0f - powf(b2, t);
-  const float gi = g[i];
-  const float mi = b1 * m[i] + (1.0f - b1) * gi;
-  const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
+  float c1, c2, wi = w[i], mi = m[i], vi = v[i];
+  adam_corrections(ctr[1], c1, c2);
+  adam_update(wi, mi, vi, g[i], lr, c1, c2);
   m[i] = mi;
   v[i] = vi;
-  const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
   w[i] = wi;
   if (Wb) {
     const bf16 b = __float2bfloat16_rn(wi);
@@ -609,9 +633,488 @@ __global__ void k_refresh(const float *w, int rows, int cols, bf16 *Wb, bf16 *Wt
   Wt[(size_t)c * rows + r] = b;
 }
 
+// ---- persistent training kernel ----------------------------------------------
+// One launch runs an epoch's Adam steps over batches of kBatch = 256 rows.  The
+// network's row dependencies decide the split: given the weights, forward and
+// backward of a row need no other row, so kRowCtas CTAs take kRowsCta = 16 rows
+// each through all layers with no exchange; only the weight gradients sum over
+// rows, and a CTA per 128 x 16 tile of a layer's weights forms its sum, keeps
+// the tile's weights and Adam moments in registers for the launch and updates
+// them.  Two grid barriers a step.
+//
+// Row CTAs: D[features x rows] = W . H^T, so an epilogue thread owns a feature
+// with its 16 rows; it writes the next layer's operand to shared memory and the
+// transposed activations the gradient tiles read with two coalesced 16-byte
+// stores.  The weights (0.6 MB a step, more than shared memory) stream from L2
+// through a ring of 16 KB chunks (two to a slot), contiguous in the blocked layout the tile
+// CTAs write: [128 rows x 64 k] as eight boxes of 128 rows x 16 bytes, the
+// no-swizzle K-major core-matrix order.  Every accumulator sums the same
+// products over K in the same order as k_gemm_tn.
+//
+// The step this replaces was 28 graph nodes, each a launch of a few CTAs: 146 us
+// for about 1 us of tensor work; now 22.6 us (surrogate, 32-256-256-256-59).
+// What bounds it is the chain of small products (seven of them, each waits for
+// its operand, its accumulator and its epilogue), the tile update (about 9,000
+// cycles: load, product, Adam with its IEEE divisions, publication) and the
+// two barriers (2,000 each).
+constexpr int kBatch = 256;     // training rows per step
+constexpr int kRowsCta = 16, kRowCtas = kBatch / kRowsCta;
+constexpr int kMaxTrainL = 24;
+constexpr int kTrThreads = 320;  // warps 0-7 epilogues, 8 copies, 9 MMAs
+constexpr int kRing = 4;         // slots of two 16 KB chunks (a K chunk of up to two row tiles)
+constexpr uint32_t kChunkB = 16384;
+// Bytes between the 8-wide K boxes of a row CTA's operand ([K/8][16 rows][8] and
+// 16 bytes of padding, so that the lanes of a feature store hit four times the
+// banks)
+constexpr uint32_t kHsBox = kRowsCta * 16 + 16;
+constexpr int kTileN = 16;       // weight columns of a tile CTA
+
+struct TrainLayer {
+  int in, out;           // padded widths
+  bf16 *Wk, *Wt;         // blocked W [out x in] and W^T [in x out]
+  bf16 *HT;              // the layer's input, transposed: [in/kTileN][row/8][kTileN][8]
+  bf16 *dZT;             // its output gradient, transposed: [out/128][row/8][128][8]
+  float *W, *mW, *vW, *b, *mb, *vb;
+};
+struct TrainArgs {
+  TrainLayer l[kMaxTrainL];
+  int L, steps, din, dout, tiles;
+  const float *x, *t;
+  const int *perm;
+  const uint32_t *tile;  // layer | out tile << 8 | in tile << 16
+  float lr;
+  float *loss;
+  int *ctr;
+  unsigned int *bar;
+  int *err;
+};
+
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count));
+}
+__device__ __forceinline__ void mbar_expect(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst),
+               "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
+  return p != 0;
+}
+__device__ __forceinline__ void mma_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async;\n" ::: "memory"); }
+__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
+__device__ __forceinline__ uint32_t bf2(float a, float b) {
+  const __nv_bfloat162 v = __halves2bfloat162(__float2bfloat16_rn(a), __float2bfloat16_rn(b));
+  return *(const uint32_t *)&v;
+}
+
+// barriers in shared memory
+struct TrainBars {
+  uint64_t full[kRing], empty[kRing], done;
+  uint32_t tmem;
+  int src[2][kRowsCta];
+  int fail;
+};
+
+// The products of one step of a row CTA: forward layers, then backward ones.
+template <class F>
+__device__ __forceinline__ void for_stages(const TrainArgs &g, F &&f) {
+  for (int l = 0; l < g.L; l++) f(l, false, g.l[l].Wk, g.l[l].out, g.l[l].in);
+  for (int l = g.L - 1; l > 0; l--) f(l, true, g.l[l].Wt, g.l[l].in, g.l[l].out);
+}
+
+// Sixteen rows through the network (CTAs [0, kRowCtas)).
+__device__ __forceinline__ void train_rows(const TrainArgs &g, uint8_t *smem, TrainBars &B) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int row0 = (int)blockIdx.x * kRowsCta, L = g.L;
+  bf16 *Hs = (bf16 *)(smem + kRing * 2 * kChunkB);  // operand, K-major boxes kHsBox apart
+  const uint32_t hs = smem_u32(Hs), tmem = B.tmem, done = smem_u32(&B.done);
+  unsigned long long target = 0;
+  uint32_t slot = 0, ph = 0;  // copies and MMAs: chunk slot and its round's parity
+  uint32_t dph = 0;           // parity of `done`
+  bool ok = true;
+  const int p0 = g.l[0].in;
+  // rows of step s and their inputs into the operand buffer
+  auto rows_of = [&](int s) {
+    if (tid < kRowsCta) B.src[s & 1][tid] = __ldg(g.perm + (size_t)s * kBatch + row0 + tid);
+  };
+  auto stage_x = [&](int s) {
+    for (int e = tid; e < kRowsCta * p0; e += 256) {
+      const int r = e / p0, c = e - r * p0;
+      const float v = c < g.din ? __ldg(g.x + (size_t)B.src[s & 1][r] * g.din + c) : 0.0f;
+      Hs[(c >> 3) * (kHsBox / 2) + r * 8 + (c & 7)] = __float2bfloat16_rn(v);
+    }
+  };
+  rows_of(0);
+  __syncthreads();
+  if (tid < 256) stage_x(0);
+  if (!fsd::grid_sync(g.bar, g.err, gridDim.x, target)) return;
+  for (int s = 0; s < g.steps; s++) {
+    if (warp == 8) {
+      if (lane == 0) {
+        fence_async();  // the tiles' weights, written before the barrier
+        for_stages(g, [&](int, bool, const bf16 *W, int M, int K) {
+          const uint8_t *src = (const uint8_t *)W;
+          const uint32_t second = M > 128 ? (uint32_t)((K + 63) / 64) * kChunkB : 0u;  // the second row tile's chunks
+          for (int k0 = 0; k0 < K && ok; k0 += 64, src += kChunkB) {
+            const uint32_t bytes = (uint32_t)min(64, K - k0) * 256u, full = smem_u32(&B.full[slot]);
+            const uint32_t dst = smem_u32(smem) + slot * 2 * kChunkB;
+            ok = mbar_wait(smem_u32(&B.empty[slot]), ph ^ 1u);
+            if (!ok) break;
+            mbar_expect(full, second ? 2 * bytes : bytes);
+            bulk_load(dst, src, bytes, full);
+            if (second) bulk_load(dst + kChunkB, src + second, bytes, full);
+            if (++slot == kRing) slot = 0, ph ^= 1u;
+          }
+        });
+      }
+    } else if (warp == 9) {
+      // (the whole warp runs the loops, one elected lane issues: a product's
+      // MMAs follow each other at 41 cycles, 32 of them W's reads from shared
+      // memory, and at 75-80 from a branch that only one lane enters)
+      const uint64_t ra = sdesc(smem_u32(smem), 2048, 128), rb = sdesc(hs, kHsBox, 128);
+      constexpr uint32_t kB = 2 * kHsBox >> 4;  // descriptors advance by adding to the address field
+      const uint32_t id = idesc_bf16(128, kRowsCta);
+      for_stages(g, [&](int, bool, const bf16 *, int M, int K) {
+        asm volatile("bar.sync 2, 288;\n" ::: "memory");  // the operand is in shared memory
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        for (int k0 = 0; k0 < K && ok; k0 += 64) {
+          ok = mbar_wait(smem_u32(&B.full[slot]), ph);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+          const uint64_t a0 = ra + slot * (2 * kChunkB >> 4), a1 = a0 + (kChunkB >> 4);
+          const uint64_t b = rb + (uint32_t)(k0 >> 4) * kB;
+          const uint32_t acc = k0 > 0 ? 1u : 0u;
+          if (elect_one()) {
+            if (K - k0 >= 64 && M > 128) {
+#pragma unroll
+              for (int k = 0; k < 4; k++) {
+                mma_bf16(tmem, a0 + k * 256, b + k * kB, id, k ? 1u : acc);
+                mma_bf16(tmem + kRowsCta, a1 + k * 256, b + k * kB, id, k ? 1u : acc);
+              }
+            } else if (K - k0 >= 64) {
+#pragma unroll
+              for (int k = 0; k < 4; k++) mma_bf16(tmem, a0 + k * 256, b + k * kB, id, k ? 1u : acc);
+            } else {
+              for (int k = 0; k < (K - k0) >> 4; k++) {
+                mma_bf16(tmem, a0 + k * 256, b + k * kB, id, k ? 1u : acc);
+                if (M > 128) mma_bf16(tmem + kRowsCta, a1 + k * 256, b + k * kB, id, k ? 1u : acc);
+              }
+            }
+            mma_commit(smem_u32(&B.empty[slot]));
+            if (k0 + 64 >= K) mma_commit(done);
+          }
+          __syncwarp();
+          if (++slot == kRing) slot = 0, ph ^= 1u;
+        }
+      });
+    } else {
+      const int f = (warp & 3) * 32 + lane + (warp >> 2) * 128;  // the thread's feature
+      const int last = g.l[L - 1].out;
+      fence_async_smem();
+      asm volatile("bar.sync 2, 288;\n" ::: "memory");
+      // while the first layer runs: the targets of output feature f, and the
+      // input, transposed, for its layer's gradient
+      // (eight rows of feature f & 127 where the output layer has one row tile)
+      const bool split = last <= 128;
+      const int ft = split ? f & 127 : f, rt = split ? (warp >> 2) * 8 : 0;
+      float tt[kRowsCta];
+#pragma unroll
+      for (int r = 0; r < kRowsCta; r++)
+        tt[r] = ft < g.dout && (r < 8 || !split) ? __ldg(g.t + (size_t)B.src[s & 1][rt + r] * g.dout + ft) : 0.0f;
+      if (tid < p0) {
+        uint32_t v[8];
+#pragma unroll
+        for (int r = 0; r < kRowsCta; r += 2)
+          v[r >> 1] = (uint32_t) * (const uint16_t *)(Hs + (tid >> 3) * (kHsBox / 2) + r * 8 + (tid & 7)) |
+                      (uint32_t) * (const uint16_t *)(Hs + (tid >> 3) * (kHsBox / 2) + (r + 1) * 8 + (tid & 7)) << 16;
+        uint4 *dst = (uint4 *)(g.l[0].HT + (size_t)(tid / kTileN) * (kTileN * kBatch) +
+                               (size_t)(row0 >> 3) * (kTileN * 8) + (tid % kTileN) * 8);
+        dst[0] = make_uint4(v[0], v[1], v[2], v[3]);
+        dst[kTileN] = make_uint4(v[4], v[5], v[6], v[7]);
+      }
+      asm volatile("bar.sync 3, 256;\n" ::: "memory");  // Hs is read before the next operand goes there
+      float lsum = 0.0f;
+      for_stages(g, [&](int l, bool back, const bf16 *, int M, int) {
+        const TrainLayer &Y = g.l[l];
+        const float bias = !back && f < M ? __ldcg(Y.b + f) : 0.0f;
+        // backward: the input of layer l, whose sign is the ReLU's mask
+        uint4 h0 = make_uint4(0, 0, 0, 0), h1 = h0;
+        if (back && f < M) {
+          const uint4 *src = (const uint4 *)(Y.HT + (size_t)(f / kTileN) * (kTileN * kBatch) +
+                                             (size_t)(row0 >> 3) * (kTileN * 8) + (f % kTileN) * 8);
+          h0 = __ldcg(src);
+          h1 = __ldcg(src + kTileN);
+        }
+        ok = mbar_wait(done, dph) && ok;
+        dph ^= 1u;
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        if (!back && l + 1 == L && M <= 128) {
+          // the output layer fills four warps' accumulator lanes: warps w and
+          // w + 4 take eight rows each of the loss and its gradient
+          const int fo = (warp & 3) * 32 + lane, h8 = warp >> 2;
+          uint32_t a[8], v[4];
+          tmem_ld8(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(h8 * 8), a);
+          asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+          const float bo = fo < M ? __ldcg(Y.b + fo) : 0.0f;
+          float x[8];
+#pragma unroll
+          for (int r = 0; r < 8; r++) {
+            float lo;
+            loss_element(__uint_as_float(a[r]) + bo, tt[r], fo, g.dout - 1, kBatch, lo, x[r]);
+            lsum += lo;
+          }
+#pragma unroll
+          for (int r = 0; r < 8; r += 2) v[r >> 1] = bf2(x[r], x[r + 1]);
+          if (fo < M && L > 1) {
+            uint16_t *h = (uint16_t *)(Hs + (fo >> 3) * (kHsBox / 2) + (fo & 7) + h8 * 64);
+#pragma unroll
+            for (int r = 0; r < 8; r++) h[r * 8] = (uint16_t)(v[r >> 1] >> (16 * (r & 1)));
+          }
+          fence_async_smem();
+          if (L > 1) asm volatile("bar.sync 2, 288;\n" ::: "memory");
+          if (fo < M)
+            *(uint4 *)(Y.dZT + (size_t)((row0 >> 3) + h8) * 1024 + (size_t)fo * 8) = make_uint4(v[0], v[1], v[2], v[3]);
+          return;
+        }
+        uint32_t v[8];
+        if ((f & ~127) < M) {  // (whole warps)
+          uint32_t a[16];
+          tmem_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)((warp >> 2) * kRowsCta), a);
+          asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+          float x[kRowsCta];
+          const bf16 *m0 = (const bf16 *)&h0, *m1 = (const bf16 *)&h1;
+#pragma unroll
+          for (int r = 0; r < kRowsCta; r++) x[r] = __uint_as_float(a[r]);
+          if (back) {
+#pragma unroll
+            for (int r = 0; r < kRowsCta; r++)
+              if (!(__bfloat162float(r < 8 ? m0[r & 7] : m1[r & 7]) > 0.0f)) x[r] = 0.0f;
+          } else if (l + 1 < L) {
+#pragma unroll
+            for (int r = 0; r < kRowsCta; r++) x[r] = fmaxf(x[r] + bias, 0.0f);
+          } else {
+#pragma unroll 4
+            for (int r = 0; r < kRowsCta; r++) {
+              float lo, d;
+              loss_element(x[r] + bias, tt[r], f, g.dout - 1, kBatch, lo, d);
+              lsum += lo;
+              x[r] = d;
+            }
+          }
+#pragma unroll
+          for (int r = 0; r < kRowsCta; r += 2) v[r >> 1] = bf2(x[r], x[r + 1]);
+          if (f < M && (!back || l > 1)) {  // the next stage's operand
+            uint16_t *h = (uint16_t *)(Hs + (f >> 3) * (kHsBox / 2) + (f & 7));
+#pragma unroll
+            for (int r = 0; r < kRowsCta; r++) h[r * 8] = (uint16_t)(v[r >> 1] >> (16 * (r & 1)));
+          }
+        }
+        fence_async_smem();
+        if (!(back && l == 1) && L > 1) asm volatile("bar.sync 2, 288;\n" ::: "memory");
+        // while the next stage runs: the next layer's input (forward), the
+        // gradients of the output and of each layer's input, for the tiles
+        if (f < M) {
+          const bool act = !back && l + 1 < L;
+          const int T = act ? kTileN : 128;
+          bf16 *base = act ? g.l[l + 1].HT : back ? g.l[l - 1].dZT : Y.dZT;
+          uint4 *dst = (uint4 *)(base + (size_t)(f / T) * (T * kBatch) + (size_t)(row0 >> 3) * (T * 8) +
+                                 (size_t)(f % T) * 8);
+          dst[0] = make_uint4(v[0], v[1], v[2], v[3]);
+          dst[T] = make_uint4(v[4], v[5], v[6], v[7]);
+        }
+      });
+      fence_async();  // the tiles read what was written above
+      if ((split ? warp & 3 : warp) * 32 < last) {
+        for (int o = 16; o; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+        if (lane == 0) atomicAdd(g.loss, lsum);
+      }
+    }
+    if (!ok) B.fail = 1;
+    if (!fsd::grid_sync(g.bar, g.err, gridDim.x, target)) return;  // activations and gradients are out
+    if (B.fail) {
+      if (tid == 0) atomicExch(g.err, 6);
+      return;
+    }
+    if (s + 1 < g.steps) {  // while the tiles update
+      rows_of(s + 1);
+      __syncthreads();
+      if (tid < 256) stage_x(s + 1);
+    }
+    if (!fsd::grid_sync(g.bar, g.err, gridDim.x, target)) return;  // the weights are updated
+  }
+}
+
+// One tile of a layer's weights (CTAs from kRowCtas on): rows [128 mt, ...) of
+// W [out x in], columns [kTileN nt, ...).
+__device__ __forceinline__ void train_tile(const TrainArgs &g, uint8_t *smem, TrainBars &B) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  constexpr int kC = kTileN / 2;  // columns of a thread
+  constexpr uint32_t kBc = kTileN * 128;  // bytes of H^T in a chunk of 64 rows
+  const uint32_t code = __ldg(g.tile + blockIdx.x - kRowCtas);
+  const TrainLayer &Y = g.l[code & 0xffu];
+  const int mt = (int)(code >> 8) & 0xff, nt = (int)(code >> 16), NT = (Y.in + kTileN - 1) / kTileN;
+  uint8_t *sA = smem, *sB = smem + 4 * kChunkB;        // dZ^T [32][128][8], H^T [32][kTileN][8]
+  bf16 *tr = (bf16 *)(smem + 5 * kChunkB);             // the tile's W^T [kTileN in][128 out]
+  const int o = mt * 128 + (warp & 3) * 32 + lane;     // the thread's weight row and kC columns
+  const int i0 = nt * kTileN + (warp >> 2) * kC;
+  const bool mine = tid < 256 && o < Y.out && i0 < Y.in;
+  // biases: the row tile's are dealt to its column tiles, in a tile to the
+  // warps; lane k of a warp has its k-th, row fb(k) of the row tile
+  auto fb = [&](int k) { return nt + NT * (warp + 8 * k); };
+  const int nb = tid < 256 ? max(0, (min(128, Y.out - mt * 128) - nt + NT * (8 - warp) - 1) / (NT * 8)) : 0;
+  const int ob = mt * 128 + fb(lane);
+  float w[kC], m[kC], v[kC], b = 0.0f, bm = 0.0f, bv = 0.0f;
+#pragma unroll
+  for (int k = 0; k < kC; k++) {
+    const size_t e = (size_t)o * Y.in + i0 + k;
+    w[k] = mine ? Y.W[e] : 0.0f;
+    m[k] = mine ? Y.mW[e] : 0.0f;
+    v[k] = mine ? Y.vW[e] : 0.0f;
+  }
+  if (lane < nb) b = Y.b[ob], bm = Y.mb[ob], bv = Y.vb[ob];
+  // the BF16 copies, blocked (see above); the transposed one through shared
+  // memory, eight rows of a column a thread
+  auto publish = [&]() {
+    if (tid < 256) {
+      uint32_t p[kC / 2];
+#pragma unroll
+      for (int k = 0; k < kC; k += 2) p[k >> 1] = bf2(w[k], w[k + 1]);
+      if (mine) {
+        const int kc = (Y.in + 63) / 64;
+        *(uint4 *)(Y.Wk + ((size_t)mt * kc + i0 / 64) * (kChunkB / 2) + (size_t)((i0 & 63) >> 3) * 1024 +
+                   (size_t)(o & 127) * 8) = make_uint4(p[0], p[1], p[2], p[3]);
+      }
+#pragma unroll
+      for (int k = 0; k < kC; k++)
+        ((uint16_t *)tr)[((warp >> 2) * kC + k) * 128 + (o & 127)] = (uint16_t)(p[k >> 1] >> (16 * (k & 1)));
+      asm volatile("bar.sync 3, 256;\n" ::: "memory");
+      for (int q = tid; q < kTileN * 16; q += 256) {
+        const int i = nt * kTileN + q % kTileN, oo = mt * 128 + q / kTileN * 8;
+        if (i < Y.in && oo < Y.out) {
+          const int kc = (Y.out + 63) / 64;
+          *(uint4 *)(Y.Wt + ((size_t)(i / 128) * kc + oo / 64) * (kChunkB / 2) + (size_t)((oo & 63) >> 3) * 1024 +
+                     (size_t)(i & 127) * 8) = *(const uint4 *)(tr + q % kTileN * 128 + q / kTileN * 8);
+        }
+      }
+      if (lane < nb) Y.b[ob] = b;
+      fence_async();
+    }
+  };
+  static_assert(kC == 8, "a thread's columns are one 16-byte store");
+  publish();
+  unsigned long long target = 0;
+  const int t0 = g.ctr[1];
+  bool ok = true;
+  if (!fsd::grid_sync(g.bar, g.err, gridDim.x, target)) return;
+  for (int s = 0; s < g.steps; s++) {
+    const uint32_t ph = (uint32_t)s & 1u;
+    if (!fsd::grid_sync(g.bar, g.err, gridDim.x, target)) return;  // the step's gradients are out
+    if (warp == 8) {
+      if (lane == 0) {
+        fence_async();
+        for (int c = 0; c < 4; c++) {
+          const uint32_t bar = smem_u32(&B.full[c]);
+          mbar_expect(bar, kChunkB + kBc);
+          bulk_load(smem_u32(sA + c * kChunkB), Y.dZT + (size_t)mt * (128 * kBatch) + (size_t)c * (kChunkB / 2), kChunkB,
+                    bar);
+          bulk_load(smem_u32(sB + c * kBc), (const uint8_t *)(Y.HT + (size_t)nt * (kTileN * kBatch)) + c * kBc, kBc,
+                    bar);
+        }
+      }
+    } else if (warp == 9) {
+      if (lane == 0) {
+        const uint64_t da = sdesc(smem_u32(sA), 2048, 128), db = sdesc(smem_u32(sB), kTileN * 16u, 128);
+        for (int c = 0; c < 4 && ok; c++) {
+          ok = mbar_wait(smem_u32(&B.full[c]), ph);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+#pragma unroll
+          for (int k = 0; k < 4; k++)
+            mma_bf16(B.tmem, da + (4 * c + k) * 256, db + (4 * c + k) * (kTileN * 2), idesc_bf16(128, kTileN),
+                     c + k > 0 ? 1u : 0u);
+        }
+        mma_commit(smem_u32(&B.done));
+      }
+    } else {
+      float c1, c2;
+      adam_corrections(t0 + s, c1, c2);
+      if (nb) {  // gradient of the biases: row sums of dZ^T, in k_bias_grad's order
+        for (int c = 0; c < 4; c++) ok = mbar_wait(smem_u32(&B.full[c]), ph) && ok;
+        float gb = 0.0f;
+        for (int k = 0; k < nb; k++) {
+          const bf16 *p = (const bf16 *)sA + fb(k) * 8 + (lane & 7);
+          float a = 0.0f;
+#pragma unroll
+          for (int j = 0; j < 8; j++) a += __bfloat162float(p[(size_t)((lane >> 3) + 4 * j) * 1024]);
+          for (int q = 16; q; q >>= 1) a += __shfl_xor_sync(0xffffffffu, a, q);
+          if (lane == k) gb = a;
+        }
+        if (lane < nb) adam_update(b, bm, bv, gb, g.lr, c1, c2);
+      }
+      ok = mbar_wait(smem_u32(&B.done), ph) && ok;
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      uint32_t a[kC];
+      tmem_ld8(B.tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)((warp >> 2) * kC), a);
+      asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+      if (mine)
+#pragma unroll
+        for (int k = 0; k < kC; k++) adam_update(w[k], m[k], v[k], __uint_as_float(a[k]), g.lr, c1, c2);
+      publish();
+    }
+    if (!ok) B.fail = 1;
+    if (!fsd::grid_sync(g.bar, g.err, gridDim.x, target)) return;
+    if (B.fail) {
+      if (tid == 0) atomicExch(g.err, 6);
+      return;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < kC; k++) {
+    const size_t e = (size_t)o * Y.in + i0 + k;
+    if (mine) Y.W[e] = w[k], Y.mW[e] = m[k], Y.vW[e] = v[k];
+  }
+  if (lane < nb) Y.mb[ob] = bm, Y.vb[ob] = bv;
+  if (blockIdx.x == kRowCtas && tid == 0) g.ctr[1] = t0 + g.steps;
+}
+
+__global__ void __launch_bounds__(kTrThreads, 1) k_train(const __grid_constant__ TrainArgs g) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  __shared__ TrainBars B;
+  const int tid = threadIdx.x, warp = tid >> 5;
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 32;\n" ::"r"(smem_u32(&B.tmem)));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
+  }
+  if (tid == 0) {
+    for (int c = 0; c < kRing; c++) {
+      mbar_init(smem_u32(&B.full[c]), 1);
+      mbar_init(smem_u32(&B.empty[c]), 1);
+    }
+    mbar_init(smem_u32(&B.done), 1);
+    B.fail = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::);
+    fence_async();
+  }
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  if (blockIdx.x < kRowCtas) train_rows(g, smem, B);
+  else train_tile(g, smem, B);
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 32;\n" ::"r"(B.tmem));
+}
+constexpr int kTrainSmem = kRing * 2 * (int)kChunkB + 32 * (int)kHsBox;
+
 inline int pad16(int x) { return (x + 15) / 16 * 16; }
 
-constexpr int kBatch = 256;     // training rows per step
 constexpr int kChunk = 65536;   // inference rows per pass
 
 struct Mlp {
@@ -630,8 +1133,19 @@ struct Mlp {
   bf16 *PX = nullptr;
   std::vector<bf16 *> PH;
   float *PZ = nullptr, *px = nullptr;
-  cudaGraphExec_t step_graph = nullptr;
-  const float *graph_x = nullptr;
+  // k_train: its blocked buffers and tiles (lazily), grid barrier
+  std::vector<TrainLayer> tl;
+  uint32_t *tile = nullptr;
+  int tiles = 0;
+  unsigned int *bar = nullptr;
+  // the training set on the device, kept (grown) across calls: fit() trains in
+  // rounds on the same rows
+  float *xall = nullptr, *tall = nullptr, *eloss = nullptr;
+  int *perm = nullptr;
+  int *order = nullptr;  // pinned: the orders of two epochs
+  cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};  // order copied (2), device time
+  uint64_t cap_rows = 0;
+  uint32_t cap_epochs = 0;
   std::vector<void *> allocs;
   float lr = 1e-3f;
 };
@@ -680,8 +1194,10 @@ void destroy(Mlp *m) {
   if (!m) return;
   cudaSetDevice(m->device);
   if (m->st) cudaStreamSynchronize(m->st);
-  if (m->step_graph) cudaGraphExecDestroy(m->step_graph);
   for (void *p : m->allocs) cudaFree(p);
+  if (m->order) cudaFreeHost(m->order);
+  for (cudaEvent_t x : m->ev)
+    if (x) cudaEventDestroy(x);
   if (m->st) cudaStreamDestroy(m->st);
   delete m;
 }
@@ -990,29 +1506,56 @@ int forward(Mlp *m, const float *x, uint64_t rows, float *y, double *device_ms, 
   return rc;
 }
 
-int train(Mlp *m, const float *x, const float *t, uint64_t rows, uint32_t epochs, float lr, uint64_t seed,
-          float *epoch_loss, double *device_ms, std::string &err) {
-  const int steps = (int)(rows / kBatch);
-  if (steps < 1) {
-    err = "mlp train: need at least 256 rows";
-    return FS_ERR_ARG;
+// Buffers and tiles of k_train; m->tiles = -1: the network has more weight
+// tiles than SMs beside the row CTAs (each tile's owner keeps it in registers).
+int ensure_train(Mlp *m, std::string &err) {
+  if (m->tiles) return FS_OK;
+  std::vector<uint32_t> tile;
+  for (int l = 0; l < m->L; l++)
+    for (int mt = 0; mt * 128 < m->pd[l + 1]; mt++)
+      for (int nt = 0; nt * kTileN < m->pd[l]; nt++) tile.push_back((uint32_t)(l | mt << 8 | nt << 16));
+  int sms = 0, coop = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device);
+  cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, m->device);
+  if (m->L > kMaxTrainL || !coop || (int)tile.size() + kRowCtas > sms) {
+    m->tiles = -1;
+    return FS_OK;
   }
-  m->lr = lr;
-  float *xall = nullptr, *tall = nullptr;
-  int *perm = nullptr;
-  int rc;
-  if ((rc = mal(m, &xall, rows * m->dims[0], err)) || (rc = mal(m, &tall, rows * m->dims[m->L], err)) ||
-      (rc = mal(m, &perm, (size_t)steps * kBatch, err))) {
-    release(m, xall);
-    release(m, tall);
-    release(m, perm);
-    return rc;
+  std::vector<TrainLayer> tl(m->L);
+  int rc = FS_OK;
+  for (int l = 0; l < m->L && !rc; l++) {
+    TrainLayer &y = tl[l];
+    y.in = m->pd[l];
+    y.out = m->pd[l + 1];
+    const auto up = [](int v, int k) { return (size_t)((v + k - 1) / k); };
+    if ((rc = mal(m, &y.Wk, up(y.out, 128) * up(y.in, 64) * (kChunkB / 2), err)) ||
+        (rc = mal(m, &y.Wt, up(y.in, 128) * up(y.out, 64) * (kChunkB / 2), err)) ||
+        (rc = mal(m, &y.HT, up(y.in, kTileN) * kTileN * kBatch, err)) ||
+        (rc = mal(m, &y.dZT, up(y.out, 128) * 128 * kBatch, err)))
+      break;
+    y.W = m->W[l]; y.mW = m->mW[l]; y.vW = m->vW[l];
+    y.b = m->b[l]; y.mb = m->mb[l]; y.vb = m->vb[l];
   }
-  cudaMemcpyAsync(xall, x, rows * m->dims[0] * 4, cudaMemcpyHostToDevice, m->st);
-  cudaMemcpyAsync(tall, t, rows * m->dims[m->L] * 4, cudaMemcpyHostToDevice, m->st);
-  // one training step, captured once and replayed
+  if (!rc) rc = mal(m, &m->tile, tile.size(), err);
+  if (!rc) rc = mal(m, &m->bar, 64, err);
+  if (rc) return rc;
+  cudaError_t e = cudaMemcpyAsync(m->tile, tile.data(), tile.size() * 4, cudaMemcpyHostToDevice, m->st);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_train, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrainSmem);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(m->st);
+  if (e != cudaSuccess) {
+    err = std::string("mlp train set-up: ") + cudaGetErrorString(e);
+    return FS_ERR_CUDA;
+  }
+  m->tl = tl;
+  m->tiles = (int)tile.size();
+  return FS_OK;
+}
+
+// One Adam step, captured once and replayed (networks k_train does not take).
+int capture_step(Mlp *m, const float *xall, const float *tall, const int *perm, cudaGraphExec_t *exec,
+                 std::string &err) {
   cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
+  int rc = FS_OK;
   cudaError_t e = cudaStreamBeginCapture(m->st, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
     k_stage_x<<<(kBatch * m->pd[0] + 255) / 256, 256, 0, m->st>>>(xall, kBatch, m->dims[0], m->pd[0], perm, m->ctr,
@@ -1024,50 +1567,131 @@ int train(Mlp *m, const float *x, const float *t, uint64_t rows, uint32_t epochs
     cudaError_t e2 = cudaStreamEndCapture(m->st, &graph);
     if (!rc && e2 != cudaSuccess) e = e2;
   }
-  if (!rc && e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
+  if (!rc && e == cudaSuccess) e = cudaGraphInstantiate(exec, graph, 0);
   if (graph) cudaGraphDestroy(graph);
   if (!rc && e != cudaSuccess) {
     err = std::string("mlp train graph: ") + cudaGetErrorString(e);
     rc = FS_ERR_CUDA;
   }
-  std::mt19937_64 gen(seed ? seed : 1);
-  std::vector<int> order(rows);
-  cudaEvent_t e0, e1;
-  cudaEventCreate(&e0);
-  cudaEventCreate(&e1);
-  double ms_total = 0.0;
-  for (uint32_t ep = 0; ep < epochs && !rc; ep++) {
-    std::iota(order.begin(), order.end(), 0);
-    std::shuffle(order.begin(), order.end(), gen);
-    cudaMemcpyAsync(perm, order.data(), (size_t)steps * kBatch * 4, cudaMemcpyHostToDevice, m->st);
-    cudaMemsetAsync(m->ctr, 0, 4, m->st);  // batch index (the Adam count in ctr[1] runs on)
-    cudaMemsetAsync(m->loss, 0, 4, m->st);
-    cudaEventRecord(e0, m->st);
-    for (int s = 0; s < steps; s++) {
-      e = cudaGraphLaunch(exec, m->st);
-      if (e != cudaSuccess) break;
+  return rc;
+}
+
+// Device and pinned buffers for `rows` training rows and `epochs` epochs.
+int ensure_rows(Mlp *m, uint64_t rows, uint32_t epochs, std::string &err) {
+  int rc = FS_OK;
+  if (rows > m->cap_rows) {
+    m->cap_rows = 0;
+    release(m, m->xall);
+    release(m, m->tall);
+    release(m, m->perm);
+    m->xall = m->tall = nullptr;
+    m->perm = nullptr;
+    if (m->order) cudaFreeHost(m->order);
+    m->order = nullptr;
+    if ((rc = mal(m, &m->xall, rows * m->dims[0], err)) || (rc = mal(m, &m->tall, rows * m->dims[m->L], err)) ||
+        (rc = mal(m, &m->perm, rows, err)))
+      return rc;
+    if (cudaMallocHost((void **)&m->order, 2 * rows * sizeof(int)) != cudaSuccess) {
+      m->order = nullptr;
+      err = "mlp train: pinned host memory";
+      return FS_ERR_NOMEM;
     }
-    cudaEventRecord(e1, m->st);
-    if (e != cudaSuccess) {
-      err = std::string("mlp train: ") + cudaGetErrorString(e);
-      rc = FS_ERR_CUDA;
-      break;
-    }
-    if ((rc = check(m, err))) break;
-    float ms = 0, l = 0;
-    cudaEventElapsedTime(&ms, e0, e1);
-    ms_total += ms;
-    cudaMemcpy(&l, m->loss, 4, cudaMemcpyDeviceToHost);
-    if (epoch_loss) epoch_loss[ep] = l / (float)steps;
+    m->cap_rows = rows;
   }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
+  if (epochs > m->cap_epochs) {
+    m->cap_epochs = 0;
+    release(m, m->eloss);
+    m->eloss = nullptr;
+    if ((rc = mal(m, &m->eloss, epochs, err))) return rc;
+    m->cap_epochs = epochs;
+  }
+  for (cudaEvent_t &e : m->ev)
+    if (!e && cudaEventCreate(&e) != cudaSuccess) {
+      e = nullptr;
+      err = "mlp train: event create";
+      return FS_ERR_CUDA;
+    }
+  return FS_OK;
+}
+
+int train(Mlp *m, const float *x, const float *t, uint64_t rows, uint32_t epochs, float lr, uint64_t seed,
+          float *epoch_loss, double *device_ms, std::string &err) {
+  const int steps = (int)(rows / kBatch);
+  if (steps < 1) {
+    err = "mlp train: need at least 256 rows";
+    return FS_ERR_ARG;
+  }
+  m->lr = lr;
+  int rc = ensure_train(m, err);
+  if (!rc) rc = ensure_rows(m, rows, epochs, err);
+  if (rc) return rc;
+  cudaMemcpyAsync(m->xall, x, rows * m->dims[0] * 4, cudaMemcpyHostToDevice, m->st);
+  cudaMemcpyAsync(m->tall, t, rows * m->dims[m->L] * 4, cudaMemcpyHostToDevice, m->st);
+  cudaGraphExec_t exec = nullptr;
+  if (m->tiles < 0 && (rc = capture_step(m, m->xall, m->tall, m->perm, &exec, err))) return rc;
+  TrainArgs a{};
+  for (size_t l = 0; l < m->tl.size(); l++) a.l[l] = m->tl[l];
+  a.L = m->L;
+  a.steps = steps;
+  a.din = m->dims[0];
+  a.dout = m->dims[m->L];
+  a.tiles = m->tiles;
+  a.x = m->xall;
+  a.t = m->tall;
+  a.perm = m->perm;
+  a.tile = m->tile;
+  a.lr = lr;
+  a.ctr = m->ctr;
+  a.bar = m->bar;
+  a.err = m->err;
+  std::mt19937_64 gen(seed ? seed : 1);
+  cudaError_t e = cudaSuccess;
+  auto ok = [&](cudaError_t r) {
+    if (e == cudaSuccess) e = r;
+    return e == cudaSuccess;
+  };
+  if (epochs) ok(cudaMemsetAsync(m->eloss, 0, (size_t)epochs * 4, m->st));
+  ok(cudaEventRecord(m->ev[2], m->st));
+  for (uint32_t ep = 0; ep < epochs && e == cudaSuccess; ep++) {
+    // the host draws an epoch's order while the device runs the last one
+    int *order = m->order + (ep & 1u) * m->cap_rows;
+    if (ep >= 2 && !ok(cudaEventSynchronize(m->ev[ep & 1u]))) break;
+    std::iota(order, order + rows, 0);
+    std::shuffle(order, order + rows, gen);
+    ok(cudaMemcpyAsync(m->perm, order, (size_t)steps * kBatch * 4, cudaMemcpyHostToDevice, m->st));
+    ok(cudaEventRecord(m->ev[ep & 1u], m->st));
+    if (exec) {
+      ok(cudaMemsetAsync(m->ctr, 0, 4, m->st));  // batch index (the Adam count in ctr[1] runs on)
+      ok(cudaMemsetAsync(m->loss, 0, 4, m->st));
+      for (int s = 0; s < steps && e == cudaSuccess; s++) ok(cudaGraphLaunch(exec, m->st));
+      ok(cudaMemcpyAsync(m->eloss + ep, m->loss, 4, cudaMemcpyDeviceToDevice, m->st));
+    } else {
+      a.loss = m->eloss + ep;
+      void *args[] = {&a};
+      ok(cudaMemsetAsync(m->bar, 0, 8, m->st));
+      if (e == cudaSuccess)
+        ok(cudaLaunchCooperativeKernel((const void *)k_train, kRowCtas + m->tiles, kTrThreads, args, kTrainSmem, m->st));
+    }
+  }
+  ok(cudaEventRecord(m->ev[3], m->st));
+  if (!exec)  // the row-major BF16 copies that inference and grad() read
+    for (int l = 0; l < m->L; l++) {
+      const int n = m->pd[l] * m->pd[l + 1];
+      k_refresh<<<(n + 255) / 256, 256, 0, m->st>>>(m->W[l], m->pd[l + 1], m->pd[l], m->Wb[l], m->Wt[l]);
+    }
+  std::vector<float> el(epochs, 0.0f);
+  if (epochs) ok(cudaMemcpyAsync(el.data(), m->eloss, (size_t)epochs * 4, cudaMemcpyDeviceToHost, m->st));
+  rc = check(m, err);
   if (exec) cudaGraphExecDestroy(exec);
-  cudaStreamSynchronize(m->st);
-  release(m, xall);
-  release(m, tall);
-  release(m, perm);
-  if (device_ms) *device_ms = ms_total;
+  if (!rc && e != cudaSuccess) {
+    err = std::string("mlp train: ") + cudaGetErrorString(e);
+    rc = FS_ERR_CUDA;
+  }
+  float ms = 0;
+  if (!rc) cudaEventElapsedTime(&ms, m->ev[2], m->ev[3]);
+  if (epoch_loss)
+    for (uint32_t ep = 0; ep < epochs && !rc; ep++) epoch_loss[ep] = el[ep] / (float)steps;
+  if (device_ms) *device_ms = ms;
   return rc;
 }
 
