@@ -29,9 +29,10 @@
 // contiguous range of post neurons and, per interval, (1) pulls the NMDA
 // conductances of all the interval's steps at once (one warp per post, the
 // in-edges split over the lanes, a butterfly reduction per step: the loads of
-// many steps overlap), then (2) advances its neurons one thread each through
-// the interval's steps with their state in registers, pushing the spikes of
-// each step into the delay ring (one warp per spike).  The ring depth
+// many steps overlap), then (2) advances its neurons through the interval's
+// steps in three passes (conductances by a thread per neuron and receptor,
+// membranes and then presynaptic state by a thread per neuron) and pushes the
+// interval's spikes into the delay ring.  The ring depth
 // S = next power of two >= max_delay + min_delay + 2 keeps the reuse of a
 // slot out of any interval that still reads it.
 #include <algorithm>
@@ -41,6 +42,7 @@
 #include <numeric>
 #include <string>
 #include <thread>
+#include <type_traits>
 #include <vector>
 #include <cuda_runtime.h>
 #include "fs_prod.cuh"
@@ -68,6 +70,7 @@ enum { PL_NONE = 0, PL_STD = 1, PL_STP = 2, PL_TM = 3 };
 struct Params {
   uint32_t n, slots, mask, interval, nlin;
   uint32_t dmax0;                        // every delay is 0 (single-step pull order)
+  uint32_t live;                         // receptors in use (see step_membrane)
   int lin_of_rec[4];
   const float *Vth, *El, *gl, *Cm, *Vreset, *df, *ef, *dVmax;
   const int32_t *RfPed, *SpiDy;
@@ -222,6 +225,12 @@ __device__ __forceinline__ float fma_t<float>(float a, float b, float c) { retur
 template <>
 __device__ __forceinline__ double fma_t<double>(double a, double b, double c) { return __fma_rn(a, b, c); }
 
+// one rounding each, never fused
+__device__ __forceinline__ float mul_t(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_t(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float add_t(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double add_t(double a, double b) { return __dadd_rn(a, b); }
+
 template <class T>
 __device__ __forceinline__ T warp_sum(T v) {
 #pragma unroll
@@ -256,9 +265,9 @@ __device__ __forceinline__ float comp4(const float4 &q, int k) {
 // quads by an xor butterfly over the eight groups.  The group size depends
 // on the network's interval alone, so the sums depend on neither U, the
 // block plan, the kernel nor the length of a batch.
-template <int U>
+template <int U, uint32_t KT>
 __device__ __forceinline__ void nmda_pull_f32(const Params &P, uint32_t p0, uint32_t np, uint64_t tb, uint32_t L,
-                                              float (*gn)[kTile], uint32_t wid, uint32_t lane) {
+                                              float (*gn)[KT], uint32_t wid, uint32_t lane) {
   const float4 *sh = (const float4 *)P.s_hist;
   const uint32_t S4 = P.slots >> 2, qmask = S4 - 1, mask = P.mask;
   const uint32_t nvl = (L + 3u) >> 2;  // vectors needed for L steps
@@ -357,28 +366,42 @@ __device__ __forceinline__ void nmda_pull_f32(const Params &P, uint32_t p0, uint
 // persistent kernel (k_prod1) sums its shared-memory copy of the same edges
 // in the same order, so the two kernels, and a batch instance and its solo
 // run, give the same sums bit for bit.
-template <bool kMW = false>
+//
+// kDense: s of step tb - 1 is read from s_pre itself (4 B a neuron, several of
+// a region's sources in one line) instead of the history (128 B a neuron: a
+// line per edge); for kernels that do not step any neuron between the start
+// and the end of a pull.  Four of a lane's edges are in flight.
+template <bool kMW, bool kDense, uint32_t KT>
 __device__ __forceinline__ void nmda_pull1_f32(const Params &P, uint32_t p0, uint32_t np, uint64_t tb,
-                                               float (*gn)[kTile], uint32_t wid, uint32_t lane) {
-  const float *sh = (const float *)P.s_hist;
-  const uint32_t S = P.slots, mask = P.mask;
+                                               float (*gn)[KT], uint32_t wid, uint32_t lane) {
   const uint32_t nw = kThreads / 32;
   if (!P.in_row) {
     for (uint32_t q = wid * 32 + lane; q < np; q += nw * 32) gn[0][q] = 0.0f;
     return;
   }
-  const uint32_t slot = (uint32_t)(tb - 1u) & mask;
+  // row 0 of the shifted copies holds slot i at element i
+  const float *sh = kDense ? (const float *)P.s_pre : (const float *)P.s_hist + ((uint32_t)(tb - 1u) & P.mask);
+  const size_t stride = kDense ? 1u : kSH * P.slots;
   const uint32_t h = lane >> 3, l8 = lane & 7u;
   for (uint32_t q0 = wid * 4u; q0 < np; q0 += nw * 4u) {
     const uint32_t q = q0 + h;
     const bool has = q < np;
     const uint32_t b0 = has ? __ldg(P.in_row + p0 + q) : 0u, b1 = has ? __ldg(P.in_row + p0 + q + 1) : 0u;
     float acc = 0.0f;
-    for (uint32_t e = b0 + l8; e < b1; e += 8) {
-      const uint32_t pre = __ldg(P.in_code + e) & 0xffffffu;
-      // row 0 of the shifted copies holds slot i at element i
-      const float w = kMW ? __ldcg(P.in_w + e) : __ldg(P.in_w + e);
-      acc = __fmaf_rn(w, __ldca(sh + (size_t)pre * kSH * S + slot), acc);
+    for (uint32_t e = b0 + l8; e < b1; e += 32) {
+      uint32_t pre[4];
+      float w[4], v[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const bool ok = e + 8u * u < b1;
+        pre[u] = ok ? __ldg(P.in_code + e + 8u * u) & 0xffffffu : 0u;
+        w[u] = ok ? (kMW ? __ldcg(P.in_w + e + 8u * u) : __ldg(P.in_w + e + 8u * u)) : 0.0f;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++) v[u] = e + 8u * u < b1 ? __ldca(sh + pre[u] * stride) : 0.0f;
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (e + 8u * u < b1) acc = __fmaf_rn(w[u], v[u], acc);
     }
 #pragma unroll
     for (int o = 4; o; o >>= 1) acc += __shfl_xor_sync(fsd::kFull, acc, o);
@@ -386,9 +409,27 @@ __device__ __forceinline__ void nmda_pull1_f32(const Params &P, uint32_t p0, uin
   }
 }
 
-template <class T, bool kMW = false>
+// The FP64 pull of one step from s_pre (as kDense above), in nmda_pull's order.
+template <bool kMW>
+__device__ __forceinline__ void nmda_pull1_f64(const Params &P, uint32_t p0, uint32_t np, double *gn, uint32_t wid,
+                                               uint32_t lane) {
+  const double *sh = (const double *)P.s_pre;
+  for (uint32_t q = wid; q < np; q += kThreads / 32) {
+    double acc = 0.0;
+    if (P.in_row) {
+      const uint32_t e1 = __ldg(P.in_row + p0 + q + 1);
+      for (uint32_t e = __ldg(P.in_row + p0 + q) + lane; e < e1; e += 32)
+        acc = __fma_rn((double)(kMW ? __ldcg(P.in_w + e) : __ldg(P.in_w + e)),
+                       __ldca(sh + (__ldg(P.in_code + e) & 0xffffffu)), acc);
+    }
+    acc = warp_sum<double>(acc);
+    if (lane == 0) gn[q] = acc;
+  }
+}
+
+template <class T, uint32_t KT>
 __device__ __forceinline__ void nmda_pull(const Params &P, uint32_t p0, uint32_t np, uint64_t tb, uint32_t L,
-                                          T (*gn)[TileW<T>::W], uint32_t wid, uint32_t lane) {
+                                          T (*gn)[KT], uint32_t wid, uint32_t lane) {
   const T *sh = (const T *)P.s_hist;
   const uint32_t S = P.slots, mask = P.mask;
   const uint32_t nw = kThreads / 32;
@@ -401,7 +442,7 @@ __device__ __forceinline__ void nmda_pull(const Params &P, uint32_t p0, uint32_t
       const uint32_t e0 = __ldg(P.in_row + p), e1 = __ldg(P.in_row + p + 1);
       for (uint32_t e = e0 + lane; e < e1; e += 32) {
         const uint32_t code = __ldg(P.in_code + e);
-        const T w = (T)(kMW ? __ldcg(P.in_w + e) : __ldg(P.in_w + e));
+        const T w = (T)__ldg(P.in_w + e);
         const uint32_t pre = code & 0xffffffu, d = code >> 24;
         const T *row = sh + (size_t)pre * S;
         const uint32_t a = (uint32_t)(tb - 1u - d) & mask;
@@ -496,14 +537,14 @@ __device__ __forceinline__ uint32_t draw_one(const Params &P, uint32_t p, uint64
 
 // Draws of L steps for a tile, by all threads at once, off the neurons'
 // per-step dependency chain.
-template <class T>
+template <class T, uint32_t KT>
 __device__ __forceinline__ void draw_inputs(const Params &P, uint32_t p0, uint32_t np, uint64_t tb, uint32_t L,
-                                            uint8_t (*hits)[TileW<T>::W], T (*gauss)[TileW<T>::W]) {
+                                            uint8_t (*hits)[KT], T (*gauss)[KT]) {
   for (uint32_t idx = threadIdx.x; idx < np * L; idx += kThreads) {
     const uint32_t j = idx / np, q = idx - j * np;
     T gv = (T)0;
     hits[j][q] = (uint8_t)draw_one<T>(P, p0 + q, tb + j, gv);
-    gauss[j][q] = gv;
+    if (gauss) gauss[j][q] = gv;  // (null: no neuron has injection)
   }
 }
 
@@ -566,13 +607,12 @@ struct NeuronState {
   float tmu, tmx;  // Tsodyks-Markram u, x (float between steps)
 };
 
-// kTM = false: the caller never runs a Tsodyks-Markram network (no
-// registers are spent on its state).
-template <class T, bool kTM = true>
-__device__ __forceinline__ void load_neuron(const Params &P, uint32_t p, NeuronPar<T> &q, NeuronState<T> &st) {
+// Loads and stores of a neuron's parameters and state by the part that uses
+// them (below): drive and conductances, membrane, presynaptic.
+template <class T>
+__device__ __forceinline__ void load_membrane(const Params &P, uint32_t p, NeuronPar<T> &q, NeuronState<T> &st) {
   const uint32_t n = P.n;
   q.a = P.act[p];
-  q.pj = P.proj[p];
   q.rf = __ldg(P.RfPed + p);
   q.sd = __ldg(P.SpiDy + p);
   q.vth = (T)__ldg(P.Vth + p);
@@ -584,63 +624,91 @@ __device__ __forceinline__ void load_neuron(const Params &P, uint32_t p, NeuronP
   q.leak = (T)__ldg(P.gl + p) * (T)__ldg(P.El + p) * (T)1e3;
   q.mg = (T)__ldg(P.nmda_mg + p) / (T)3.57;
 #pragma unroll
-  for (int r = 0; r < 5; r++) {
-    q.vrev[r] = (T)__ldg(P.Vrev + (size_t)r * n + p);
-    q.dfs[r] = (T)__ldg(P.dfst + (size_t)r * n + p);
-    q.extg[r] = (T)__ldg(P.ext_g + (size_t)r * n + p);
-  }
-  q.ndfxt = (T)__ldg(P.nmda_dfxt + p);
-  q.nefas = (T)__ldg(P.nmda_efst + p) * (T)__ldg(P.nmda_as + p);
+  for (int r = 0; r < 5; r++) q.vrev[r] = (T)__ldg(P.Vrev + (size_t)r * n + p);
+  st.V = ((T *)P.V)[p];
+  st.cnt = P.Count[p];
+  st.ns = P.NS[p];
+}
+template <class T>
+__device__ __forceinline__ void store_membrane(const Params &P, uint32_t p, const NeuronState<T> &st) {
+  ((T *)P.V)[p] = st.V;
+  P.Count[p] = st.cnt;
+  P.NS[p] = st.ns;
+}
+
+// kTM = false: the caller never runs a Tsodyks-Markram network (no
+// registers are spent on its state).
+template <class T, bool kTM = true>
+__device__ __forceinline__ void load_pre(const Params &P, uint32_t p, NeuronPar<T> &q, NeuronState<T> &st) {
+  const uint32_t n = P.n;
+  q.pj = P.proj[p];
 #pragma unroll
-  for (int r = 0; r < 4; r++) q.pdf[r] = (T)__ldg(P.pdf + (size_t)r * n + p);
+  for (int r = 0; r < 4; r++) {
+    q.pdf[r] = P.lin_of_rec[r] >= 0 ? (T)__ldg(P.pdf + (size_t)r * n + p) : (T)0;
+    st.sp[r] = P.lin_of_rec[r] >= 0 ? ((T *)P.st_pre)[(size_t)r * n + p] : (T)0;
+  }
   q.pdfxt = (T)__ldg(P.p_dfxt + p);
   q.pdfst = (T)__ldg(P.p_dfst + p);
   q.pefas = (T)__ldg(P.p_efas + p);
-  // the Tsodyks-Markram state lives in registers for the launch (or batch;
-  // its parameters are read-only loads of each step); a neuron without
-  // projections has no presynaptic state
+  st.xp = ((T *)P.x_pre)[p];
+  st.spre = ((T *)P.s_pre)[p];
+  // the Tsodyks-Markram state lives in registers for the launch (or batch);
+  // a neuron without projections has no presynaptic state
   st.tmu = st.tmx = 0.0f;
   if (kTM && P.plast == PL_TM && q.pj && P.tm_on[p]) {
     q.pj |= kPjTM;
     st.tmu = P.tm_u[p];
     st.tmx = P.tm_x[p];
   }
-  st.V = ((T *)P.V)[p];
-  st.cnt = P.Count[p];
-  st.ns = P.NS[p];
+}
+template <class T, bool kTM = true>
+__device__ __forceinline__ void store_pre(const Params &P, uint32_t p, const NeuronPar<T> &q, const NeuronState<T> &st) {
+  const uint32_t n = P.n;
+#pragma unroll
+  for (int r = 0; r < 4; r++)
+    if (P.lin_of_rec[r] >= 0) ((T *)P.st_pre)[(size_t)r * n + p] = st.sp[r];
+  ((T *)P.x_pre)[p] = st.xp;
+  ((T *)P.s_pre)[p] = st.spre;
+  if (kTM && (q.pj & kPjTM)) {
+    P.tm_u[p] = st.tmu;
+    P.tm_x[p] = st.tmx;
+  }
+}
+
+template <class T, bool kTM = true>
+__device__ __forceinline__ void load_neuron(const Params &P, uint32_t p, NeuronPar<T> &q, NeuronState<T> &st) {
+  const uint32_t n = P.n;
+  load_membrane<T>(P, p, q, st);
+  load_pre<T, kTM>(P, p, q, st);
+#pragma unroll
+  for (int r = 0; r < 5; r++) {
+    q.dfs[r] = (T)__ldg(P.dfst + (size_t)r * n + p);
+    q.extg[r] = (T)__ldg(P.ext_g + (size_t)r * n + p);
+  }
+  q.ndfxt = (T)__ldg(P.nmda_dfxt + p);
+  q.nefas = (T)__ldg(P.nmda_efst + p) * (T)__ldg(P.nmda_as + p);
 #pragma unroll
   for (int r = 0; r < 4; r++) {
     st.G[r] = ((T *)P.G)[(size_t)r * n + p];
     st.est[r] = ((T *)P.ext_st)[(size_t)r * n + p];
-    st.sp[r] = ((T *)P.st_pre)[(size_t)r * n + p];
   }
   st.ex = ((T *)P.ext_x)[p];
   st.es = ((T *)P.ext_s)[p];
-  st.xp = ((T *)P.x_pre)[p];
-  st.spre = ((T *)P.s_pre)[p];
 }
 
 template <class T, bool kTM = true>
 __device__ __forceinline__ void store_neuron(const Params &P, uint32_t p, const NeuronPar<T> &q,
                                              const NeuronState<T> &st) {
   const uint32_t n = P.n;
-  if (kTM && (q.pj & kPjTM)) {
-    P.tm_u[p] = st.tmu;
-    P.tm_x[p] = st.tmx;
-  }
-  ((T *)P.V)[p] = st.V;
-  P.Count[p] = st.cnt;
-  P.NS[p] = st.ns;
+  store_membrane<T>(P, p, st);
+  store_pre<T, kTM>(P, p, q, st);
 #pragma unroll
   for (int r = 0; r < 4; r++) {
     ((T *)P.G)[(size_t)r * n + p] = st.G[r];
     ((T *)P.ext_st)[(size_t)r * n + p] = st.est[r];
-    ((T *)P.st_pre)[(size_t)r * n + p] = st.sp[r];
   }
   ((T *)P.ext_x)[p] = st.ex;
   ((T *)P.ext_s)[p] = st.es;
-  ((T *)P.x_pre)[p] = st.xp;
-  ((T *)P.s_pre)[p] = st.spre;
 }
 
 // NMDA presynaptic kinetics of one step (code/EqsGnl2.cpp:493): x jumps by
@@ -663,18 +731,194 @@ struct LtpTrace {
   int32_t clp, spd;
 };
 
-// One step of neuron p: fold the linear conductances' delivered sums
-// (rv: 2^-40 fixed point) into G, add the external drive (hit bits, injection
-// current) and the NMDA sum gnmda, VmEul + firing (code/EqsGnl2.cpp:152-251),
-// per-step outputs of step s, then the presynaptic state: the increment inc of
-// a spike and, per linear receptor, c = inc + st(t-1)(1 - df) for the push.
-// kLTP: also the LP trace of a neuron with LTP on (lt; firLP and ltpEul,
-// code/EqsGnl2.cpp:207-216, :254-280).  Returns whether the neuron spiked.
-template <class T, bool kTM = true, bool kLTP = false>
+// One step of neuron p is three parts, each defined once for every kernel:
+//  * conductances: the delivered sums (rv: 2^-40 fixed point) folded into the
+//    linear conductances G, the external drive's gates (hit bits) and the NMDA
+//    sum (fold_linear, drive_linear, drive_nmda);
+//  * step_membrane: VmEul + firing (code/EqsGnl2.cpp:152-251) over them and the
+//    per-step outputs; returns whether the neuron spikes;
+//  * step_pre: the presynaptic state after a spike or none: the increment inc
+//    and, per linear receptor, c = inc + st(t-1)(1 - df) for the push.
+// Only the middle one is a chain from step to step that a neuron's spikes run
+// through: the conductances of a batch of steps depend on nothing of the batch
+// but drive draws and finished deliveries, and the presynaptic state only on
+// the spikes, so kernels may spread them over other threads or do them
+// earlier and later.  Sums and products are fused in the one way written here
+// (the receptor currents' sum is not fused).  P.live says which receptors any
+// neuron of the network uses (bits 0-3: linear receptor r has synapses or
+// drive; 8-12: receptor r has had drive; 16: some neuron has injection): a dead
+// one's gates are 0 and its current is +-0, which no sum shows.
+__device__ __forceinline__ uint32_t act_of_rec(uint32_t r) {
+  return r == 0 ? FS_ACT_AMPA : r == 1 ? FS_ACT_GABA : r == 2 ? FS_ACT_ACH : FS_ACT_GCL;
+}
+
+template <class T>
+__device__ __forceinline__ T fold_linear(T dfs, T G, long long rv) {
+  return fma_t<T>(dfs, G, (T)rv * (T)kInvFix);  // exact power-of-two scale
+}
+template <class T>
+__device__ __forceinline__ T drive_linear(T est, T dfs, bool hit) {
+  return hit ? est + (T)1 : est * dfs;
+}
+template <class T>
+__device__ __forceinline__ void drive_nmda(T &ex, T &es, T ndfxt, T dfs, T nefas, bool hit) {
+  ex = hit ? ex + (T)1 : ex * ndfxt;
+  es = fma_t<T>(dfs, es, mul_t(mul_t(nefas, ex), add_t((T)1, -es)));
+}
+
+// g: the step's conductances, by receptor (dead linear receptors' are not read).
+template <class T, bool kLTP = false>
+__device__ __forceinline__ bool step_membrane(const Params &P, const NeuronPar<T> &q, NeuronState<T> &st, const T (&g)[5],
+                                              T gauss, T gapI, uint32_t p, bool own, uint32_t s,
+                                              LtpTrace<T> *lt = nullptr) {
+  const uint32_t n = P.n;
+  T isyn = (T)0;
+  if (q.a & FS_ACT_INJ) isyn = gauss;
+  if (P.gap_row) isyn = isyn + gapI;  // steps of networks with gap junctions come one at a time
+  // the production modes scale the Mg block and the current by per-neuron
+  // constants formed once (Mg / 3.57, 1e-3 / Cm), where the reference divides
+  // every step: two divisions off each step's dependency chain, at a rounding
+  // difference the FP32 and FP64 modes share
+  uint32_t ns = st.ns;
+  bool fire_now = false;
+  if (ns & FS_NS_FIRE) {
+    fire_now = true;
+  } else {
+    const T v = st.V;
+    const T Ir2 = mul_t(g[FS_NMDA], q.vrev[FS_NMDA] - v) / fma_t<T>(q.mg, exp_t<T>(mul_t((T)-0.062, v)), (T)1);
+    T I = (T)0;
+    if (P.live & 1u) I = mul_t(g[FS_AMPA], q.vrev[FS_AMPA] - v);
+    if (P.live & 2u) I = add_t(I, mul_t(g[FS_GABA], q.vrev[FS_GABA] - v));
+    I = add_t(I, Ir2);
+    if (P.live & 4u) I = add_t(I, mul_t(g[FS_ACH], q.vrev[FS_ACH] - v));
+    if (P.live & 8u) I = add_t(I, mul_t(g[FS_GCL], q.vrev[FS_GCL] - v));
+    I = add_t(fma_t<T>(isyn, (T)1e3, I), q.leak);
+    I = mul_t(I, q.icm);
+    if (I > q.dvm) {
+      I = q.dvm;
+      ns = (ns | FS_NS_MEMDV_OVF) & ~FS_NS_MEMDV_UDF;
+    } else if (I < -q.dvm) {
+      I = -q.dvm;
+      ns = (ns & ~FS_NS_MEMDV_OVF) | FS_NS_MEMDV_UDF;
+    } else {
+      ns &= ~(FS_NS_MEMDV_OVF | FS_NS_MEMDV_UDF);
+    }
+    st.V = fma_t<T>(q.df, v, mul_t(q.ef, I));
+    if (P.outI && own) {  // kept only while requested (code/EqsGnl2.cpp:196-206)
+      P.Irep[p] = (float)((P.live & 1u) ? mul_t(g[FS_AMPA], q.vrev[FS_AMPA] - v) : (T)0);
+      P.Irep[(size_t)n + p] = (float)((P.live & 2u) ? mul_t(g[FS_GABA], q.vrev[FS_GABA] - v) : (T)0);
+      P.Irep[(size_t)FS_NMDA * n + p] = (float)Ir2;
+      P.Irep[(size_t)FS_ACH * n + p] = (float)((P.live & 4u) ? mul_t(g[FS_ACH], q.vrev[FS_ACH] - v) : (T)0);
+      P.Irep[(size_t)FS_GCL * n + p] = (float)((P.live & 8u) ? mul_t(g[FS_GCL], q.vrev[FS_GCL] - v) : (T)0);
+    }
+    if (st.V > q.vth) {
+      ns |= FS_NS_FIRE;
+      fire_now = true;
+      if constexpr (kLTP) {
+        if (q.a & FS_ACT_LTP) ns |= FS_NS_LP_FIRE;
+      }
+    }
+  }
+  if (fire_now) {
+    if (st.cnt < q.rf) {
+      st.V = (st.cnt == 0) ? (T)0 : q.vreset;
+      if (st.cnt == q.sd) ns |= FS_NS_SPIKE;
+      else ns &= ~FS_NS_SPIKE;
+      st.cnt++;
+    } else {
+      st.cnt = 0;
+      ns &= ~FS_NS_FIRE;
+    }
+  }
+  if constexpr (kLTP) {
+    if (q.a & FS_ACT_LTP) {  // firLP + ltpEul
+      if (ns & FS_NS_LP_FIRE) {
+        if (lt->clp == lt->spd) {
+          ns = (ns | FS_NS_LP_SPIKE) & ~FS_NS_LP_FIRE;
+          lt->clp = 0;
+        } else {
+          ns &= ~FS_NS_LP_SPIKE;
+          lt->clp++;
+        }
+      } else {
+        ns &= ~FS_NS_LP_SPIKE;
+      }
+      lt->lp = (ns & FS_NS_LP_SPIKE) ? __fadd_rn(lt->lp, 1.0f) : __fmul_rn(lt->dflp, lt->lp);
+    }
+  }
+  st.ns = ns;
+  if (own && P.outV) P.outV[(size_t)s * n + p] = (float)st.V;
+  if (own && P.outNS) P.outNS[(size_t)s * n + p] = ns;
+  if (own && P.outI)
+#pragma unroll
+    for (int r = 0; r < 5; r++) P.outI[(size_t)s * 5 * n + (size_t)r * n + p] = P.Irep[(size_t)r * n + p];
+  return own && (ns & FS_NS_SPIKE) != 0;
+}
+
+// kTM = false: the caller never runs a Tsodyks-Markram network.  tm: the
+// Tsodyks-Markram U, dff, dfr from the caller's per-thread copy, or null (read
+// from global memory).
+template <class T, bool kTM = true>
+__device__ __forceinline__ void step_pre(const Params &P, const NeuronPar<T> &q, NeuronState<T> &st, bool spk, uint32_t p,
+                                         bool own, T (&cinc)[4], T &inc_out, const float *tm = nullptr) {
+#pragma unroll
+  for (int r = 0; r < 4; r++) cinc[r] = (T)0;
+  T inc = (T)1;
+  if (q.pj && own) {
+    if (P.plast == PL_STD) inc = (T)P.D[p];
+    else if (P.plast == PL_STP) inc = (T)P.D[p] * (T)P.F[p];
+    else if (kTM && (q.pj & kPjTM)) {
+      const T u = (T)st.tmu, x = (T)st.tmx;
+      const T U = (T)(tm ? tm[0] : __ldg(P.tm_U + p));
+      const T us = fma_t<T>(U, (T)1 - u, u), rel = us * x;
+      const T ud = fma_t<T>(u - U, (T)(tm ? tm[1] : __ldg(P.tm_dff + p)), U);
+      const T xd = fma_t<T>(x - (T)1, (T)(tm ? tm[2] : __ldg(P.tm_dfr + p)), (T)1);
+      inc = spk ? rel : inc;
+      st.tmu = (float)(spk ? us : ud);
+      st.tmx = (float)(spk ? x - rel : xd);
+    }
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+      if (P.lin_of_rec[r] >= 0) {
+        const bool on = (q.pj & (1u << r)) != 0;
+        const T a = st.sp[r];
+        cinc[r] = on && spk ? fma_t<T>(a, (T)1 - q.pdf[r], inc) : (T)0;
+        st.sp[r] = !on ? a : spk ? a + inc : a * q.pdf[r];
+      }
+    }
+    {
+      T x = st.xp, y = st.spre;
+      nmda_pre_step<T>(x, y, spk, inc, q.pdfxt, q.pdfst, q.pefas);
+      const bool on = (q.pj & (1u << FS_NMDA)) != 0;
+      st.xp = on ? x : st.xp;
+      st.spre = on ? y : st.spre;
+    }
+    if (P.plast == PL_STD) {
+      P.D[p] = spk ? P.D[p] * (1.0f - P.stp_pv[p]) : P.stp_dfD[p] * P.D[p] + P.stp_efD[p];
+    } else if (P.plast == PL_STP) {
+      float Dv = P.D[p], Fv = P.F[p], Cp = P.Cap[p], Cr = P.Car[p];
+      if (spk) {
+        Cr += P.stp_aCar[p];
+        Cp += P.stp_aCap[p];
+        Fv += (Cp + Cr) * (1.0f - Fv) * P.stp_aF[p];
+        Dv *= (1.0f - P.stp_pv[p] * Fv);
+      } else {
+        Cr = P.stp_dfCar[p] * Cr + P.stp_efCar[p];
+        Cp = P.stp_dfCap[p] * Cp;
+        Fv = P.stp_dfF[p] * Fv + P.stp_efF[p] * (Cp + Cr) * (1.0f - Fv) * P.stp_aF[p];
+        Dv = P.stp_dfD[p] * Dv + P.stp_efD[p];
+      }
+      P.D[p] = Dv; P.F[p] = Fv; P.Cap[p] = Cp; P.Car[p] = Cr;
+    }
+  }
+  inc_out = inc;
+}
+
+// The three parts in one thread (k_prod1).
+template <class T, bool kTM>
 __device__ __forceinline__ bool neuron_step(const Params &P, const NeuronPar<T> &q, NeuronState<T> &st,
                                             const long long (&rv)[4], T gnmda, uint32_t hit, T gauss, T gapI,
-                                            uint32_t p, bool own, uint32_t s, T (&cinc)[4], T &inc_out,
-                                            const float *tm = nullptr, LtpTrace<T> *lt = nullptr) {
+                                            uint32_t p, bool own, uint32_t s, T (&cinc)[4], T &inc_out) {
   const uint32_t n = P.n;
   T g[5];
 #pragma unroll
@@ -742,9 +986,6 @@ __device__ __forceinline__ bool neuron_step(const Params &P, const NeuronPar<T> 
     if (st.V > q.vth) {
       ns |= FS_NS_FIRE;
       fire_now = true;
-      if constexpr (kLTP) {
-        if (q.a & FS_ACT_LTP) ns |= FS_NS_LP_FIRE;
-      }
     }
   }
   if (fire_now) {
@@ -756,22 +997,6 @@ __device__ __forceinline__ bool neuron_step(const Params &P, const NeuronPar<T> 
     } else {
       st.cnt = 0;
       ns &= ~FS_NS_FIRE;
-    }
-  }
-  if constexpr (kLTP) {
-    if (q.a & FS_ACT_LTP) {  // firLP + ltpEul
-      if (ns & FS_NS_LP_FIRE) {
-        if (lt->clp == lt->spd) {
-          ns = (ns | FS_NS_LP_SPIKE) & ~FS_NS_LP_FIRE;
-          lt->clp = 0;
-        } else {
-          ns &= ~FS_NS_LP_SPIKE;
-          lt->clp++;
-        }
-      } else {
-        ns &= ~FS_NS_LP_SPIKE;
-      }
-      lt->lp = (ns & FS_NS_LP_SPIKE) ? __fadd_rn(lt->lp, 1.0f) : __fmul_rn(lt->dflp, lt->lp);
     }
   }
   st.ns = ns;
@@ -790,17 +1015,15 @@ __device__ __forceinline__ bool neuron_step(const Params &P, const NeuronPar<T> 
     else if (P.plast == PL_STP) inc = (T)P.D[p] * (T)P.F[p];
     else if (kTM && (q.pj & kPjTM)) {
       T u = (T)st.tmu, x = (T)st.tmx;
-      // parameters from the caller's per-thread copy (tm: U, dff, dfr) or
-      // from global memory
-      const T U = (T)(tm ? tm[0] : __ldg(P.tm_U + p));
+      const T U = (T)__ldg(P.tm_U + p);
       if (spk) {
         u = u + U * ((T)1 - u);
         const T rel = u * x;
         inc = rel;
         x = x - rel;
       } else {
-        u = U + (u - U) * (T)(tm ? tm[1] : __ldg(P.tm_dff + p));
-        x = (T)1 + (x - (T)1) * (T)(tm ? tm[2] : __ldg(P.tm_dfr + p));
+        u = U + (u - U) * (T)__ldg(P.tm_dff + p);
+        x = (T)1 + (x - (T)1) * (T)__ldg(P.tm_dfr + p);
       }
       st.tmu = (float)u;
       st.tmx = (float)x;
@@ -869,60 +1092,184 @@ __device__ __forceinline__ void gv_write(const Params &P, uint32_t p, uint32_t s
   }
 }
 
-// ---- L steps of a tile's neurons (thread per neuron), with the pushes ----
-// Per-neuron parameters and state stay in registers for the L steps; the
-// ring slots of the next PD steps are in flight while the current step
-// computes (they are final: every push into them happened before the
-// interval began); a warp pushes the spikes of its own lanes, so a step
-// needs no block barrier.  neuron_load issues a thread's loads (parameters,
-// state, Tsodyks-Markram parameters into its shared-memory copy, the first
-// ring slots).  (Issuing them before the batch's drive draws, to overlap
-// the draws, measured the same on the 1 M network: 0.7538 -> 0.7541.)
-template <class T>
-struct StepRegs {
-  NeuronPar<T> q;
-  NeuronState<T> st;
-  long long rv[4], rv2[4];  // ring slots of the first steps (step 0, step 1)
-};
-
-template <class T, int PD>
-__device__ __forceinline__ void neuron_load(const Params &P, uint32_t p0, uint32_t np, uint32_t sb, uint32_t L,
-                                            StepRegs<T> &R, float *tm3) {
-  static_assert(PD == 1 || PD == 2, "ring prefetch distance 1 or 2");
-  const uint32_t tid = threadIdx.x, mask = P.mask;
-  const bool own = tid < np;
-  const uint32_t p = own ? p0 + tid : p0;  // non-owners read a valid neuron, write nothing
-  load_neuron<T>(P, p, R.q, R.st);
-  if (R.q.pj & kPjTM) {
-    tm3[3 * tid] = P.tm_U[p];
-    tm3[3 * tid + 1] = P.tm_dff[p];
-    tm3[3 * tid + 2] = P.tm_dfr[p];
+// ---- L steps of a tile's neurons ---------------------------------------------
+// Shared memory of a tile (the posts a block advances together): this struct,
+// then the conductances of the live linear receptors [live][kLB][kT] and, when
+// some neuron has injection, its current [kLB][kT].
+template <class T, uint32_t KT>
+struct TileBufs {
+  static constexpr uint32_t kT = KT;
+  static constexpr uint32_t kCap = sizeof(T) == 4 ? 320 : 192;
+  T gn[kLB][kT];
+  T gapI[kT];
+  uint8_t hits[kLB][kT];
+  uint32_t l_n, l_p[kCap];
+  uint16_t l_tm[kCap];
+  T l_c[kCap][4];
+  __device__ __forceinline__ T (*lin())[kLB][kT] { return (T(*)[kLB][kT])(this + 1); }
+  __device__ __forceinline__ T (*gauss(const Params &P))[kT] {
+    return (P.live & 0x10000u) ? lin()[__popc(P.live & 15u)] : nullptr;
   }
-  const uint32_t tprev = (uint32_t)(P.t0 + sb - 1u) & mask, tn = (uint32_t)(P.t0 + sb) & mask;
+};
+template <class T, uint32_t KT>
+size_t tile_smem(uint32_t live) {
+  return sizeof(TileBufs<T, KT>) +
+         (size_t)(__builtin_popcount(live & 15u) + ((live >> 16) & 1u)) * kLB * KT * sizeof(T);
+}
+
+// Conductances of the batch: a thread per (live linear receptor, neuron) folds
+// the delivered sums and the drive of all L steps, another per neuron the NMDA
+// drive where there is any; four ring slots in flight (they are final: every
+// push into them happened before the interval began).  (Issuing an item's loads
+// before the drive draws hides them, 475 -> 300 cycles a step, but the registers
+// held meanwhile cost the draws, the pull and the membranes more.)
+template <class T>
+struct CondItem {
+  uint32_t q, k, r;
+  bool lin, ext;
+  T dfs, extg, G, est;
+  unsigned long long *ring;
+  long long nx[4];
+};
+template <class T>
+__device__ __forceinline__ uint32_t cond_items(const Params &P, uint32_t np) {
+  return (__popc(P.live & 15u) + ((P.live >> (8 + FS_NMDA)) & 1u)) * np;
+}
+template <class T>
+__device__ __forceinline__ void cond_load(const Params &P, uint32_t p0, uint32_t np, uint32_t sb, uint32_t L, uint32_t i,
+                                          CondItem<T> &I) {
+  const uint32_t n = P.n, nl = __popc(P.live & 15u);
+  I.k = i / np;
+  I.q = i - I.k * np;
+  if (I.k >= nl) return;
+  const uint32_t p = p0 + I.q;
+  uint32_t left = P.live & 15u;
+  for (uint32_t c = 0; c < I.k; c++) left &= left - 1u;
+  I.r = (uint32_t)__ffs(left) - 1u;
+  const int ri = P.lin_of_rec[I.r];
+  const size_t at = (size_t)I.r * n + p;
+  I.lin = ri >= 0;
+  I.ext = (P.live & (256u << I.r)) && (P.act[p] & act_of_rec(I.r));
+  I.dfs = (T)__ldg(P.dfst + at);
+  I.extg = (T)__ldg(P.ext_g + at);
+  I.G = ((T *)P.G)[at];
+  I.est = ((T *)P.ext_st)[at];
+  I.ring = I.lin ? ring_at(P, ri, p, 0) : nullptr;
 #pragma unroll
-  for (int r = 0; r < 4; r++) {
-    const int ri = P.lin_of_rec[r];
-    R.rv[r] = (ri >= 0 && own) ? (long long)__ldcg(ring_at(P, ri, p, tprev)) : 0ll;
-    R.rv2[r] = (PD == 2 && ri >= 0 && own && L > 1) ? (long long)__ldcg(ring_at(P, ri, p, tn)) : 0ll;
+  for (uint32_t u = 0; u < 4; u++)  // slot of step j: the deliveries of step t0 + sb + j - 1
+    I.nx[u] = I.lin && u < L ? (long long)__ldcg(I.ring + (size_t)(((uint32_t)P.t0 + sb - 1u + u) & P.mask) * n) : 0ll;
+}
+template <class T, uint32_t KT>
+__device__ __forceinline__ void cond_steps(const Params &P, uint32_t p0, uint32_t sb, uint32_t L, CondItem<T> &I,
+                                           T (*gn)[KT], const uint8_t (*hits)[KT],
+                                           T (*gl)[kLB][KT]) {
+  const uint32_t n = P.n, mask = P.mask, q = I.q, p = p0 + q;
+  if (I.k < __popc(P.live & 15u)) {
+    const uint32_t s0 = (uint32_t)P.t0 + sb - 1u, r = I.r;
+    T G = I.G, est = I.est;
+    for (uint32_t j0 = 0; j0 < L; j0 += 4) {
+      long long cur[4];
+#pragma unroll
+      for (uint32_t u = 0; u < 4; u++) {
+        cur[u] = I.nx[u];
+        I.nx[u] = I.lin && j0 + 4 + u < L ? (long long)__ldcg(I.ring + (size_t)((s0 + j0 + 4 + u) & mask) * n) : 0ll;
+      }
+#pragma unroll
+      for (uint32_t u = 0; u < 4; u++) {
+        const uint32_t j = j0 + u;
+        if (j >= L) break;
+        if (cur[u]) __stcg(I.ring + (size_t)((s0 + j) & mask) * n, 0ull);
+        T g = (T)0;
+        if (I.lin) g = G = fold_linear<T>(I.dfs, G, cur[u]);
+        const T e = drive_linear<T>(est, I.dfs, (hits[j][q] >> r) & 1u);
+        est = I.ext ? e : est;
+        gl[I.k][j][q] = I.ext ? fma_t<T>(I.extg, e, g) : g;
+      }
+    }
+    const size_t at = (size_t)r * n + p;
+    if (I.lin) ((T *)P.G)[at] = G;
+    if (I.ext) ((T *)P.ext_st)[at] = est;
+  } else if (P.act[p] & FS_ACT_NMDA) {
+    const size_t at = (size_t)FS_NMDA * n + p;
+    const T dfs = (T)__ldg(P.dfst + at), extg = (T)__ldg(P.ext_g + at), ndfxt = (T)__ldg(P.nmda_dfxt + p);
+    const T nefas = (T)__ldg(P.nmda_efst + p) * (T)__ldg(P.nmda_as + p);
+    T ex = ((T *)P.ext_x)[p], es = ((T *)P.ext_s)[p];
+    for (uint32_t j = 0; j < L; j++) {
+      drive_nmda<T>(ex, es, ndfxt, dfs, nefas, (hits[j][q] >> FS_NMDA) & 1u);
+      gn[j][q] = fma_t<T>(extg, es, gn[j][q] * (T)P.rg[FS_NMDA]);
+    }
+    ((T *)P.ext_x)[p] = ex;
+    ((T *)P.ext_s)[p] = es;
+  } else {
+    for (uint32_t j = 0; j < L; j++) gn[j][q] = gn[j][q] * (T)P.rg[FS_NMDA];
   }
 }
 
-// The L steps of neuron_load's neuron; tm3: the thread's Tsodyks-Markram
-// parameters (read every step from shared memory rather than from global
-// memory on the step's dependency chain).
-template <class T, int PD, bool kLTP = false>
-__device__ __forceinline__ void neuron_steps(const Params &P, uint32_t p0, uint32_t np, uint32_t sb, uint32_t L,
-                                             T (*gn)[TileW<T>::W], const uint8_t (*hits)[TileW<T>::W],
-                                             const T (*gauss)[TileW<T>::W], const SpikeList<T> &lst,
-                                             const T *gapI, StepRegs<T> &R, const float *tm3) {
-  const uint32_t tid = threadIdx.x, lane = tid & 31;
-  const uint32_t n = P.n, S = P.slots, mask = P.mask;
-  const bool own = tid < np;
-  const uint32_t p = own ? p0 + tid : p0;
-  NeuronPar<T> &q = R.q;
-  NeuronState<T> &st = R.st;
-  long long(&rv)[4] = R.rv, (&rv2)[4] = R.rv2;
-  uint32_t nsp = 0;
+// step_pre's state changes over the batch's L steps (bit j of mask: a spike at
+// step j) of a network with Tsodyks-Markram plasticity (kTM) or none: the
+// increments' chain, then each linear gate's, then x and s.
+template <class T, bool kTM, bool kKeepS, uint32_t KT>
+__device__ __forceinline__ void pre_batch(const Params &P, const NeuronPar<T> &N, NeuronState<T> &st, uint32_t mask,
+                                          uint32_t L, T (*gn)[KT], uint32_t q, const float (&tm)[3]) {
+  const bool on_tm = kTM && (N.pj & kPjTM);
+  T sp[4] = {st.sp[0], st.sp[1], st.sp[2], st.sp[3]}, x = st.xp, y = st.spre;
+  float tmu = st.tmu, tmx = st.tmx;
+  const uint32_t lin = (P.lin_of_rec[0] >= 0 ? 1u : 0u) | (P.lin_of_rec[1] >= 0 ? 2u : 0u) |
+                       (P.lin_of_rec[2] >= 0 ? 4u : 0u) | (P.lin_of_rec[3] >= 0 ? 8u : 0u);
+  auto run = [&](auto rc) {  // rc: linear receptors that can be in use, as a compile-time mask
+    constexpr uint32_t R = decltype(rc)::value;
+#pragma unroll 2
+    for (uint32_t j = 0; j < L; j++) {
+      const bool spk = (mask >> j) & 1u;
+      T inc = (T)1;
+      if constexpr (kTM) {
+        const T u = (T)tmu, v = (T)tmx, U = (T)tm[0];
+        const T us = fma_t<T>(U, (T)1 - u, u), rel = us * v;
+        const T ud = fma_t<T>(u - U, (T)tm[1], U), vd = fma_t<T>(v - (T)1, (T)tm[2], (T)1);
+        inc = on_tm ? rel : inc;
+        tmu = (float)(spk ? us : ud);
+        tmx = (float)(spk ? v - rel : vd);
+      }
+#pragma unroll
+      for (int r = 0; r < 4; r++)
+        if (R & (1u << r)) sp[r] = spk ? sp[r] + inc : sp[r] * N.pdf[r];
+      nmda_pre_step<T>(x, y, spk, inc, N.pdfxt, N.pdfst, N.pefas);
+      if (kKeepS) gn[j][q] = y;
+    }
+  };
+  if ((lin & ~3u) == 0) run(std::integral_constant<uint32_t, 3u>());
+  else run(std::integral_constant<uint32_t, 15u>());
+#pragma unroll
+  for (int r = 0; r < 4; r++)
+    if (N.pj & (1u << r)) st.sp[r] = sp[r];
+  if (N.pj & (1u << FS_NMDA)) {
+    st.xp = x;
+    st.spre = y;
+  }
+  if (on_tm) {
+    st.tmu = tmu;
+    st.tmx = tmx;
+  }
+}
+
+// Membrane and presynaptic state of the batch, a thread per neuron: the
+// membrane's L steps first (the spikes as a bit mask), then the presynaptic
+// part with the spike outputs and the list of spikes that the block pushes at
+// the end of the batch (a push lands >= min_delay steps ahead, so it may wait
+// until the interval's end; past the list's room a thread pushes its spike
+// itself).  kKeepS: the s values of the batch are left in gn for
+// store_history.
+template <class T, bool kLTP, bool kKeepS, uint32_t KT>
+__device__ __forceinline__ void tile_neurons(const Params &P, uint32_t p0, uint32_t np, uint32_t sb, uint32_t L,
+                                             T (*gn)[KT], const T (*gl)[kLB][KT],
+                                             const T (*gauss)[KT], const SpikeList<T> &lst, const T *gapI) {
+  const uint32_t n = P.n, q = threadIdx.x;
+  if (q >= np) return;
+  const uint32_t p = p0 + q;
+  NeuronPar<T> N;
+  NeuronState<T> st;
+  load_membrane<T>(P, p, N, st);
+  if (kLTP) load_pre<T>(P, p, N, st);  // one step: its latency would not hide
   LtpTrace<T> lt;
   if constexpr (kLTP) {
     lt.lp = ((float *)P.ltp_lp)[p];
@@ -930,117 +1277,114 @@ __device__ __forceinline__ void neuron_steps(const Params &P, uint32_t p0, uint3
     lt.dflp = __ldg(P.ltp_dflp + p);
     lt.spd = __ldg(P.ltp_spd + p);
   }
+  const uint32_t l0 = P.live & 1u, l1 = l0 + ((P.live >> 1) & 1u), l2 = l1 + ((P.live >> 2) & 1u);  // rows of gl
+  const bool raw = !((P.live >> (8 + FS_NMDA)) & 1u);  // gn holds the bare sums
+  const T gap = P.gap_row ? gapI[q] : (T)0;
+  uint32_t mask = 0;
   for (uint32_t j = 0; j < L; j++) {
-    const uint32_t s = sb + j;
-    const uint64_t t = P.t0 + s;
-    const uint32_t tm = (uint32_t)t & mask, tprev = (uint32_t)(t - 1u) & mask;
-    // the slots this step folds in; the ones of step j + PD go in flight
-    long long cur[4];
+    T g[5];
+    if (P.live & 1u) g[0] = gl[0][j][q];
+    if (P.live & 2u) g[1] = gl[l0][j][q];
+    if (P.live & 4u) g[2] = gl[l1][j][q];
+    if (P.live & 8u) g[3] = gl[l2][j][q];
+    g[FS_NMDA] = raw ? gn[j][q] * (T)P.rg[FS_NMDA] : gn[j][q];
+    if (step_membrane<T, kLTP>(P, N, st, g, gauss ? gauss[j][q] : (T)0, gap, p, true, sb + j, &lt)) mask |= 1u << j;
+  }
+  store_membrane<T>(P, p, st);
+  if (P.gap_row) ((T *)P.Vg)[(size_t)((P.t0 + sb) & 1u) * n + p] = st.V;
+  if (!kLTP) load_pre<T>(P, p, N, st);  // (held through the membranes' steps, its registers cost more)
+  float tm[3] = {0.0f, 0.0f, 0.0f};
+  if (N.pj & kPjTM) {
+    tm[0] = __ldg(P.tm_U + p);
+    tm[1] = __ldg(P.tm_dff + p);
+    tm[2] = __ldg(P.tm_dfr + p);
+  }
+  // the spike outputs and list entries of step j
+  auto emit = [&](uint32_t j, const T (&cinc)[4]) {
+    const uint32_t s = sb + j, t = (uint32_t)P.t0 + s;
+    if (P.bits) atomicOr(P.bits + (size_t)s * P.words + (p >> 5), 1u << (p & 31));
+    if (P.counts) atomicAdd(P.counts + s, 1u);
+    const uint32_t k = atomicAdd(lst.n, 1u);
+    if (k < lst.cap) {
+      lst.p[k] = p;
+      lst.tm[k] = (uint16_t)(t & P.mask);
 #pragma unroll
-    for (int r = 0; r < 4; r++) {
-      cur[r] = rv[r];
-      const int ri = P.lin_of_rec[r];
-      if (ri >= 0) {
-        if (own && rv[r]) __stcg(ring_at(P, ri, p, tprev), 0ull);
-        if constexpr (PD == 2) {
-          rv[r] = rv2[r];
-          rv2[r] = (own && j + 2 < L) ? (long long)__ldcg(ring_at(P, ri, p, (tm + 1u) & mask)) : 0ll;
-        } else {
-          rv[r] = (own && j + 1 < L) ? (long long)__ldcg(ring_at(P, ri, p, tm)) : 0ll;
-        }
+      for (int r = 0; r < 4; r++) lst.c[k][r] = cinc[r];
+    } else {
+      push_spike<T>(P, p, t & P.mask, cinc, 0, 1);
+    }
+  };
+  if (!kLTP && !P.gv_row && (P.plast == PL_NONE || P.plast == PL_TM)) {
+    // the state alone first, without branches; the few neurons that spiked go
+    // through their steps again for the spikes' increments
+    const NeuronState<T> was = st;
+    if (P.plast == PL_TM) pre_batch<T, true, kKeepS, KT>(P, N, st, mask, L, gn, q, tm);
+    else pre_batch<T, false, kKeepS, KT>(P, N, st, mask, L, gn, q, tm);
+    if (mask) {
+      NeuronState<T> a = was;
+      for (uint32_t j = 0; j < L && (mask >> j); j++) {
+        T cinc[4], inc;
+        step_pre<T>(P, N, a, (mask >> j) & 1u, p, true, cinc, inc, tm);
+        if ((mask >> j) & 1u) emit(j, cinc);
       }
     }
-    const uint32_t qs = tid < np ? tid : 0;
-    T cinc[4], inc;
-    const bool spk = neuron_step<T, true, kLTP>(P, q, st, cur, gn[j][qs], hits[j][qs], gauss[j][qs],
-                                                P.gap_row ? gapI[qs] : (T)0, p, own, s, cinc, inc, tm3 + 3 * tid,
-                                                &lt);
-    nsp += spk ? 1u : 0u;
-    if constexpr (kLTP) {
-      // what the LTP phase of this step reads while the owners run the next
-      if (own) {
-        const uint32_t par = (uint32_t)t & 1u;
+  } else {
+    for (uint32_t j = 0; j < L; j++) {
+      const bool spk = (mask >> j) & 1u;
+      T cinc[4], inc;
+      step_pre<T>(P, N, st, spk, p, true, cinc, inc, tm);
+      if (kKeepS) gn[j][q] = st.spre;
+      if constexpr (kLTP) {
+        // what the LTP phase of this step reads while the owners run the next
+        const uint32_t par = ((uint32_t)P.t0 + sb + j) & 1u;
         ((float *)P.ltp_lp2)[(size_t)par * n + p] = lt.lp;
         P.ltp_spk2[(size_t)par * n + p] = spk ? 1 : 0;
 #pragma unroll
-        for (int r = 0; r < 4; r++) ((T *)P.ltp_sp2)[((size_t)par * 4 + r) * n + p] = st.sp[r];
+        for (int r = 0; r < 4; r++)
+          if (P.lin_of_rec[r] >= 0) ((T *)P.ltp_sp2)[((size_t)par * 4 + r) * n + p] = st.sp[r];
       }
-    }
-    if (own && P.gv_row) gv_write<T>(P, p, s, st);
-    if (own && (q.pj & (1u << FS_NMDA))) {
-      if constexpr (sizeof(T) == 4) {
-#pragma unroll
-        for (uint32_t k = 0; k < kSH; k++)
-          __stcg((T *)P.s_hist + ((size_t)p * kSH + k) * S + ((tm - k) & mask), st.spre);
-      } else {
-        __stcg((T *)P.s_hist + (size_t)p * S + tm, st.spre);
-      }
-    }
-    // spikes of this warp: outputs, and the spike list the block pushes at
-    // the end of the batch (a push lands >= min_delay steps ahead, so it may
-    // wait until the interval's end); a full list falls back to a push by
-    // this warp right away
-    uint32_t m = __ballot_sync(fsd::kFull, spk);
-    if (m) {
-      spike_outputs(P, m, spk, p, s, lane);
-      bool listed = false;
-      if (spk) {
-        const uint32_t k = atomicAdd(lst.n, 1u);
-        if (k < lst.cap) {
-          lst.p[k] = p;
-          lst.tm[k] = (uint16_t)tm;
-#pragma unroll
-          for (int r = 0; r < 4; r++) lst.c[k][r] = cinc[r];
-          listed = true;
-        }
-      }
-      uint32_t over = __ballot_sync(fsd::kFull, spk && !listed);
-      while (over) {
-        const int jl = __ffs(over) - 1;
-        over &= over - 1;
-        const uint32_t qq = __shfl_sync(fsd::kFull, p, jl);
-        T cj[4];
-#pragma unroll
-        for (int r = 0; r < 4; r++) cj[r] = __shfl_sync(fsd::kFull, cinc[r], jl);
-        push_spike<T>(P, qq, tm, cj, lane, 32);
-      }
+      if (P.gv_row) gv_write<T>(P, p, sb + j, st);
+      if (spk) emit(j, cinc);
     }
   }
-  if (own) {
-    store_neuron<T>(P, p, q, st);
-    if (P.gap_row) ((T *)P.Vg)[(size_t)((P.t0 + sb) & 1u) * n + p] = st.V;
-    if (P.nspk && nsp) P.nspk[p] += nsp;
-    if constexpr (kLTP) {
-      ((float *)P.ltp_lp)[p] = lt.lp;
-      P.ltp_clp[p] = lt.clp;
-    }
+  store_pre<T>(P, p, N, st);
+  if (mask) {
+    atomicAdd(P.spike_total, (unsigned long long)__popc(mask));
+    if (P.nspk) P.nspk[p] += __popc(mask);
+  }
+  if constexpr (kLTP) {
+    ((float *)P.ltp_lp)[p] = lt.lp;
+    P.ltp_clp[p] = lt.clp;
   }
 }
 
-// Shared-memory buffers of one tile (the posts a block advances together).
-template <class T>
-struct TileBufs {
-  static constexpr uint32_t kT = TileW<T>::W;
-  static constexpr uint32_t kCap = sizeof(T) == 4 ? 320 : 192;
-  T gn[kLB][kT];
-  T gauss[kLB][kT];
-  T gapI[kT];
-  uint8_t hits[kLB][kT];
-  uint32_t l_n, l_p[kCap];
-  uint16_t l_tm[kCap];
-  T l_c[kCap][4];
-};
+// The s values of a batch of L steps (tile_neurons leaves them in gn) into the
+// history, by the whole block; FP32: the shifted rows.
+template <class T, uint32_t KT>
+__device__ __forceinline__ void store_history(const Params &P, uint32_t p0, uint32_t np, uint64_t tb, uint32_t L,
+                                              const T (*gn)[KT]) {
+  // thread: step j of the batch, row k of neurons q, q + 16 / K, ... (a neuron
+  // that projects on no NMDA receptor stores its zeros, which nothing reads)
+  constexpr uint32_t K = sizeof(T) == 4 ? kSH : 1u;
+  static_assert(kLB == 16 && kThreads % (16 * K) == 0, "a thread's step and row are fixed");
+  const uint32_t S = P.slots, j = threadIdx.x & 15u, k = (threadIdx.x >> 4) & (K - 1u);
+  if (j >= L) return;
+  const T *src = gn[j];
+  T *dst = (T *)P.s_hist + ((size_t)p0 * K + k) * S + (((uint32_t)tb + j - k) & P.mask);
+#pragma unroll 4
+  for (uint32_t q = threadIdx.x / (16 * K); q < np; q += kThreads / (16 * K)) __stcg(dst + (size_t)q * K * S, src[q]);
+}
 
 // NMDA sums of L steps for a tile's posts into B.gn.
-template <class T, int PU>
+template <class T, int PU, uint32_t KT>
 __device__ __forceinline__ void tile_pull(const Params &P, uint32_t tp0, uint32_t np, uint32_t bs, uint32_t L,
-                                          TileBufs<T> &B) {
+                                          TileBufs<T, KT> &B) {
   const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   if constexpr (sizeof(T) == 4) {
-    if (P.dmax0) nmda_pull1_f32(P, tp0, np, P.t0 + bs, (float (*)[kTile])B.gn, wid, lane);
-    else nmda_pull_f32<PU>(P, tp0, np, P.t0 + bs, L, (float (*)[kTile])B.gn, wid, lane);
+    if (P.dmax0) nmda_pull1_f32<false, false, KT>(P, tp0, np, P.t0 + bs, (float (*)[KT])B.gn, wid, lane);
+    else nmda_pull_f32<PU, KT>(P, tp0, np, P.t0 + bs, L, (float (*)[KT])B.gn, wid, lane);
   } else {
-    nmda_pull<T>(P, tp0, np, P.t0 + bs, L, B.gn, wid, lane);
+    nmda_pull<T, KT>(P, tp0, np, P.t0 + bs, L, B.gn, wid, lane);
   }
 }
 
@@ -1063,25 +1407,41 @@ __device__ __forceinline__ void tile_gap(const Params &P, uint32_t tp0, uint32_t
 }
 
 // The rest of a tile's batch of L steps once its NMDA sums are in B.gn: the
-// drive draws, gap currents, the neurons' steps and the spikes' pushes.
-template <class T, int PD>
+// drive draws, gap currents, the neurons' steps and the spikes' pushes.  What
+// bounds the steps is the chain of one neuron's dependent operations, not
+// their number: with a thread per neuron and everything in one loop, 3 of 8
+// warps had work (68 posts a block) and a step took 2,470 cycles.  The
+// conductances of a batch depend on nothing of it but the draws and finished
+// deliveries, so they are made first, by a thread per neuron and receptor;
+// what remains a chain is the membrane.  The history's rows (four of L values
+// a neuron, 4-byte stores 256 bytes apart from the neuron's own thread) are
+// written by the whole block in runs of L.  On the 20k connectome (cycles a
+// step): draws 270, conductances 400, loads and membranes 670, presynaptic
+// state 280, history and pushes 290; with the barrier 4.06 -> 3.88 us a step.
+// The 200k network's tile kernels (more posts than threads to start with)
+// gain from the shorter inner loops: 34.2 -> 30.8 us a step.
+template <class T, uint32_t KT>
 __device__ __forceinline__ void tile_steps(const Params &P, uint32_t tp0, uint32_t np, uint32_t bs, uint32_t L,
-                                           TileBufs<T> &B, PhaseClock &pc) {
-  constexpr uint32_t kCap = TileBufs<T>::kCap;
+                                           TileBufs<T, KT> &B, PhaseClock &pc, bool hist) {
+  constexpr uint32_t kCap = TileBufs<T, KT>::kCap;
   const SpikeList<T> lst{&B.l_n, B.l_p, B.l_tm, B.l_c, kCap};
   const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  // warps without neurons in this tile skip the steps
-  const bool act = (tid & ~31u) < np;
-  __shared__ float tm3[kThreads * 3];
-  StepRegs<T> R;
-  draw_inputs<T>(P, tp0, np, P.t0 + bs, L, B.hits, B.gauss);
+  const uint32_t items = cond_items<T>(P, np);
+  draw_inputs<T, KT>(P, tp0, np, P.t0 + bs, L, B.hits, B.gauss(P));
   if (P.gap_row) tile_gap<T>(P, tp0, np, bs, B.gapI);
   __syncthreads();
   pc.mark(1);
-  if (act) neuron_load<T, PD>(P, tp0, np, bs, L, R, tm3);
-  if (act) neuron_steps<T, PD>(P, tp0, np, bs, L, B.gn, B.hits, B.gauss, lst, B.gapI, R, tm3);
+  for (uint32_t i = tid; i < items; i += kThreads) {
+    CondItem<T> I;
+    cond_load<T>(P, tp0, np, bs, L, i, I);
+    cond_steps<T, KT>(P, tp0, bs, L, I, B.gn, B.hits, B.lin());
+  }
+  __syncthreads();
+  pc.mark(9);
+  tile_neurons<T, false, true, KT>(P, tp0, np, bs, L, B.gn, B.lin(), B.gauss(P), lst, B.gapI);
   __syncthreads();
   pc.mark(2);
+  if (hist) store_history<T, KT>(P, tp0, np, P.t0 + bs, L, B.gn);
   // the batch's spikes: with fewer spikes than warps the whole block
   // walks each spike's out-edges (a hub's hundreds of edges in one or
   // two rounds); with more, one spike per warp, eight in flight
@@ -1108,12 +1468,12 @@ __device__ __forceinline__ void tile_steps(const Params &P, uint32_t tp0, uint32
 
 // The steps of one block: posts [B0, B1) of the network P, whose blocks
 // (nblk of them) meet at a barrier after every interval.  PU: NMDA edges in
-// flight per lane in the pull; PD: ring slots in flight per neuron in the
-// steps (results depend on neither).
-template <class T, int PU, int PD>
+// flight per lane in the pull (results do not depend on it).
+template <class T, int PU, uint32_t KT>
 __device__ __forceinline__ void prod_blocks(const Params &P, uint32_t B0, uint32_t B1, uint32_t nblk) {
-  constexpr uint32_t kT = TileW<T>::W;
-  __shared__ TileBufs<T> B;
+  constexpr uint32_t kT = KT;
+  extern __shared__ __align__(16) unsigned char smt[];
+  TileBufs<T, KT> &B = *(TileBufs<T, KT> *)smt;
   PhaseClock pc;
   pc.start(P);
   unsigned long long target = 0;  // barrier arrivals so far (thread 0)
@@ -1126,9 +1486,9 @@ __device__ __forceinline__ void prod_blocks(const Params &P, uint32_t B0, uint32
       const uint32_t L = min(kLB, iv_end - bs);
       for (uint32_t tp0 = B0; tp0 < B1; tp0 += kT) {
         const uint32_t np = min(kT, B1 - tp0);
-        tile_pull<T, PU>(P, tp0, np, bs, L, B);
+        tile_pull<T, PU, KT>(P, tp0, np, bs, L, B);
         pc.mark(0);
-        tile_steps<T, PD>(P, tp0, np, bs, L, B, pc);
+        tile_steps<T, KT>(P, tp0, np, bs, L, B, pc, P.in_row != nullptr);
       }
     }
     s = iv_end;
@@ -1145,9 +1505,9 @@ __device__ __forceinline__ void prod_blocks(const Params &P, uint32_t B0, uint32
 // they span several (250k network: 43.3 against 46.3 us); ring slots two
 // steps ahead (4.60 us with one).  Batches of small networks run eight edges
 // and one step ahead (their kernel has fewer registers to spare).
-template <class T, int PU>
+template <class T, int PU, uint32_t KT>
 __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1) k_prod(const __grid_constant__ Params P) {
-  prod_blocks<T, PU, 2>(P, P.block_post[blockIdx.x], P.block_post[blockIdx.x + 1], gridDim.x);
+  prod_blocks<T, PU, KT>(P, P.block_post[blockIdx.x], P.block_post[blockIdx.x + 1], gridDim.x);
 }
 
 // ---- long-term plasticity (networks with LTP, delays 0) ---------------------
@@ -1270,11 +1630,11 @@ __device__ __forceinline__ void ltp_phase(const Params &P, const uint32_t *ids, 
 // nothing), the pushes and the LTP of step t1 - 1.  So between launches the
 // weights are those after the last step's LTP, as the reference's are, and
 // nothing else is pending.
-template <class T>
+template <class T, uint32_t KT>
 __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1) k_prod_ltp(const __grid_constant__ Params P) {
-  constexpr uint32_t kT = TileW<T>::W;
-  __shared__ TileBufs<T> B;
-  __shared__ float tm3[kThreads * 3];
+  constexpr uint32_t kT = KT;
+  extern __shared__ __align__(16) unsigned char smt[];
+  TileBufs<T, KT> &B = *(TileBufs<T, KT> *)smt;
   const uint32_t B0 = P.block_post[blockIdx.x], B1 = P.block_post[blockIdx.x + 1];
   const uint32_t nblk = gridDim.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const uint32_t gw = blockIdx.x * (kThreads / 32) + wid, nwarps = nblk * (kThreads / 32);
@@ -1289,8 +1649,8 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1) k_prod_ltp(c
       for (uint32_t tp0 = B0; tp0 < B1; tp0 += kT) {
         const uint32_t np = min(kT, B1 - tp0);
         T(*gn)[kT] = (T(*)[kT])((T *)P.ltp_gn + tp0);
-        if constexpr (sizeof(T) == 4) nmda_pull1_f32<true>(P, tp0, np, t, (float(*)[kTile])gn, wid, lane);
-        else nmda_pull<T, true>(P, tp0, np, t, 1, gn, wid, lane);
+        if constexpr (sizeof(T) == 4) nmda_pull1_f32<true, true, KT>(P, tp0, np, t, (float(*)[KT])gn, wid, lane);
+        else nmda_pull1_f64<true>(P, tp0, np, (double *)gn[0], wid, lane);
       }
       pc.mark(0);
     }
@@ -1322,16 +1682,19 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1) k_prod_ltp(c
                            (T(*)[4])((T *)P.ltp_c + (size_t)par * n * 4), n};
     for (uint32_t tp0 = B0; tp0 < B1; tp0 += kT) {
       const uint32_t np = min(kT, B1 - tp0);
-      draw_inputs<T>(P, tp0, np, t, 1, B.hits, B.gauss);
+      T(*gn)[kT] = (T(*)[kT])((T *)P.ltp_gn + tp0);
+      const uint32_t items = cond_items<T>(P, np);
+      draw_inputs<T, KT>(P, tp0, np, t, 1, B.hits, B.gauss(P));
       if (P.gap_row) tile_gap<T>(P, tp0, np, s, B.gapI);
       __syncthreads();
       pc.mark(1);
-      if ((tid & ~31u) < np) {
-        StepRegs<T> R;
-        neuron_load<T, 1>(P, tp0, np, s, 1, R, tm3);
-        neuron_steps<T, 1, true>(P, tp0, np, s, 1, (T(*)[kT])((T *)P.ltp_gn + tp0), B.hits, B.gauss, lst, B.gapI, R,
-                                 tm3);
+      for (uint32_t i = tid; i < items; i += kThreads) {
+        CondItem<T> I;
+        cond_load<T>(P, tp0, np, s, 1, i, I);
+        cond_steps<T, KT>(P, tp0, s, 1, I, gn, B.hits, B.lin());
       }
+      __syncthreads();
+      tile_neurons<T, true, false, KT>(P, tp0, np, s, 1, gn, B.lin(), B.gauss(P), lst, B.gapI);
       __syncthreads();
       pc.mark(2);
     }
@@ -1784,10 +2147,11 @@ __global__ void __launch_bounds__(kThreads, U == 4 ? 4 : 2) k_tile_pull(const Pa
   const Params &P = Psh;
   const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   if constexpr (sizeof(T) == 4) {
-    if (P.dmax0) nmda_pull1_f32(P, tl.p0, tl.np, P.t0 + bs, (float (*)[kTile])gn, wid, lane);
-    else nmda_pull_f32<U>(P, tl.p0, tl.np, P.t0 + bs, L, (float (*)[kTile])gn, wid, lane);
+    if (P.dmax0) nmda_pull1_f32<false, true, TileW<T>::W>(P, tl.p0, tl.np, P.t0 + bs, (float (*)[TileW<T>::W])gn, wid, lane);
+    else nmda_pull_f32<U, TileW<T>::W>(P, tl.p0, tl.np, P.t0 + bs, L, (float (*)[TileW<T>::W])gn, wid, lane);
   } else {
-    nmda_pull<T>(P, tl.p0, tl.np, P.t0 + bs, L, gn, wid, lane);
+    if (P.dmax0) nmda_pull1_f64<false>(P, tl.p0, tl.np, (double *)gn[0], wid, lane);
+    else nmda_pull<T, TileW<T>::W>(P, tl.p0, tl.np, P.t0 + bs, L, gn, wid, lane);
   }
   __syncthreads();
   T *out = (T *)P.gn_buf;
@@ -1797,12 +2161,13 @@ __global__ void __launch_bounds__(kThreads, U == 4 ? 4 : 2) k_tile_pull(const Pa
   }
 }
 
-template <class T, int PD>
-__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1) k_tile_step(const Params *__restrict__ Ps,
+template <class T>
+__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 3 : 1) k_tile_step(const Params *__restrict__ Ps,
                                                                               const IvTile *__restrict__ tiles,
                                                                               uint32_t bs, uint32_t L) {
   __shared__ __align__(16) Params Psh;
-  __shared__ TileBufs<T> B;
+  extern __shared__ __align__(16) unsigned char smt[];
+  TileBufs<T, TileW<T>::W> &B = *(TileBufs<T, TileW<T>::W> *)smt;
   const IvTile tl = tiles[blockIdx.x];
   params_to_smem(Psh, Ps, tl.inst);
   if (threadIdx.x == 0) B.l_n = 0;
@@ -1815,7 +2180,9 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1) k_tile_step(
   }
   PhaseClock pc;
   pc.out = nullptr;
-  tile_steps<T, PD>(P, tl.p0, tl.np, bs, L, B, pc);  // its first barrier orders the loads above
+  // (its first barrier orders the loads above; the pull of networks without
+  // delays reads s_pre)
+  tile_steps<T, TileW<T>::W>(P, tl.p0, tl.np, bs, L, B, pc, P.in_row != nullptr && !P.dmax0);
 }
 
 
@@ -1861,6 +2228,12 @@ struct Prod {
   float *gv_st = nullptr, *gv_xt = nullptr;
   uint64_t gv_out_cap = 0;
   uint32_t gv_ent_cap = 0;
+  // drive receptors: with a positive probability now, at any step since the
+  // reset; parameters finite (else every receptor counts as live)
+  uint32_t pb_live = 0, ext_live = 0;
+  bool inj = false;  // some neuron has injection
+  uint32_t max_posts = 0;  // of a persistent kernel's block
+  bool finite = true;
   std::vector<uint32_t> in_row_h;  // NMDA in-degree prefix (block partitioning)
   // networks with LTP: where each synapse-list entry's weight lives (index
   // in out_w, or in in_w with the top bit set)
@@ -1894,6 +2267,67 @@ int dup(Prod *p, X **ptr, const X *src, size_t count, cudaStream_t st, std::stri
     return FS_ERR_CUDA;
   }
   return FS_OK;
+}
+
+uint32_t drive_mask(const float *pb, size_t n) {
+  uint32_t m = 0;
+  for (uint32_t r = 0; r < FS_NREC; r++)
+    for (size_t i = 0; i < n; i++)
+      if (pb[r * n + i] > 0.0f) {
+        m |= 1u << r;
+        break;
+      }
+  return m;
+}
+constexpr uint32_t kLiveAll = 0x11f0fu;
+
+// The persistent kernel of a network: tiles as narrow as its blocks allow (a
+// tile's shared memory is L1 that the pull's windows lose), eight NMDA edges in
+// flight where blocks span several tiles.
+const void *prod_kernel(const Prod *p) {
+  if (p->fp64) return p->max_posts <= 64 ? (const void *)k_prod<double, 4, 64> : (const void *)k_prod<double, 4, 128>;
+  if (p->wide) return (const void *)k_prod<float, 8, 256>;
+  return p->max_posts <= 128 ? (const void *)k_prod<float, 4, 128> : (const void *)k_prod<float, 4, 256>;
+}
+const void *ltp_kernel(const Prod *p) {
+  if (p->fp64) return (const void *)k_prod_ltp<double, 128>;
+  return p->max_posts <= 128 ? (const void *)k_prod_ltp<float, 128> : (const void *)k_prod_ltp<float, 256>;
+}
+// Dynamic shared memory of that kernel.
+size_t prod_smem(const Prod *p, uint32_t live) {
+  if (p->fp64)
+    return !p->ltp && p->max_posts <= 64 ? tile_smem<double, 64>(live) : tile_smem<double, 128>(live);
+  return p->max_posts <= 128 ? tile_smem<float, 128>(live) : tile_smem<float, 256>(live);
+}
+
+// The kernels' dynamic shared memory limit (per kernel, not per handle).
+void tile_attributes() {
+  const int f = (int)tile_smem<float, 256>(kLiveAll), d = (int)tile_smem<double, 128>(kLiveAll);
+  for (const void *k : {(const void *)k_prod<float, 4, 128>, (const void *)k_prod<float, 4, 256>,
+                        (const void *)k_prod<float, 8, 256>, (const void *)k_prod_ltp<float, 128>,
+                        (const void *)k_prod_ltp<float, 256>, (const void *)k_tile_step<float>})
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, f);
+  for (const void *k : {(const void *)k_prod<double, 4, 64>, (const void *)k_prod<double, 4, 128>,
+                        (const void *)k_prod_ltp<double, 128>, (const void *)k_tile_step<double>})
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, d);
+}
+
+// Params::live after a change of the drive.
+void set_live(Prod *p) {
+  uint32_t live = p->ext_live << 8;
+  for (int r = 0; r < 4; r++)
+    if (p->P.lin_of_rec[r] >= 0 || (p->ext_live & (1u << r))) live |= 1u << r;
+  p->P.live = (p->finite ? live : 0x1f0fu) | (p->inj ? 0x10000u : 0u);
+}
+bool any_injection(const uint32_t *act, size_t n) {
+  for (size_t i = 0; act && i < n; i++)
+    if (act[i] & FS_ACT_INJ) return true;
+  return false;
+}
+void drive_changed(Prod *p, const float *pb) {
+  p->pb_live = drive_mask(pb, p->n);
+  p->ext_live |= p->pb_live;
+  set_live(p);
 }
 
 int ensure_buffers(Prod *p, uint32_t steps, bool wantV, bool wantI, bool wantNS, std::string &err) {
@@ -1994,20 +2428,17 @@ int launch(Prod *p, uint32_t nsteps, bool want_bits, bool wantV, cudaStream_t st
     if (launches) *launches += k;
     return FS_OK;
   }
+  const size_t smem = prod_smem(p, P.live);
   if (p->ltp) {
     // both spike lists start empty (a launch leaves none pending)
     e = cudaMemsetAsync(P.ltp_cnt, 0, 8, st);
     if (e == cudaSuccess)
-      e = cudaLaunchCooperativeKernel(p->fp64 ? (const void *)k_prod_ltp<double> : (const void *)k_prod_ltp<float>,
-                                      p->blocks, kThreads, args, 0, st);
+      e = cudaLaunchCooperativeKernel(ltp_kernel(p), p->blocks, kThreads, args, smem, st);
   } else if (p->single) {
     const void *k1 = P.plast == PL_TM ? (const void *)k_prod1<true> : (const void *)k_prod1<false>;
     e = cudaLaunchCooperativeKernel(k1, p->b1_blocks, kT1, args, P.t1_smem, st);
   } else {
-    // (the FP64 pull does not take the edges-in-flight parameter)
-    const void *k = p->fp64 ? (const void *)k_prod<double, 4>
-                            : (p->wide ? (const void *)k_prod<float, 8> : (const void *)k_prod<float, 4>);
-    e = cudaLaunchCooperativeKernel(k, p->blocks, kThreads, args, 0, st);
+    e = cudaLaunchCooperativeKernel(prod_kernel(p), p->blocks, kThreads, args, smem, st);
   }
   cudaEventRecord(evp.second, st);
   if (e != cudaSuccess) {
@@ -2713,12 +3144,24 @@ static int prod_create_from(Prod **out, const fs_net_desc *d, const fs_run_opts 
   p->nlin = H.nlin;
   for (int r = 0; r < 4; r++) P.lin_of_rec[r] = H.lin_of_rec[r];
   P.nlin = p->nlin;
+  if (v.pb) p->pb_live = p->ext_live = drive_mask(v.pb, n);
+  for (const auto &a : {std::pair<const float *, size_t>{v.ext_g, nr}, {v.Vrev, nr}, {v.dfst, nr}, {v.nmda_dfxt, n},
+                        {v.nmda_efst, n}, {v.nmda_as, n}, {v.dVmax, n}, {v.df, n}, {v.ef, n}})
+    if (a.first) {
+      float z = 0.0f;  // 0 * x is 0 for a finite x, else NaN
+      for (size_t i = 0; i < a.second; i++) z += 0.0f * a.first[i];
+      if (!(z == 0.0f)) p->finite = false;
+    }
+  p->inj = any_injection(v.act, n);
+  set_live(p);
   // ---- grid: all blocks co-resident; posts split by estimated cost ----
   int occ = 0;
   {
-    const void *kq = ltp ? (p->fp64 ? (const void *)k_prod_ltp<double> : (const void *)k_prod_ltp<float>)
-                         : (p->fp64 ? (const void *)k_prod<double, 4> : (const void *)k_prod<float, 4>);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kq, kThreads, 0);
+    const void *kq = ltp ? (p->fp64 ? (const void *)k_prod_ltp<double, 128> : (const void *)k_prod_ltp<float, 256>)
+                         : (p->fp64 ? (const void *)k_prod<double, 4, 128> : (const void *)k_prod<float, 4, 256>);
+    // (at the largest shared memory a change of the drive can ask for)
+    tile_attributes();
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kq, kThreads, p->fp64 ? tile_smem<double, 128>(kLiveAll) : tile_smem<float, 256>(kLiveAll));
   }
   if (occ < 1) occ = 1;
   int per_sm = std::min(occ, 4);
@@ -2741,8 +3184,8 @@ static int prod_create_from(Prod **out, const fs_net_desc *d, const fs_run_opts 
     for (; b < blocks; b++) block_post[b] = n;
   }
   p->chunks = blocks;
-  for (uint32_t b = 0; b < blocks; b++)
-    if (block_post[b + 1] - block_post[b] > kTile) p->wide = true;
+  for (uint32_t b = 0; b < blocks; b++) p->max_posts = std::max(p->max_posts, block_post[b + 1] - block_post[b]);
+  p->wide = p->max_posts > kTile;
   p->in_row_h = in_row;
   // ---- device arrays ----
   int rc = 0;
@@ -2916,6 +3359,8 @@ void prod_destroy(Prod *p) {
 int prod_upload_params(Prod *p, const float *pb, const uint32_t *act, const float *inj_mean, const float *inj_std,
                        cudaStream_t st, std::string &err) {
   const size_t n = p->n;
+  p->inj = any_injection(act, n);
+  drive_changed(p, pb);
   cudaError_t e = cudaMemcpyAsync((void *)p->P.pb, pb, FS_NREC * n * 4, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync((void *)p->P.act, act, n * 4, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync((void *)p->P.inj_mean, inj_mean, n * 4, cudaMemcpyHostToDevice, st);
@@ -2969,6 +3414,8 @@ int prod_reset(Prod *p, uint32_t seed, cudaStream_t st, std::string &err) {
     return FS_ERR_CUDA;
   }
   // stream key: user key and the run seed
+  p->ext_live = p->pb_live;
+  set_live(p);
   P.key0 = (uint32_t)p->key ^ seed;
   P.key1 = (uint32_t)(p->key >> 32) ^ 0x5eed5eedu;
   p->t = 0;
@@ -3173,6 +3620,7 @@ struct Tiles {
   int U = 8;                   // NMDA edges in flight per lane in the pull
   uint32_t Lmax = 1;           // steps per launch pair
   uint32_t dev_nsteps = 0;     // nsteps the device parameters hold (0: stale)
+  size_t smem = 0;             // dynamic shared memory of the step kernel (all networks)
   cudaGraphExec_t exec = nullptr;
   uint32_t graph_steps = 0;
   bool graph_ok = true, graph_used = false;
@@ -3241,6 +3689,13 @@ int tiles_upload(Tiles &T, const Params *hp, uint32_t count, uint32_t nsteps, cu
     }
     T.count = count;
   }
+  size_t smem = 0;
+  for (uint32_t i = 0; i < count; i++)
+    smem = std::max(smem, T.fp64 ? tile_smem<double, 128>(hp[i].live) : tile_smem<float, 256>(hp[i].live));
+  if (smem != T.smem) {  // the captured launches carry the old size
+    T.smem = smem;
+    T.graph_steps = 0;
+  }
   cudaError_t e = cudaMemcpyAsync(T.dP, hp, count * sizeof(Params), cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) {
@@ -3262,11 +3717,11 @@ cudaError_t tiles_enqueue(const Tiles &T, uint32_t nsteps, cudaStream_t st) {
     const uint32_t L = std::min(T.Lmax, nsteps - bs);
     if (T.fp64) {
       k_tile_pull<double, 4><<<T.ntiles, kThreads, 0, st>>>(T.dP, T.dT, bs, L);
-      k_tile_step<double, 1><<<T.ntiles, kThreads, 0, st>>>(T.dP, T.dT, bs, L);
+      k_tile_step<double><<<T.ntiles, kThreads, T.smem, st>>>(T.dP, T.dT, bs, L);
     } else {
       if (T.U == 4) k_tile_pull<float, 4><<<T.ntiles, kThreads, 0, st>>>(T.dP, T.dT, bs, L);
       else k_tile_pull<float, 8><<<T.ntiles, kThreads, 0, st>>>(T.dP, T.dT, bs, L);
-      k_tile_step<float, 2><<<T.ntiles, kThreads, 0, st>>>(T.dP, T.dT, bs, L);
+      k_tile_step<float><<<T.ntiles, kThreads, T.smem, st>>>(T.dP, T.dT, bs, L);
     }
   }
   k_tiles_advance<<<(T.count + 255) / 256, 256, 0, st>>>(T.dP, T.count, nsteps);
@@ -3524,7 +3979,8 @@ int batch_tune(Batch *B, uint32_t sample_steps, cudaStream_t st, BatchPlan *out,
 void batch_info(const Batch *B, BatchPlan *out) {
   int occ = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-      &occ, B->fp64 ? (const void *)k_tile_step<double, 1> : (const void *)k_tile_step<float, 2>, kThreads, 0);
+      &occ, B->fp64 ? (const void *)k_tile_step<double> : (const void *)k_tile_step<float>, kThreads,
+      B->T.smem ? B->T.smem : B->fp64 ? tile_smem<double, 128>(kLiveAll) : tile_smem<float, 256>(kLiveAll));
   out->blocks = B->T.ntiles;
   out->blocks_per_sm = (uint32_t)std::max(0, occ);
   out->tile_posts = B->T.tile_w;
@@ -3645,7 +4101,7 @@ __global__ void __launch_bounds__(kThreads) k_debug_drive(const __grid_constant_
   const uint32_t np = min(kT, count - q0), p0 = first + q0;
   for (uint32_t j0 = 0; j0 < nsteps; j0 += kLB) {
     const uint32_t L = min(kLB, nsteps - j0);
-    draw_inputs<T>(P, p0, np, t0 + j0, L, hits, gauss);
+    draw_inputs<T, kT>(P, p0, np, t0 + j0, L, hits, gauss);
     __syncthreads();
     for (uint32_t idx = threadIdx.x; idx < np * L; idx += kThreads) {
       const uint32_t j = idx / np, q = idx - j * np;
@@ -3710,8 +4166,8 @@ int prod_debug_drive(Prod *p, uint64_t t0, uint32_t nsteps, uint32_t first, uint
 // kernels since it was switched on (k_prod1: 0 spike-list lookups, 1 NMDA
 // copies of listed spikes, 2 last deliveries and NMDA sums, 3 neuron steps
 // and spike lists, 6 thread 0's barrier wait, 4 the rest of the barrier,
-// 5 set-up; k_prod: 0 NMDA pull, 1 drive draws, 2 neuron steps, 3 pushes,
-// 4 grid barrier).
+// 5 set-up; k_prod: 0 NMDA pull, 1 drive draws, 9 conductances, 2 membranes and
+// presynaptic state, 3 history and pushes, 4 grid barrier).
 int prod_phase_clock(Prod *p, int enable, cudaStream_t st, std::string &err) {
   const uint32_t nb = std::max(p->blocks, p->b1_blocks);
   if (!enable) {
@@ -3839,6 +4295,21 @@ int prod_state_save(Prod *p, uint8_t *buf, cudaStream_t st, std::string &err) {
   return FS_OK;
 }
 
+// The history slot that networks without delays read (the step before the
+// next) is s_pre: kernels that read s_pre itself do not keep the history, so a
+// restored state rebuilds it for those that do.
+__global__ void k_hist_fill(const __grid_constant__ Params P, uint64_t t, int fp64) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= P.n) return;
+  const uint32_t tm = (uint32_t)(t - 1u);
+  if (fp64) {
+    ((double *)P.s_hist)[(size_t)i * P.slots + (tm & P.mask)] = ((const double *)P.s_pre)[i];
+  } else {
+    for (uint32_t k = 0; k < kSH; k++)
+      ((float *)P.s_hist)[((size_t)i * kSH + k) * P.slots + ((tm - k) & P.mask)] = ((const float *)P.s_pre)[i];
+  }
+}
+
 int prod_state_load(Prod *p, const uint8_t *buf, cudaStream_t st, std::string &err) {
   cudaError_t e = cudaStreamSynchronize(st);
   StateHead h;
@@ -3851,11 +4322,17 @@ int prod_state_load(Prod *p, const uint8_t *buf, cudaStream_t st, std::string &e
     off += x.second;
   }
   if (e == cudaSuccess) e = cudaMemsetAsync(p->err, 0, 4, st);
+  if (e == cudaSuccess && p->P.dmax0 && h.t) {
+    k_hist_fill<<<(p->n + 255) / 256, 256, 0, st>>>(p->P, h.t, p->fp64 ? 1 : 0);
+    e = cudaGetLastError();
+  }
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) {
     err = std::string("checkpoint load: ") + cudaGetErrorString(e);
     return FS_ERR_CUDA;
   }
+  p->ext_live = 0x1fu;  // the state may hold any receptor's gates
+  set_live(p);
   p->t = h.t;
   p->P.key0 = h.key0;
   p->P.key1 = h.key1;
@@ -3895,6 +4372,7 @@ void prod_set_gains(Prod *p, const float *g) {
 }
 
 int prod_set_pb(Prod *p, const float *pb, cudaStream_t st, std::string &err) {
+  drive_changed(p, pb);
   cudaError_t e = cudaMemcpyAsync((void *)p->P.pb, pb, (size_t)FS_NREC * p->n * 4, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) {
@@ -3919,6 +4397,7 @@ int batch_set_drive(Batch *B, uint32_t i, const float *pb, cudaStream_t st, std:
     err = "batch: instance index out of range";
     return FS_ERR_ARG;
   }
+  B->T.dev_nsteps = 0;  // Params::live may have changed
   return prod_set_pb(B->inst[i], pb, st, err);
 }
 uint32_t batch_neurons(const Batch *B, uint32_t i) { return i < B->inst.size() ? B->inst[i]->n : 0; }
