@@ -157,13 +157,14 @@ struct Params {
   const uint32_t *gv_row, *gv_ent;
   uint32_t gv_n;
   float *gv_st, *gv_xt;  // [steps][gv_n]
-  uint32_t *t1_cnt;      // [4] overflow entries of step t, slot t mod 4
-  uint32_t t1_slots;     // entries per block region of a step's list
-  uint32_t t1_w;         // 16-byte words per list entry: 1 or 2
-  uint4 *t1_list;        // [2][blocks][t1_slots][t1_w]: (id, inc, c, step + 1) when every neuron
-                         // projects onto at most one linear receptor (c: that receptor's),
-                         // else (id, inc, c0, c1), (c2, c3, step + 1, 0)
-  uint4 *t1_ovf;         // [2][n][t1_w] the overflow lists
+  uint32_t t1_tag;       // steps listed in earlier launches: step s of this one has tag t1_tag + s + 1
+  uint32_t t1_slots;     // spikes per block region of a step's list (at most kSlots)
+  uint32_t t1_reps;      // copies of the list: block b reads copy b mod t1_reps
+  uint32_t t1_w;         // 16-byte words per listed spike: 1 or 2
+  uint4 *t1_list;        // [2][t1_reps][blocks] regions, by tag parity: t1_slots spikes of t1_w words each;
+                         // (id, inc, c, tag) when every neuron projects onto at most one linear
+                         // receptor (c: that receptor's), else (id, inc, c0, tag), (c1, c2, c3, tag)
+  uint4 *t1_ovf;         // [2][blocks][kT1][t1_w] a block's spikes beyond its t1_slots
 };
 
 // Block plan of k_prod1: posts [post0, post0 + np); tracked neurons [trk0,
@@ -638,14 +639,16 @@ __device__ __forceinline__ void store_membrane(const Params &P, uint32_t p, cons
 
 // kTM = false: the caller never runs a Tsodyks-Markram network (no
 // registers are spent on its state).
-template <class T, bool kTM = true>
+// kRec: the linear receptors that can be live (the others' state stays 0).
+template <class T, bool kTM = true, uint32_t kRec = 15>
 __device__ __forceinline__ void load_pre(const Params &P, uint32_t p, NeuronPar<T> &q, NeuronState<T> &st) {
   const uint32_t n = P.n;
   q.pj = P.proj[p];
 #pragma unroll
   for (int r = 0; r < 4; r++) {
-    q.pdf[r] = P.lin_of_rec[r] >= 0 ? (T)__ldg(P.pdf + (size_t)r * n + p) : (T)0;
-    st.sp[r] = P.lin_of_rec[r] >= 0 ? ((T *)P.st_pre)[(size_t)r * n + p] : (T)0;
+    const bool on = (kRec >> r & 1u) && P.lin_of_rec[r] >= 0;
+    q.pdf[r] = on ? (T)__ldg(P.pdf + (size_t)r * n + p) : (T)0;
+    st.sp[r] = on ? ((T *)P.st_pre)[(size_t)r * n + p] : (T)0;
   }
   q.pdfxt = (T)__ldg(P.p_dfxt + p);
   q.pdfst = (T)__ldg(P.p_dfst + p);
@@ -661,12 +664,12 @@ __device__ __forceinline__ void load_pre(const Params &P, uint32_t p, NeuronPar<
     st.tmx = P.tm_x[p];
   }
 }
-template <class T, bool kTM = true>
+template <class T, bool kTM = true, uint32_t kRec = 15>
 __device__ __forceinline__ void store_pre(const Params &P, uint32_t p, const NeuronPar<T> &q, const NeuronState<T> &st) {
   const uint32_t n = P.n;
 #pragma unroll
   for (int r = 0; r < 4; r++)
-    if (P.lin_of_rec[r] >= 0) ((T *)P.st_pre)[(size_t)r * n + p] = st.sp[r];
+    if ((kRec >> r & 1u) && P.lin_of_rec[r] >= 0) ((T *)P.st_pre)[(size_t)r * n + p] = st.sp[r];
   ((T *)P.x_pre)[p] = st.xp;
   ((T *)P.s_pre)[p] = st.spre;
   if (kTM && (q.pj & kPjTM)) {
@@ -675,13 +678,14 @@ __device__ __forceinline__ void store_pre(const Params &P, uint32_t p, const Neu
   }
 }
 
-template <class T, bool kTM = true>
+template <class T, bool kTM, uint32_t kRec>
 __device__ __forceinline__ void load_neuron(const Params &P, uint32_t p, NeuronPar<T> &q, NeuronState<T> &st) {
   const uint32_t n = P.n;
   load_membrane<T>(P, p, q, st);
-  load_pre<T, kTM>(P, p, q, st);
+  load_pre<T, kTM, kRec>(P, p, q, st);
 #pragma unroll
   for (int r = 0; r < 5; r++) {
+    if (r != FS_NMDA && !(kRec >> r & 1u)) continue;
     q.dfs[r] = (T)__ldg(P.dfst + (size_t)r * n + p);
     q.extg[r] = (T)__ldg(P.ext_g + (size_t)r * n + p);
   }
@@ -689,6 +693,7 @@ __device__ __forceinline__ void load_neuron(const Params &P, uint32_t p, NeuronP
   q.nefas = (T)__ldg(P.nmda_efst + p) * (T)__ldg(P.nmda_as + p);
 #pragma unroll
   for (int r = 0; r < 4; r++) {
+    if (!(kRec >> r & 1u)) continue;
     st.G[r] = ((T *)P.G)[(size_t)r * n + p];
     st.est[r] = ((T *)P.ext_st)[(size_t)r * n + p];
   }
@@ -696,14 +701,15 @@ __device__ __forceinline__ void load_neuron(const Params &P, uint32_t p, NeuronP
   st.es = ((T *)P.ext_s)[p];
 }
 
-template <class T, bool kTM = true>
+template <class T, bool kTM, uint32_t kRec>
 __device__ __forceinline__ void store_neuron(const Params &P, uint32_t p, const NeuronPar<T> &q,
                                              const NeuronState<T> &st) {
   const uint32_t n = P.n;
   store_membrane<T>(P, p, st);
-  store_pre<T, kTM>(P, p, q, st);
+  store_pre<T, kTM, kRec>(P, p, q, st);
 #pragma unroll
   for (int r = 0; r < 4; r++) {
+    if (!(kRec >> r & 1u)) continue;
     ((T *)P.G)[(size_t)r * n + p] = st.G[r];
     ((T *)P.ext_st)[(size_t)r * n + p] = st.est[r];
   }
@@ -766,11 +772,20 @@ __device__ __forceinline__ void drive_nmda(T &ex, T &es, T ndfxt, T dfs, T nefas
   es = fma_t<T>(dfs, es, mul_t(mul_t(nefas, ex), add_t((T)1, -es)));
 }
 
-// g: the step's conductances, by receptor (dead linear receptors' are not read).
-template <class T, bool kLTP = false>
+// The NMDA Mg block at membrane potential v: the divisor of its current.
+template <class T>
+__device__ __forceinline__ T mg_block(const NeuronPar<T> &q, T v) {
+  return fma_t<T>(q.mg, exp_t<T>(mul_t((T)-0.062, v)), (T)1);
+}
+
+// g: the step's conductances, by receptor (dead linear receptors' are not
+// read).  mgb: mg_block of the potential, when the caller has it already.
+// kRec: the linear receptors to add where that is known when compiling (no
+// branches: for a kernel whose schedulers have one warp each), 0: P.live says.
+template <class T, bool kLTP = false, uint32_t kRec = 0>
 __device__ __forceinline__ bool step_membrane(const Params &P, const NeuronPar<T> &q, NeuronState<T> &st, const T (&g)[5],
                                               T gauss, T gapI, uint32_t p, bool own, uint32_t s,
-                                              LtpTrace<T> *lt = nullptr) {
+                                              LtpTrace<T> *lt = nullptr, const T *mgb = nullptr) {
   const uint32_t n = P.n;
   T isyn = (T)0;
   if (q.a & FS_ACT_INJ) isyn = gauss;
@@ -779,19 +794,20 @@ __device__ __forceinline__ bool step_membrane(const Params &P, const NeuronPar<T
   // constants formed once (Mg / 3.57, 1e-3 / Cm), where the reference divides
   // every step: two divisions off each step's dependency chain, at a rounding
   // difference the FP32 and FP64 modes share
+  const uint32_t live = kRec ? kRec : P.live;
   uint32_t ns = st.ns;
   bool fire_now = false;
   if (ns & FS_NS_FIRE) {
     fire_now = true;
   } else {
     const T v = st.V;
-    const T Ir2 = mul_t(g[FS_NMDA], q.vrev[FS_NMDA] - v) / fma_t<T>(q.mg, exp_t<T>(mul_t((T)-0.062, v)), (T)1);
+    const T Ir2 = mul_t(g[FS_NMDA], q.vrev[FS_NMDA] - v) / (mgb ? *mgb : mg_block<T>(q, v));
     T I = (T)0;
-    if (P.live & 1u) I = mul_t(g[FS_AMPA], q.vrev[FS_AMPA] - v);
-    if (P.live & 2u) I = add_t(I, mul_t(g[FS_GABA], q.vrev[FS_GABA] - v));
+    if (live & 1u) I = mul_t(g[FS_AMPA], q.vrev[FS_AMPA] - v);
+    if (live & 2u) I = add_t(I, mul_t(g[FS_GABA], q.vrev[FS_GABA] - v));
     I = add_t(I, Ir2);
-    if (P.live & 4u) I = add_t(I, mul_t(g[FS_ACH], q.vrev[FS_ACH] - v));
-    if (P.live & 8u) I = add_t(I, mul_t(g[FS_GCL], q.vrev[FS_GCL] - v));
+    if (live & 4u) I = add_t(I, mul_t(g[FS_ACH], q.vrev[FS_ACH] - v));
+    if (live & 8u) I = add_t(I, mul_t(g[FS_GCL], q.vrev[FS_GCL] - v));
     I = add_t(fma_t<T>(isyn, (T)1e3, I), q.leak);
     I = mul_t(I, q.icm);
     if (I > q.dvm) {
@@ -805,11 +821,11 @@ __device__ __forceinline__ bool step_membrane(const Params &P, const NeuronPar<T
     }
     st.V = fma_t<T>(q.df, v, mul_t(q.ef, I));
     if (P.outI && own) {  // kept only while requested (code/EqsGnl2.cpp:196-206)
-      P.Irep[p] = (float)((P.live & 1u) ? mul_t(g[FS_AMPA], q.vrev[FS_AMPA] - v) : (T)0);
-      P.Irep[(size_t)n + p] = (float)((P.live & 2u) ? mul_t(g[FS_GABA], q.vrev[FS_GABA] - v) : (T)0);
+      P.Irep[p] = (float)((live & 1u) ? mul_t(g[FS_AMPA], q.vrev[FS_AMPA] - v) : (T)0);
+      P.Irep[(size_t)n + p] = (float)((live & 2u) ? mul_t(g[FS_GABA], q.vrev[FS_GABA] - v) : (T)0);
       P.Irep[(size_t)FS_NMDA * n + p] = (float)Ir2;
-      P.Irep[(size_t)FS_ACH * n + p] = (float)((P.live & 4u) ? mul_t(g[FS_ACH], q.vrev[FS_ACH] - v) : (T)0);
-      P.Irep[(size_t)FS_GCL * n + p] = (float)((P.live & 8u) ? mul_t(g[FS_GCL], q.vrev[FS_GCL] - v) : (T)0);
+      P.Irep[(size_t)FS_ACH * n + p] = (float)((live & 4u) ? mul_t(g[FS_ACH], q.vrev[FS_ACH] - v) : (T)0);
+      P.Irep[(size_t)FS_GCL * n + p] = (float)((live & 8u) ? mul_t(g[FS_GCL], q.vrev[FS_GCL] - v) : (T)0);
     }
     if (st.V > q.vth) {
       ns |= FS_NS_FIRE;
@@ -855,10 +871,29 @@ __device__ __forceinline__ bool step_membrane(const Params &P, const NeuronPar<T
   return own && (ns & FS_NS_SPIKE) != 0;
 }
 
+// What a spike of neuron p carries, before step_pre advances its state: the
+// increment inc and, per linear receptor, c (step_pre's values).
+template <class T, bool kTM, uint32_t kRec>
+__device__ __forceinline__ void spike_carries(const Params &P, const NeuronPar<T> &q, const NeuronState<T> &st, uint32_t p,
+                                              T (&cinc)[4], T &inc) {
+  inc = (T)1;
+  if (q.pj) {
+    if (P.plast == PL_STD) inc = (T)P.D[p];
+    else if (P.plast == PL_STP) inc = (T)P.D[p] * (T)P.F[p];
+    else if (kTM && (q.pj & kPjTM)) {
+      const T u = (T)st.tmu, U = (T)__ldg(P.tm_U + p);
+      inc = fma_t<T>(U, (T)1 - u, u) * (T)st.tmx;
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < 4; r++)
+    cinc[r] = (kRec >> r & 1u) && (q.pj & (1u << r)) ? fma_t<T>(st.sp[r], (T)1 - q.pdf[r], inc) : (T)0;
+}
+
 // kTM = false: the caller never runs a Tsodyks-Markram network.  tm: the
 // Tsodyks-Markram U, dff, dfr from the caller's per-thread copy, or null (read
 // from global memory).
-template <class T, bool kTM = true>
+template <class T, bool kTM = true, uint32_t kRec = 15>
 __device__ __forceinline__ void step_pre(const Params &P, const NeuronPar<T> &q, NeuronState<T> &st, bool spk, uint32_t p,
                                          bool own, T (&cinc)[4], T &inc_out, const float *tm = nullptr) {
 #pragma unroll
@@ -879,7 +914,7 @@ __device__ __forceinline__ void step_pre(const Params &P, const NeuronPar<T> &q,
     }
 #pragma unroll
     for (int r = 0; r < 4; r++) {
-      if (P.lin_of_rec[r] >= 0) {
+      if ((kRec >> r & 1u) && P.lin_of_rec[r] >= 0) {
         const bool on = (q.pj & (1u << r)) != 0;
         const T a = st.sp[r];
         cinc[r] = on && spk ? fma_t<T>(a, (T)1 - q.pdf[r], inc) : (T)0;
@@ -912,154 +947,6 @@ __device__ __forceinline__ void step_pre(const Params &P, const NeuronPar<T> &q,
     }
   }
   inc_out = inc;
-}
-
-// The three parts in one thread (k_prod1).
-template <class T, bool kTM>
-__device__ __forceinline__ bool neuron_step(const Params &P, const NeuronPar<T> &q, NeuronState<T> &st,
-                                            const long long (&rv)[4], T gnmda, uint32_t hit, T gauss, T gapI,
-                                            uint32_t p, bool own, uint32_t s, T (&cinc)[4], T &inc_out) {
-  const uint32_t n = P.n;
-  T g[5];
-#pragma unroll
-  for (int r = 0; r < 4; r++) {
-    g[r] = (T)0;
-    if (P.lin_of_rec[r] >= 0) {
-      st.G[r] = fma_t<T>(q.dfs[r], st.G[r], (T)rv[r] * (T)kInvFix);  // exact power-of-two scale
-      g[r] = st.G[r];
-    }
-  }
-  g[FS_NMDA] = gnmda * (T)P.rg[FS_NMDA];
-  // external drive (BgInit): bit r of hit = receptor r's Bernoulli outcome
-  const uint32_t bitsr[4] = {FS_ACT_AMPA, FS_ACT_GABA, FS_ACT_ACH, FS_ACT_GCL};
-#pragma unroll
-  for (int r = 0; r < 4; r++) {
-    if (q.a & bitsr[r]) {
-      st.est[r] = (hit & (1u << r)) ? st.est[r] + (T)1 : st.est[r] * q.dfs[r];
-      g[r] = fma_t<T>(q.extg[r], st.est[r], g[r]);
-    }
-  }
-  T isyn = (T)0;
-  if (q.a & FS_ACT_NMDA) {
-    st.ex = (hit & (1u << FS_NMDA)) ? st.ex + (T)1 : st.ex * q.ndfxt;
-    st.es = fma_t<T>(q.dfs[FS_NMDA], st.es, (q.nefas * st.ex) * ((T)1 - st.es));
-    g[FS_NMDA] = fma_t<T>(q.extg[FS_NMDA], st.es, g[FS_NMDA]);
-  }
-  if (q.a & FS_ACT_INJ) isyn = gauss;
-  if (P.gap_row) isyn = isyn + gapI;  // steps of networks with gap junctions come one at a time
-  // VmEul + firing (code/EqsGnl2.cpp:152-251); the production modes scale
-  // the Mg block and the current by per-neuron constants formed once
-  // (Mg / 3.57, 1e-3 / Cm), where the reference divides every step: two
-  // divisions off each step's dependency chain (775 -> 664 SM cycles per
-  // step for one warp), at a rounding difference the FP32 and FP64 modes
-  // share
-  uint32_t ns = st.ns;
-  bool fire_now = false;
-  if (ns & FS_NS_FIRE) {
-    fire_now = true;
-  } else {
-    const T v = st.V;
-    const T Ir0 = g[FS_AMPA] * (q.vrev[FS_AMPA] - v);
-    const T Ir1 = g[FS_GABA] * (q.vrev[FS_GABA] - v);
-    const T Ir2 = g[FS_NMDA] * (q.vrev[FS_NMDA] - v) / ((T)1 + q.mg * exp_t<T>((T)-0.062 * v));
-    const T Ir3 = g[FS_ACH] * (q.vrev[FS_ACH] - v);
-    const T Ir4 = g[FS_GCL] * (q.vrev[FS_GCL] - v);
-    T I = fma_t<T>(isyn, (T)1e3, Ir0 + Ir1 + Ir2 + Ir3 + Ir4) + q.leak;
-    I = I * q.icm;
-    if (I > q.dvm) {
-      I = q.dvm;
-      ns = (ns | FS_NS_MEMDV_OVF) & ~FS_NS_MEMDV_UDF;
-    } else if (I < -q.dvm) {
-      I = -q.dvm;
-      ns = (ns & ~FS_NS_MEMDV_OVF) | FS_NS_MEMDV_UDF;
-    } else {
-      ns &= ~(FS_NS_MEMDV_OVF | FS_NS_MEMDV_UDF);
-    }
-    st.V = fma_t<T>(q.df, v, q.ef * I);
-    if (P.outI && own) {  // kept only while requested (code/EqsGnl2.cpp:196-206)
-      P.Irep[p] = (float)Ir0;
-      P.Irep[(size_t)n + p] = (float)Ir1;
-      P.Irep[(size_t)FS_NMDA * n + p] = (float)Ir2;
-      P.Irep[(size_t)FS_ACH * n + p] = (float)Ir3;
-      P.Irep[(size_t)FS_GCL * n + p] = (float)Ir4;
-    }
-    if (st.V > q.vth) {
-      ns |= FS_NS_FIRE;
-      fire_now = true;
-    }
-  }
-  if (fire_now) {
-    if (st.cnt < q.rf) {
-      st.V = (st.cnt == 0) ? (T)0 : q.vreset;
-      if (st.cnt == q.sd) ns |= FS_NS_SPIKE;
-      else ns &= ~FS_NS_SPIKE;
-      st.cnt++;
-    } else {
-      st.cnt = 0;
-      ns &= ~FS_NS_FIRE;
-    }
-  }
-  st.ns = ns;
-  if (own && P.outV) P.outV[(size_t)s * n + p] = (float)st.V;
-  if (own && P.outNS) P.outNS[(size_t)s * n + p] = ns;
-  if (own && P.outI)
-#pragma unroll
-    for (int r = 0; r < 5; r++) P.outI[(size_t)s * 5 * n + (size_t)r * n + p] = P.Irep[(size_t)r * n + p];
-  const bool spk = own && (ns & FS_NS_SPIKE) != 0;
-  // presynaptic state: increment per spike, then plasticity update
-#pragma unroll
-  for (int r = 0; r < 4; r++) cinc[r] = (T)0;
-  T inc = (T)1;
-  if (q.pj && own) {
-    if (P.plast == PL_STD) inc = (T)P.D[p];
-    else if (P.plast == PL_STP) inc = (T)P.D[p] * (T)P.F[p];
-    else if (kTM && (q.pj & kPjTM)) {
-      T u = (T)st.tmu, x = (T)st.tmx;
-      const T U = (T)__ldg(P.tm_U + p);
-      if (spk) {
-        u = u + U * ((T)1 - u);
-        const T rel = u * x;
-        inc = rel;
-        x = x - rel;
-      } else {
-        u = U + (u - U) * (T)__ldg(P.tm_dff + p);
-        x = (T)1 + (x - (T)1) * (T)__ldg(P.tm_dfr + p);
-      }
-      st.tmu = (float)u;
-      st.tmx = (float)x;
-    }
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-      if (q.pj & (1u << r)) {
-        if (spk) {
-          cinc[r] = inc + st.sp[r] * ((T)1 - q.pdf[r]);
-          st.sp[r] = st.sp[r] + inc;
-        } else {
-          st.sp[r] = st.sp[r] * q.pdf[r];
-        }
-      }
-    }
-    if (q.pj & (1u << FS_NMDA)) nmda_pre_step<T>(st.xp, st.spre, spk, inc, q.pdfxt, q.pdfst, q.pefas);
-    if (P.plast == PL_STD) {
-      P.D[p] = spk ? P.D[p] * (1.0f - P.stp_pv[p]) : P.stp_dfD[p] * P.D[p] + P.stp_efD[p];
-    } else if (P.plast == PL_STP) {
-      float Dv = P.D[p], Fv = P.F[p], Cp = P.Cap[p], Cr = P.Car[p];
-      if (spk) {
-        Cr += P.stp_aCar[p];
-        Cp += P.stp_aCap[p];
-        Fv += (Cp + Cr) * (1.0f - Fv) * P.stp_aF[p];
-        Dv *= (1.0f - P.stp_pv[p] * Fv);
-      } else {
-        Cr = P.stp_dfCar[p] * Cr + P.stp_efCar[p];
-        Cp = P.stp_dfCap[p] * Cp;
-        Fv = P.stp_dfF[p] * Fv + P.stp_efF[p] * (Cp + Cr) * (1.0f - Fv) * P.stp_aF[p];
-        Dv = P.stp_dfD[p] * Dv + P.stp_efD[p];
-      }
-      P.D[p] = Dv; P.F[p] = Fv; P.Cap[p] = Cp; P.Car[p] = Cr;
-    }
-  }
-  inc_out = inc;
-  return spk;
 }
 
 // Spike outputs of a warp's step: the per-step bitmap and count, the total.
@@ -1714,9 +1601,9 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1) k_prod_ltp(c
 //    x and s, advanced every step by nmda_pre_step from the spike list (the
 //    same function and operands as the neuron's owner, so every copy equals
 //    the owner's value bit for bit);
-//  * the NMDA in-edges of its posts live in shared memory as (tracked index,
-//    weight), summed per post by eight lanes (lane-strided, then an xor
-//    butterfly: the order of nmda_pull1_f32);
+//  * the NMDA in-edges of its posts live in shared memory as (slot, weight),
+//    summed per post by eight lanes (lane-strided, then an xor butterfly: the
+//    order of nmda_pull1_f32; group_sum);
 //  * a listed spike is matched to the block's tracked neurons through a
 //    bitmap of their ids with per-word ranks (two shared-memory loads);
 //  * a spike's linear synapses are delivered by the blocks of its targets:
@@ -1724,15 +1611,37 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1) k_prod_ltp(c
 //    w*c (2^-40 fixed point, integer atomics: any order gives the same sum)
 //    into per-post accumulators, the same integers the interval kernel's
 //    delay ring sums;
-//  * the owner of a neuron that spikes appends (id, inc, c[4]) to the step's
-//    list; lists alternate by step parity and the last block at a barrier
-//    empties the next step's list.
+//  * a block's spikes go into its region of the step's list: two entries
+//    (id, inc, c, tag), written every step, used or not, each as one 128-bit
+//    word.  The other blocks poll the entries themselves: the entry that carries
+//    the step's tag is the arrival and the spike, so a step has no grid barrier
+//    and no list to fetch behind it (a barrier's wait and the list's round trip
+//    were 2,830 + 1,360 cycles of a step).  Regions alternate by tag parity: a block
+//    lists step t + 2 only after it has read every block's entries of step
+//    t + 1, which those wrote after they had read step t's.  A block's third and
+//    later spikes lie in its overflow region, tagged too; the first entry
+//    has their number.  The polls of 148 blocks on the same lines hold up each
+//    other and the writes: each step's list exists 16 times (a warp writes a
+//    block's region into all), read by about nine blocks each (publishing to B's
+//    arrival, 1,000 neurons: 4,170 cycles with one list of three slots, 3,070 with
+//    eight, 2,050 with 16 of two slots; 37 to 148 lists, or two spikes in one word,
+//    are no faster).
+// What bounds a step is the chain of its phases, so work is taken off it: with
+// posts in at most half of the warps (the usual case) the others are helpers
+// without neuron state, which make the draws and advance the copies while the
+// neurons step, then wait for the lists; the neurons' warps list their spikes as
+// soon as the membranes have stepped, and make the presynaptic state, the
+// drive's gates and the Mg block of the next step while the entries travel.
+// Cycles a step, 20k connectome: sums 4,150 -> 3,420, membranes and list 1,900 ->
+// 1,800, barrier, list and look-ups 6,400 -> 3,150; 7.1 -> 4.9 us a step (calls
+// of 400).  1,000 neurons: 5.6 -> 3.5 us (calls of 200).
 // Across launches the pending deliveries travel through the delay ring as
 // in the interval kernel: the last step pushes its spikes into the ring and
-// the first step of the next launch folds its ring slot.  The drive draws
-// of step t + 1 are made while a block waits at the barrier of step t.
+// the first step of the next launch folds its ring slot.
 constexpr uint32_t kT1 = 512;   // threads of k_prod1 (= max posts per block)
-constexpr uint32_t kT1F = 512;  // listed spikes looked up per pass
+constexpr uint32_t kT1F = 512;  // list entries of a step's blocks
+constexpr uint32_t kSlots = 2;  // (three: a third more lines to poll; one: 64 % of the 20k connectome's steps overflow)
+constexpr uint32_t kInline = 8;  // spikes beyond a region that the thread of its entry reads itself
 
 // Tracked index of neuron id in a block (or -1): bit id of the block's
 // bitmap (words [w0, w0 + nwd) of the id space) says whether it is
@@ -1768,32 +1677,129 @@ __device__ __forceinline__ void deliver_listed(const Params &P, const Blk1 &me, 
   }
 }
 
-// Grid barrier of k_prod1: as grid_sync, with threads of warps 1.. running
-// work() while thread 0 waits.
-template <class F>
-__device__ __forceinline__ bool grid_sync_work(unsigned int *bar, int *err, uint32_t count,
-                                               unsigned long long &target, PhaseClock &pc, F &&work,
-                                               unsigned int limit = 1u << 24) {
-  __shared__ int ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    ok = count > 1 ? arrive_and_wait(bar, err, count, target, limit) : 1;
-    pc.mark(6);  // thread 0's wait for the other blocks
-  } else if (threadIdx.x >= 32) {
-    work();
+// List entries are read and written as one 128-bit word each (single-copy
+// atomic), so an entry's tag says that the rest of it is there.
+__device__ __forceinline__ uint4 ld_entry(const uint4 *p) {
+  unsigned long long lo, hi;
+  asm volatile("{\n .reg .b128 v;\n ld.relaxed.gpu.global.b128 v, [%2];\n mov.b128 {%0, %1}, v;\n}"
+               : "=l"(lo), "=l"(hi) : "l"(p) : "memory");
+  return make_uint4((uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)hi, (uint32_t)(hi >> 32));
+}
+__device__ __forceinline__ void st_entry(uint4 *p, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+  asm volatile("{\n .reg .b128 v;\n mov.b128 v, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], v;\n}" ::"l"(p),
+               "l"((unsigned long long)x | (unsigned long long)y << 32),
+               "l"((unsigned long long)z | (unsigned long long)w << 32) : "memory");
+}
+// Waits until entry e (W words) carries the tag; false: the wait's limit ran out or
+// another block gave up.  b is the second word (W = 2).
+__device__ __forceinline__ bool await_entry(const uint4 *e, uint32_t W, uint32_t tag, uint4 &a, uint4 &b, int *err) {
+  for (uint32_t spins = 0;;) {
+    a = ld_entry(e);
+    if (W == 2) b = ld_entry(e + 1);
+    if (a.w == tag && (W == 1 || b.w == tag)) return true;
+    if ((++spins & 63u) == 0u) {
+      if (*(volatile int *)err) return false;
+      if (spins > (1u << 22)) {
+        atomicExch(err, 2);
+        return false;
+      }
+    }
   }
-  __syncthreads();
-  return ok != 0;
+}
+// The c of a neuron that projects onto at most one linear receptor: at most
+// one of them is not 0, so the sum is that one exactly.
+__device__ __forceinline__ float one_c(const float (&c)[4]) { return ((c[0] + c[1]) + c[2]) + c[3]; }
+__device__ __forceinline__ void put_entry(uint4 *e, uint32_t W, uint32_t id, float inc, const float (&c)[4],
+                                          uint32_t tag) {
+  if (W == 2) {
+    st_entry(e, id, __float_as_uint(inc), __float_as_uint(c[0]), tag);
+    st_entry(e + 1, __float_as_uint(c[1]), __float_as_uint(c[2]), __float_as_uint(c[3]), tag);
+  } else {
+    st_entry(e, id, __float_as_uint(inc), __float_as_uint(one_c(c)), tag);
+  }
+}
+constexpr uint32_t kNoSpike = 0x80000000u;  // entry's first word: an empty slot; bits 20-29 of a
+                                            // region's first: the block's spikes beyond its slots
+
+// Rows of 32 NMDA edges are kept four at a time in shared memory, lane by lane,
+// so that a lane reads four weights and four slots with one load each (what is
+// left of a group's rows stays row by row): entry x of a group with R rows.
+__device__ __forceinline__ uint32_t edge_at(uint32_t x, uint32_t R) {
+  const uint32_t r = x >> 5, l = x & 31u;
+  return (r | 3u) < R ? (r & ~3u) * 32u + 4u * l + (r & 3u) : x;
+}
+
+// NMDA sum of a group's posts over its R rows (w, x at the group's first entry):
+// lane l of quarter h sums post 4g + h's edges l, l + 8, ... in order (then
+// zero-weight fillers, which leave the sum unchanged), then a butterfly over
+// 4, 2, 1.  Eight rows are in flight; the next eight's weights and slots are
+// read while they arrive.
+__device__ __forceinline__ float group_sum(const float *w, const uint16_t *x, uint32_t R, const float *Sv, uint32_t lane) {
+  float sum = 0.0f;
+  const float4 *w4 = (const float4 *)w + lane;
+  const uint2 *x4 = (const uint2 *)x + lane;
+  uint32_t k = R >> 2;  // quads left
+  if (k) {
+    float4 wa = *w4, wb = wa;
+    uint2 xa = *x4, xb = xa;
+    if (k > 1) {
+      wb = w4[32];
+      xb = x4[32];
+    }
+    for (;;) {
+      const float a0 = Sv[xa.x & 0xffffu], a1 = Sv[xa.x >> 16], a2 = Sv[xa.y & 0xffffu], a3 = Sv[xa.y >> 16];
+      const float b0 = Sv[xb.x & 0xffffu], b1 = Sv[xb.x >> 16], b2 = Sv[xb.y & 0xffffu], b3 = Sv[xb.y >> 16];
+      const float4 ca = wa, cb = wb;
+      const bool two = k > 1;
+      k = k > 2 ? k - 2 : 0;
+      w4 += 64;
+      x4 += 64;
+      if (k) {
+        wa = *w4;
+        xa = *x4;
+        if (k > 1) {
+          wb = w4[32];
+          xb = x4[32];
+        }
+      }
+      sum = __fmaf_rn(ca.x, a0, sum);
+      sum = __fmaf_rn(ca.y, a1, sum);
+      sum = __fmaf_rn(ca.z, a2, sum);
+      sum = __fmaf_rn(ca.w, a3, sum);
+      if (two) {
+        sum = __fmaf_rn(cb.x, b0, sum);
+        sum = __fmaf_rn(cb.y, b1, sum);
+        sum = __fmaf_rn(cb.z, b2, sum);
+        sum = __fmaf_rn(cb.w, b3, sum);
+      }
+      if (!k) break;
+    }
+  }
+  const uint32_t left = R & 3u;
+  if (left) {  // (a row that is not there reads the last one's)
+    const uint32_t e0 = (R & ~3u) * 32u + lane, e1 = e0 + (left > 1 ? 32u : 0u), e2 = e0 + 32u * (left - 1u);
+    const float c0 = w[e0], c1 = w[e1], c2 = w[e2], v0 = Sv[x[e0]], v1 = Sv[x[e1]], v2 = Sv[x[e2]];
+    sum = __fmaf_rn(c0, v0, sum);
+    if (left > 1) sum = __fmaf_rn(c1, v1, sum);
+    if (left > 2) sum = __fmaf_rn(c2, v2, sum);
+  }
+#pragma unroll
+  for (int o = 4; o; o >>= 1) sum += __shfl_xor_sync(fsd::kFull, sum, o);
+  return sum;
 }
 
 // kTM: the network has Tsodyks-Markram plasticity (an instance without it
-// spends no registers on its state).
-template <bool kTM>
+// spends no registers on its state).  kRec: the linear receptors that can be
+// live (AMPA and GABA in most networks; every one an instance has costs seven
+// registers of the 128 that 512 threads have, and instructions of a chain
+// that all other blocks wait for).
+template <bool kTM, uint32_t kRec>
 __global__ void __launch_bounds__(kT1, 1) k_prod1(const __grid_constant__ Params P) {
   extern __shared__ __align__(16) unsigned char sm1[];
-  __shared__ float gn[kT1], d_gauss[kT1], f_c[kT1F][4], nf_inc[kT1F];
-  __shared__ uint8_t d_hits[kT1];
-  __shared__ uint32_t f_j[kT1F], f_n, nf_j[kT1F], nf_n, next_grp, blk_n;
+  __shared__ float gn[kT1], d_gauss[kT1 / 2], f_c[kT1F][4], sp_c[kSlots][4], sp_inc[kSlots];
+  __shared__ uint8_t d_hits[kT1 / 2];
+  __shared__ uint32_t f_j[kT1F], f_n, next_grp, blk_n, sp_p[kSlots], ov_n, ov[kT1F], in_n;
+  __shared__ int gave_up;
   const Blk1 me = P.b1[blockIdx.x];
   const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const uint32_t n = P.n, mask = P.mask, NT = me.ntrk, NS = me.nslot, np = me.np, ng = (np + 3) / 4;
@@ -1805,15 +1811,15 @@ __global__ void __launch_bounds__(kT1, 1) k_prod1(const __grid_constant__ Params
   float *const cs0 = cx0 + NS;                                 // [NS] NMDA s copies
   float *const cx1 = cs0 + NS;
   float *const cs1 = cx1 + NS;
-  float *ctab = cs1 + NS;                                      // [ncls][3]
-  float *ew = ctab + 3 * P.t1_ncls;                            // [ne] edge weights, group rows
-  uint32_t *bits = (uint32_t *)(ew + me.ne);                   // [nwd] tracked-neuron bitmap
+  float *ew = cs1 + NS;                                        // [ne] edge weights, groups' rows (edge_at)
+  uint16_t *eidx = (uint16_t *)(ew + me.ne);                   // [ne] edge sources' slots
+  uint8_t *cls = (uint8_t *)(eidx + me.ne);                    // [NS] kinetics class, 255: none
+  float *ctab = (float *)(cls + NS);                           // [ncls][3]
+  uint32_t *bits = (uint32_t *)(ctab + 3 * P.t1_ncls);         // [nwd] tracked-neuron bitmap
   uint32_t *grow = bits + me.nwd;                              // [ng + 1] first row of each group
-  uint16_t *eidx = (uint16_t *)(grow + ng + 1);                // [ne] edge sources' slots
-  uint16_t *rank = eidx + me.ne;                               // [nwd]
+  uint16_t *rank = (uint16_t *)(grow + ng + 1);                // [nwd]
   uint16_t *lrow = rank + me.nwd;                              // [NT + 1] linear rows
   uint16_t *perm = lrow + NT + 1;                              // [NT] slots
-  uint8_t *cls = (uint8_t *)(perm + NT);                       // [NS] kinetics class, 255: none
   // ---- tables ----
   for (uint32_t i = tid; i < max(1u, P.nlin) * kT1; i += kT1) acc[i] = 0ll;
   for (uint32_t i = tid; i < 3 * P.t1_ncls; i += kT1) ctab[i] = __ldg(P.t1_cls_tab + i);
@@ -1836,9 +1842,206 @@ __global__ void __launch_bounds__(kT1, 1) k_prod1(const __grid_constant__ Params
   for (uint32_t j = tid; j <= NT; j += kT1) lrow[j] = __ldg(P.t1_lrow + me.lrow0 + j);
   for (uint32_t j = tid; j < NT; j += kT1) perm[j] = __ldg(P.t1_perm + me.trk0 + j);
   for (uint32_t g = tid; g <= ng; g += kT1) grow[g] = __ldg(P.t1_grow + me.grow0 + g);
-  for (uint32_t e = tid; e < me.ne; e += kT1) {
-    ew[e] = __ldg(P.t1_ew + me.e0 + e);
-    eidx[e] = __ldg(P.t1_eidx + me.e0 + e);
+  for (uint32_t g = tid >> 5; g < ng; g += kT1 / 32) {
+    const uint32_t r0 = __ldg(P.t1_grow + me.grow0 + g), R = __ldg(P.t1_grow + me.grow0 + g + 1) - r0;
+    for (uint32_t x = lane; x < 32u * R; x += 32) {
+      const uint32_t to = 32u * r0 + edge_at(x, R);
+      ew[to] = __ldg(P.t1_ew + me.e0 + 32u * r0 + x);
+      eidx[to] = __ldg(P.t1_eidx + me.e0 + 32u * r0 + x);
+    }
+  }
+  // A block whose posts take at most half of its warps splits its warps: those
+  // with posts (nact) hold their neurons' state and deliver the listed spikes;
+  // the helpers, which have the registers free that the state takes elsewhere,
+  // make the NMDA sums, the next step's draws, the copies' advance, and wait for
+  // the other blocks' entries, all but the sums while the neurons step.
+  // In a block with more posts every warp does everything in turn.
+  const uint32_t nact = (np + 31) / 32, help = nact <= kT1 / 64 ? nact : 0, h0 = help * 32, H = kT1 - h0;
+  const uint32_t W = P.t1_w, slots = P.t1_slots, reps = P.t1_reps;
+  const uint32_t nreg = gridDim.x * slots;
+  auto ovf_at = [&](uint32_t tag, uint32_t b, uint32_t k) {
+    return P.t1_ovf + (((size_t)(tag & 1u) * gridDim.x + b) * kT1 + k) * W;
+  };
+  // a listed spike (entry words a, b): its NMDA copy is redone from the one of
+  // the step before, and its linear synapses onto this block are listed for
+  // delivery
+  auto take = [&](const float *X, const float *Sv, float *Xn, float *Sn, const uint4 &a, const uint4 &b) {
+    const int j = find_tracked(bits, rank, me.w0, me.nwd, a.x & 0xfffffu);
+    if (j < 0) return;
+    const uint32_t sl = perm[j], c = cls[sl];
+    if (c != 255) {
+      float xv = X[sl], sv = Sv[sl];
+      nmda_pre_step<float>(xv, sv, true, __uint_as_float(a.y), ctab[3 * c], ctab[3 * c + 1], ctab[3 * c + 2]);
+      Xn[sl] = xv;
+      Sn[sl] = sv;
+    }
+    if (lrow[j + 1] > lrow[j]) {
+      const uint32_t k = atomicAdd(&f_n, 1u);
+      f_j[k] = (uint32_t)j;
+      f_c[k][0] = __uint_as_float(a.z);
+      f_c[k][1] = __uint_as_float(W == 2 ? b.x : a.z);
+      f_c[k][2] = __uint_as_float(W == 2 ? b.y : a.z);
+      f_c[k][3] = __uint_as_float(W == 2 ? b.z : a.z);
+    }
+  };
+  PhaseClock pc;
+  pc.start(P);
+  // the copies after step t - 1 (X, Sv) and after step t (Xn, Sn)
+  auto buf = [&](uint32_t s, float *&X, float *&Sv, float *&Xn, float *&Sn) {
+    X = (s & 1u) ? cx1 : cx0;
+    Sv = (s & 1u) ? cs1 : cs0;
+    Xn = (s & 1u) ? cx0 : cx1;
+    Sn = (s & 1u) ? cs0 : cs1;
+  };
+  // Deliveries of step t - 1's spikes by D of the warps, which join the sums
+  // after: those with posts (or the first kDelW) and, from the last one down, the
+  // helpers that have no group of posts to sum.
+  const uint32_t first = help ? help : kDelW, idle = ng < kT1 / 32 - first ? kT1 / 32 - first - ng : 0u;
+  const uint32_t D = first + idle;
+  auto deliver = [&]() {
+    const uint32_t w = wid < first ? wid : first + (kT1 / 32 - 1 - wid);
+    if (w < D) deliver_listed(P, me, f_n, f_j, f_c, lrow, acc, w, lane, D);
+  };
+  // The NMDA sums: the first groups of the block by number to the warps that do
+  // not deliver, then from a shared counter (asked for a group ahead).
+  auto sums = [&](const float *Sv) {
+    uint32_t g = wid - first, nx = 0;
+    if (wid < first) g = __shfl_sync(fsd::kFull, lane == 0 ? atomicAdd(&next_grp, 1u) : 0u, 0);
+    while (g < ng) {
+      if (lane == 0) nx = atomicAdd(&next_grp, 1u);
+      const uint32_t r = grow[g], R = grow[g + 1] - r;
+      const float sum = group_sum(ew + 32u * r, eidx + 32u * r, R, Sv, lane);
+      const uint32_t qq = 4 * g + (lane >> 3);
+      if ((lane & 7u) == 0 && qq < np) gn[qq] = sum;
+      g = __shfl_sync(fsd::kFull, nx, 0);
+    }
+  };
+  const uint32_t grp0 = kT1 / 32 - first;  // groups taken by number
+  // The copies of the next step, as if no neuron had spiked.
+  auto advance_copies = [&](const float *X, const float *Sv, float *Xn, float *Sn, uint32_t h) {
+    // four slots a thread (an empty slot holds 0 in both buffers)
+    auto advance = [&](uint32_t j, auto kin) {
+      const uint32_t cl = ((const uint32_t *)cls)[j];
+      float4 x = ((const float4 *)X)[j], v = ((const float4 *)Sv)[j];
+      float *xe = &x.x, *ve = &v.x;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const uint32_t c = (cl >> (8 * k)) & 255u;
+        float k0, k1, k2, xv = xe[k], sv = ve[k];
+        kin(c, k0, k1, k2);
+        nmda_pre_step<float>(xv, sv, false, 1.0f, k0, k1, k2);
+        xe[k] = c != 255 ? xv : 0.0f;
+        ve[k] = c != 255 ? sv : 0.0f;
+      }
+      ((float4 *)Xn)[j] = x;
+      ((float4 *)Sn)[j] = v;
+    };
+    if (P.t1_ncls == 1) {  // one class (the usual case): its constants in registers
+      const float a0 = ctab[0], a1 = ctab[1], a2 = ctab[2];
+#pragma unroll 2
+      for (uint32_t j = h; j < NS / 4; j += H)
+        advance(j, [&](uint32_t, float &k0, float &k1, float &k2) { k0 = a0; k1 = a1; k2 = a2; });
+    } else if (P.t1_ncls > 1) {
+      for (uint32_t j = h; j < NS / 4; j += H)
+        advance(j, [&](uint32_t c, float &k0, float &k1, float &k2) {
+          const uint32_t i = c != 255 ? 3 * c : 0u;
+          k0 = ctab[i]; k1 = ctab[i + 1]; k2 = ctab[i + 2];
+        });
+    }
+  };
+  // The other blocks' entries of the step.
+  auto lists = [&](const float *X, const float *Sv, float *Xn, float *Sn, uint32_t tag, uint32_t h) {
+    const uint4 *mine = P.t1_list + (size_t)(blockIdx.x % reps) * nreg * W;
+    for (uint32_t e = h; e < nreg; e += H) {
+      uint4 a, b;
+      if (!await_entry(mine + ((size_t)(tag & 1u) * reps * nreg + e) * W, W, tag, a, b, P.err)) {
+        gave_up = 1;
+        break;
+      }
+      if (a.x & kNoSpike) continue;
+      const uint32_t rest = a.x >> 20;
+      take(X, Sv, Xn, Sn, a, b);
+      if (!rest) continue;
+      // a few more: by this thread (f_j has room for them next to the regions'),
+      // else by the block below
+      const uint32_t ob = e / slots;
+      if (rest > kInline || atomicAdd(&in_n, rest) + rest > kT1F - gridDim.x * slots) {
+        ov[atomicAdd(&ov_n, 1u)] = ob << 10 | rest;
+        continue;
+      }
+      for (uint32_t k = 0; k < rest; k++) {
+        if (!await_entry(ovf_at(tag, ob, k), W, tag, a, b, P.err)) {
+          gave_up = 1;
+          break;
+        }
+        take(X, Sv, Xn, Sn, a, b);
+      }
+    }
+  };
+  auto all = [&]() { asm volatile("bar.sync 4, %0;" ::"n"(kT1) : "memory"); };  // the block's warps, wherever they are
+  // Blocks with more spikes than slots: the rest of theirs, a block at a time
+  // (every thread of the block comes here, after a barrier).  False: a wait gave
+  // up.
+  auto overflow = [&](const float *X, const float *Sv, float *Xn, float *Sn, uint32_t tag) {
+    if (gave_up) return false;
+    if (ov_n) {
+      // (the deliveries listed so far come first; a block has at most kT1 - 1 left)
+      deliver_listed(P, me, f_n, f_j, f_c, lrow, acc, wid, lane, kT1 / 32);
+      for (uint32_t k = 0, nk = ov_n; k < nk; k++) {
+        all();
+        if (tid == 0) f_n = 0;
+        all();
+        const uint32_t ob = ov[k] >> 10, on = ov[k] & 1023u;
+        if (tid < on) {
+          uint4 a, b;
+          if (!await_entry(ovf_at(tag, ob, tid), W, tag, a, b, P.err)) gave_up = 1;
+          else take(X, Sv, Xn, Sn, a, b);
+        }
+        all();
+        if (gave_up) return false;
+        deliver_listed(P, me, f_n, f_j, f_c, lrow, acc, wid, lane, kT1 / 32);
+      }
+      all();
+      if (tid == 0) f_n = 0;
+      all();
+    }
+    return true;
+  };
+  if (tid == 0) {
+    f_n = blk_n = ov_n = in_n = 0;
+    next_grp = grp0;
+    gave_up = 0;
+  }
+  __syncthreads();
+  pc.mark(5);
+  bool ok = true;
+  float *X, *Sv, *Xn, *Sn;
+  if (wid >= help && help) {
+    const uint32_t h = tid - h0;
+    for (uint32_t s = 0; s < P.nsteps && ok; s++) {
+      const uint32_t tag = P.t1_tag + s + 1u;
+      buf(s, X, Sv, Xn, Sn);
+      deliver();
+      sums(Sv);
+      all();
+      if (s + 1 == P.nsteps) break;
+      if (h < np) {
+        float gv = 0.0f;
+        d_hits[h] = (uint8_t)draw_one<float>(P, me.post0 + h, P.t0 + s + 1, gv);
+        d_gauss[h] = gv;
+      }
+      asm volatile("bar.arrive 3, %0;" ::"n"(kT1) : "memory");
+      if (h == 0) {  // (last read before the barrier after the sums)
+        f_n = ov_n = in_n = 0;
+        next_grp = grp0;
+      }
+      advance_copies(X, Sv, Xn, Sn, h);
+      asm volatile("bar.sync 2, %0;" ::"n"(kT1) : "memory");
+      lists(X, Sv, Xn, Sn, tag, h);
+      all();
+      ok = overflow(X, Sv, Xn, Sn, tag);
+    }
+    return;
   }
   // ---- own neuron (thread tid owns post post0 + tid) ----
   const bool own = tid < np;
@@ -1846,263 +2049,170 @@ __global__ void __launch_bounds__(kT1, 1) k_prod1(const __grid_constant__ Params
   const uint32_t p = own ? me.post0 + tid : me.post0;
   NeuronPar<float> q;
   NeuronState<float> st;
-  if (active) load_neuron<float, kTM>(P, p, q, st);
+  if (active) load_neuron<float, kTM, kRec>(P, p, q, st);
   uint32_t nsp = 0;
-  if (own) {
-    float gv = 0.0f;
-    d_hits[tid] = (uint8_t)draw_one<float>(P, p, P.t0, gv);
-    d_gauss[tid] = gv;
-  }
-  PhaseClock pc;
-  pc.start(P);
-  unsigned long long target = 0;  // barrier arrivals so far (thread 0)
-  if (tid == 0) {
-    f_n = 0;
-    next_grp = 0;
-  }
-  __syncthreads();
-  pc.mark(5);
-  for (uint32_t s = 0; s < P.nsteps; s++) {
+  // what a neuron's next step needs and no other neuron decides: the drive's
+  // gates (hit: the draws) and the Mg block
+  float gauss = 0.0f, mgb = 1.0f;
+  auto ahead = [&](uint32_t hit) {
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+      if ((kRec >> r & 1u) && (q.a & act_of_rec(r))) st.est[r] = drive_linear<float>(st.est[r], q.dfs[r], (hit >> r) & 1u);
+    if (q.a & FS_ACT_NMDA)
+      drive_nmda<float>(st.ex, st.es, q.ndfxt, q.dfs[FS_NMDA], q.nefas, (hit >> FS_NMDA) & 1u);
+    mgb = mg_block<float>(q, st.V);
+  };
+  if (active) ahead(draw_one<float>(P, p, P.t0, gauss));
+  uint4 *const my_entry = P.t1_list + (((size_t)(tid / slots) * gridDim.x + blockIdx.x) * slots + tid % slots) * W;
+  // The neurons' step.  Only what depends on the step's deliveries and sums
+  // comes before the block's list entries are out; the rest is done while they
+  // travel.
+  auto neurons = [&](uint32_t s, uint32_t tag, bool last) {
     const uint64_t t = P.t0 + s;
-    float *X = (s & 1u) ? cx1 : cx0, *Sv = (s & 1u) ? cs1 : cs0;
-    // spike counts rotate over four slots: the slot of step t + 2 was last
-    // read in step t - 1, so it can be emptied now (every append to it comes
-    // after two more barriers)
-    if (blockIdx.x == 0 && tid == 0) __stcg(P.t1_cnt + ((uint32_t)(t + 2u) & 3u), 0u);
-    if (tid == 0) blk_n = 0;  // this step's spikes of the block (read after the NMDA sums' barrier)
-    if (s > 0) {
-      // ---- spikes of step t - 1 ----
-      // the buffer of this step already holds every copy advanced as if its
-      // neuron had not spiked (made during the barrier wait); the listed
-      // spikes are redone from the previous buffer, and their linear
-      // synapses onto this block are delivered
-      const float *Xo = (s & 1u) ? cx0 : cx1, *So = (s & 1u) ? cs0 : cs1;
-      const uint32_t par = (uint32_t)(t - 1u) & 1u;
-      const uint32_t tag = (uint32_t)(t - 1u) + 1u;  // entries of step t - 1 carry it
-      const uint32_t nreg = gridDim.x * P.t1_slots;   // block-region entries (<= kT1F)
-      const uint32_t W = P.t1_w;
-      const uint4 *reg = P.t1_list + (size_t)par * nreg * W;
-      const uint4 *ovf = P.t1_ovf + (size_t)par * n * W;
-      // the regions' entries are loaded with the overflow count (one round
-      // trip); stale entries carry another step's tag
-      uint4 a0 = make_uint4(0u, 0u, 0u, 0u), b0 = a0;
-      if (tid < nreg) {
-        a0 = __ldcg(reg + W * (size_t)tid);
-        if (W == 2) b0 = __ldcg(reg + 2 * (size_t)tid + 1);
-      }
-      const uint32_t cnt = nreg + __ldcg(P.t1_cnt + ((uint32_t)(t - 1u) & 3u));
-      pc.lap(8, cnt);    // the list's entry count is in
-      pc.lap(12, a0.x);  // thread 0's entries are in
-      for (uint32_t c0 = 0; c0 < cnt; c0 += kT1F) {
-        if (tid == 0) {
-          f_n = 0;
-          nf_n = 0;
-        }
-        __syncthreads();
-        const uint32_t i = c0 + tid;
-        if (tid < kT1F && i < cnt) {
-          uint4 a = a0, b = b0;
-          const bool over = i >= nreg;  // an overflow entry: every one is of step t - 1
-          if (over) {
-            a = __ldcg(ovf + W * (size_t)(i - nreg));
-            if (W == 2) b = __ldcg(ovf + 2 * (size_t)(i - nreg) + 1);
-          }
-          const bool cur = over || (W == 2 ? b.z : a.w) == tag;
-          const int j = cur ? find_tracked(bits, rank, me.w0, me.nwd, a.x) : -1;
-          if (j >= 0) {
-            const uint32_t sl = perm[j];
-            if (cls[sl] != 255) {
-              const uint32_t k = atomicAdd(&nf_n, 1u);
-              nf_j[k] = sl;
-              nf_inc[k] = __uint_as_float(a.y);
-            }
-            if (lrow[j + 1] > lrow[j]) {
-              const uint32_t k = atomicAdd(&f_n, 1u);
-              f_j[k] = (uint32_t)j;
-              f_c[k][0] = __uint_as_float(a.z);
-              f_c[k][1] = __uint_as_float(W == 2 ? a.w : a.z);
-              f_c[k][2] = __uint_as_float(W == 2 ? b.x : a.z);
-              f_c[k][3] = __uint_as_float(W == 2 ? b.y : a.z);
-            }
-          }
-        }
-        __syncthreads();
-        pc.lap(9);  // the look-ups are done
-        // the NMDA copies of the listed neurons (by slot), from their
-        // previous values
-        for (uint32_t k = tid; k < nf_n; k += kT1) {
-          const uint32_t sl = nf_j[k], c = cls[sl];
-          float xv = Xo[sl], sv = So[sl];
-          nmda_pre_step<float>(xv, sv, true, nf_inc[k], ctab[3 * c], ctab[3 * c + 1], ctab[3 * c + 2]);
-          X[sl] = xv;
-          Sv[sl] = sv;
-        }
-        // the deliveries of all but the last pass (the last pass's are made
-        // by the first warps while the others start the NMDA sums)
-        if (c0 + kT1F < cnt) {
-          deliver_listed(P, me, f_n, f_j, f_c, lrow, acc, wid, lane, kT1 / 32);
-          __syncthreads();
-          if (tid == 0) f_n = 0;
-        }
-        __syncthreads();
-      }
-      pc.mark(0);
-      pc.mark(1);
-    }
-    // ---- NMDA sums of the block's posts (order of nmda_pull1_f32) ----
-    // the first kDelW warps deliver the last pass's listed spikes (their
-    // synapse rows come from L2) and then join; every warp takes groups of
-    // four posts from a shared counter and walks the group's rows of 32
-    // entries: lane l of quarter h sums post 4g + h's edges l, l + 8, ... in
-    // order (then zero-weight fillers, which leave the sum unchanged), four
-    // rows loaded ahead, then the butterfly over 4, 2, 1
-    if (wid < kDelW) {
-      deliver_listed(P, me, f_n, f_j, f_c, lrow, acc, wid, lane, kDelW);
-      pc.lap(10);  // warp 0's deliveries are issued
-    }
-    for (;;) {
-      uint32_t g = 0;
-      if (lane == 0) g = atomicAdd(&next_grp, 1u);
-      g = __shfl_sync(fsd::kFull, g, 0);
-      if (g >= ng) break;
-      const uint32_t iend = grow[g + 1] * 32u;
-      uint32_t i = grow[g] * 32u + lane;
-      float sum = 0.0f;
-      for (; i + 96u < iend; i += 128u) {
-        const float w0 = ew[i], w1 = ew[i + 32], w2 = ew[i + 64], w3 = ew[i + 96];
-        const float v0 = Sv[eidx[i]], v1 = Sv[eidx[i + 32]], v2 = Sv[eidx[i + 64]], v3 = Sv[eidx[i + 96]];
-        sum = __fmaf_rn(w0, v0, sum);
-        sum = __fmaf_rn(w1, v1, sum);
-        sum = __fmaf_rn(w2, v2, sum);
-        sum = __fmaf_rn(w3, v3, sum);
-      }
-      for (; i < iend; i += 32u) sum = __fmaf_rn(ew[i], Sv[eidx[i]], sum);
+    long long rv[4];
 #pragma unroll
-      for (int o = 4; o; o >>= 1) sum += __shfl_xor_sync(fsd::kFull, sum, o);
-      const uint32_t qq = 4 * g + (lane >> 3);
-      if ((lane & 7u) == 0 && qq < np) gn[qq] = sum;
-    }
-    pc.lap(11);  // warp 0 found no more posts to sum
-    __syncthreads();
-    pc.mark(2);
-    // (the pass counters are reset behind the barrier above, for the next step)
-    if (tid == 0) {
-      f_n = 0;
-      next_grp = 0;
-    }
-    // ---- the neurons' step ----
-    if (active) {
-      long long rv[4];
-#pragma unroll
-      for (int r = 0; r < 4; r++) {
-        rv[r] = 0ll;
-        const int ri = P.lin_of_rec[r];
-        if (ri >= 0 && own) {
-          if (s == 0) {  // deliveries of the step before this launch: the ring
-            long long *slot = (long long *)ring_at(P, ri, p, (uint32_t)(t - 1u) & mask);
-            rv[r] = __ldcg(slot);
-            if (rv[r]) __stcg(slot, 0ll);
-          } else {
-            rv[r] = acc[(size_t)ri * kT1 + tid];
-            acc[(size_t)ri * kT1 + tid] = 0ll;
-          }
-        }
-      }
-      const uint32_t qs = own ? tid : 0;
-      float cinc[4], inc;
-      const bool spk =
-          neuron_step<float, kTM>(P, q, st, rv, gn[qs], d_hits[qs], d_gauss[qs], 0.0f, p, own, s, cinc, inc);
-      pc.lap(13, spk ? 1u : 0u);  // warp 0's neurons have stepped
-      nsp += spk ? 1u : 0u;
-      if (own && P.gv_row) gv_write<float>(P, p, s, st);
-      const uint32_t m = __ballot_sync(fsd::kFull, spk);
-      if (m) {
-        spike_outputs(P, m, spk, p, s, lane, false);
-        // the spike goes to this block's region of the step's list (a
-        // shared-memory counter); past the region's slots, to the overflow
-        // list (a global counter)
-        const uint32_t par = (uint32_t)t & 1u;
-        const int leader = __ffs(m) - 1;
-        uint32_t base = 0;
-        if ((int)lane == leader) base = atomicAdd(&blk_n, (uint32_t)__popc(m));
-        base = __shfl_sync(fsd::kFull, base, leader);
-        if (spk) {
-          const uint32_t k = base + __popc(m & ((1u << lane) - 1u));
-          const uint32_t W = P.t1_w;
-          uint4 *e;
-          if (k < P.t1_slots) {
-            e = P.t1_list + (((size_t)par * gridDim.x + blockIdx.x) * P.t1_slots + k) * W;
-          } else {
-            const uint32_t o = atomicAdd(P.t1_cnt + ((uint32_t)t & 3u), 1u);
-            e = P.t1_ovf + ((size_t)par * n + o) * W;
-          }
-          if (W == 2) {
-            __stcg(e, make_uint4(p, __float_as_uint(inc), __float_as_uint(cinc[0]), __float_as_uint(cinc[1])));
-            __stcg(e + 1, make_uint4(__float_as_uint(cinc[2]), __float_as_uint(cinc[3]), (uint32_t)t + 1u, 0u));
-          } else {
-            // at most one receptor's c is not 0: the sum is that c exactly
-            const float cl = ((cinc[0] + cinc[1]) + cinc[2]) + cinc[3];
-            __stcg(e, make_uint4(p, __float_as_uint(inc), __float_as_uint(cl), (uint32_t)t + 1u));
-          }
-        }
-        if (s + 1 == P.nsteps) {
-          // the launch's last step: its spikes go into the delay ring, which
-          // the next launch's first step folds
-          const uint32_t tm = (uint32_t)t & mask;
-          uint32_t rem = m;
-          while (rem) {
-            const int jl = __ffs(rem) - 1;
-            rem &= rem - 1;
-            const uint32_t qq = __shfl_sync(fsd::kFull, p, jl);
-            float cj[4];
-#pragma unroll
-            for (int r = 0; r < 4; r++) cj[r] = __shfl_sync(fsd::kFull, cinc[r], jl);
-            push_spike<float>(P, qq, tm, cj, lane, 32);
-          }
-        }
-      }
-    }
-    pc.mark(3);
-    if (s + 1 < P.nsteps) {
-      // while the barrier is awaited: the next step's drive draws, and every
-      // NMDA copy advanced into the other buffer as if its neuron had not
-      // spiked (the listed spikes are redone after the barrier)
-      const uint64_t tn = t + 1;
-      float *Xn = (s & 1u) ? cx0 : cx1, *Sn = (s & 1u) ? cs0 : cs1;
-      const bool ok = grid_sync_work(P.bar, P.err, gridDim.x, target, pc, [&]() {
-        for (uint32_t qq = tid - 32; qq < np; qq += kT1 - 32) {
-          float gv = 0.0f;
-          d_hits[qq] = (uint8_t)draw_one<float>(P, me.post0 + qq, tn, gv);
-          d_gauss[qq] = gv;
-        }
-        if (P.t1_ncls == 1) {  // one class (the usual case): its constants in registers
-          const float k0 = ctab[0], k1 = ctab[1], k2 = ctab[2];
-          for (uint32_t j = tid - 32; j < NS; j += kT1 - 32) {
-            if (cls[j] != 255) {
-              float xv = X[j], sv = Sv[j];
-              nmda_pre_step<float>(xv, sv, false, 1.0f, k0, k1, k2);
-              Xn[j] = xv;
-              Sn[j] = sv;
-            }
-          }
+    for (int r = 0; r < 4; r++) {
+      rv[r] = 0ll;
+      const int ri = P.lin_of_rec[r];
+      if ((kRec >> r & 1u) && ri >= 0 && own) {
+        if (s == 0) {  // deliveries of the step before this launch: the ring
+          long long *slot = (long long *)ring_at(P, ri, p, (uint32_t)(t - 1u) & mask);
+          rv[r] = __ldcg(slot);
+          if (rv[r]) __stcg(slot, 0ll);
         } else {
-          for (uint32_t j = tid - 32; j < NS; j += kT1 - 32) {
-            const uint32_t c = cls[j];
-            if (c != 255) {
-              float xv = X[j], sv = Sv[j];
-              nmda_pre_step<float>(xv, sv, false, 1.0f, ctab[3 * c], ctab[3 * c + 1], ctab[3 * c + 2]);
-              Xn[j] = xv;
-              Sn[j] = sv;
-            }
-          }
+          rv[r] = acc[(size_t)ri * kT1 + tid];
+          acc[(size_t)ri * kT1 + tid] = 0ll;
         }
-      });
-      if (!ok) return;
+      }
+    }
+    float g[5];
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+      g[r] = 0.0f;
+      if (!(kRec >> r & 1u)) continue;
+      if (P.lin_of_rec[r] >= 0) g[r] = st.G[r] = fold_linear<float>(q.dfs[r], st.G[r], rv[r]);
+      if (q.a & act_of_rec(r)) g[r] = __fmaf_rn(q.extg[r], st.est[r], g[r]);
+    }
+    g[FS_NMDA] = gn[own ? tid : 0] * P.rg[FS_NMDA];
+    if (q.a & FS_ACT_NMDA) g[FS_NMDA] = __fmaf_rn(q.extg[FS_NMDA], st.es, g[FS_NMDA]);
+    const bool spk = step_membrane<float, false, kRec>(P, q, st, g, gauss, 0.0f, p, own, s, nullptr, &mgb);
+    const uint32_t m = __ballot_sync(fsd::kFull, spk);
+    float cinc[4], inc;
+    if (m) {
+      uint32_t base = 0;
+      if (lane == 0) base = atomicAdd(&blk_n, (uint32_t)__popc(m));
+      base = __shfl_sync(fsd::kFull, base, 0);
+      spike_carries<float, kTM, kRec>(P, q, st, p, cinc, inc);
+      if (spk && !last) {
+        const uint32_t k = base + __popc(m & ((1u << lane) - 1u));
+        if (k < slots) {
+          sp_p[k] = p;
+          sp_inc[k] = inc;
+#pragma unroll
+          for (int r = 0; r < 4; r++) sp_c[k][r] = cinc[r];
+        } else {
+          put_entry(ovf_at(tag, blockIdx.x, k - slots), W, p, inc, cinc, tag);
+        }
+      }
+    }
+    pc.lap(13, m);  // warp 0's neurons have stepped
+    if (!last) {
+      // the region's entries, used or not, to every replica
+      asm volatile("bar.sync 1, %0;" ::"r"(nact * 32u) : "memory");
+      if (tid < reps * slots) {
+        const uint32_t cnt = blk_n, more = cnt > slots ? cnt - slots : 0u;
+        uint4 *e = my_entry + (tag & 1u) * (size_t)(reps * nreg * W);
+        const uint32_t k = tid % slots;
+        const bool on = k < cnt;
+        const float c[4] = {on ? sp_c[k][0] : 0.0f, on ? sp_c[k][1] : 0.0f, on ? sp_c[k][2] : 0.0f,
+                            on ? sp_c[k][3] : 0.0f};
+        put_entry(e, W, on ? sp_p[k] | (k == 0 ? more << 20 : 0u) : kNoSpike, on ? sp_inc[k] : 0.0f, c, tag);
+      }
+      if (wid == 0) {
+        __syncwarp();
+        if (lane == 0) blk_n = 0;
+      }
+    }
+    if (help && !last) asm volatile("bar.arrive 2, %0;" ::"n"(kT1) : "memory");
+    pc.mark(3);
+    if (m) {
+      spike_outputs(P, m, spk, p, s, lane, false);
+      if (last) {
+        // the launch's last step: its spikes go into the delay ring, which
+        // the next launch's first step folds
+        const uint32_t tm = (uint32_t)t & mask;
+        uint32_t rem = m;
+        while (rem) {
+          const int jl = __ffs(rem) - 1;
+          rem &= rem - 1;
+          const uint32_t qq = __shfl_sync(fsd::kFull, p, jl);
+          float cj[4];
+#pragma unroll
+          for (int r = 0; r < 4; r++) cj[r] = __shfl_sync(fsd::kFull, cinc[r], jl);
+          push_spike<float>(P, qq, tm, cj, lane, 32);
+        }
+      }
+    }
+    nsp += spk ? 1u : 0u;
+    step_pre<float, kTM, kRec>(P, q, st, spk, p, own, cinc, inc);
+    if (own && P.gv_row) gv_write<float>(P, p, s, st);
+  };
+  if (help) {
+    for (uint32_t s = 0; s < P.nsteps && ok; s++) {
+      const uint32_t tag = P.t1_tag + s + 1u;  // of this step's entries
+      const bool last = s + 1 == P.nsteps;
+      deliver();
+      pc.lap(10);  // warp 0's deliveries are issued
+      buf(s, X, Sv, Xn, Sn);
+      sums(Sv);
+      pc.lap(11);  // warp 0 found no more posts to sum
+      all();
+      pc.mark(2);
+      neurons(s, tag, last);
+      if (last) break;
+      asm volatile("bar.sync 3, %0;" ::"n"(kT1) : "memory");  // the draws are there
+      gauss = own ? d_gauss[tid] : 0.0f;
+      ahead(own ? d_hits[tid] : 0u);
       pc.mark(4);
+      all();
+      ok = overflow(X, Sv, Xn, Sn, tag);
+      pc.mark(0);
+    }
+  } else {
+    for (uint32_t s = 0; s < P.nsteps; s++) {
+      const uint32_t tag = P.t1_tag + s + 1u;
+      const bool last = s + 1 == P.nsteps;
+      buf(s, X, Sv, Xn, Sn);
+      deliver();
+      pc.lap(10);
+      sums(Sv);
+      pc.lap(11);  // warp 0 found no more posts to sum
+      __syncthreads();
+      pc.mark(2);
+      if (active) neurons(s, tag, last);
+      if (last) break;
+      if (tid == 0) {
+        f_n = ov_n = in_n = 0;
+        next_grp = grp0;
+      }
+      if (active) {
+        gauss = 0.0f;
+        const uint32_t hit = draw_one<float>(P, p, P.t0 + s + 1, gauss);
+        ahead(hit);
+      }
+      advance_copies(X, Sv, Xn, Sn, tid);
+      __syncthreads();
+      pc.mark(4);
+      lists(X, Sv, Xn, Sn, tag, tid);
+      __syncthreads();
+      ok = overflow(X, Sv, Xn, Sn, tag);
+      if (!ok) break;
+      pc.mark(0);
     }
   }
+  if (!ok) return;
   if (own) {
-    store_neuron<float, kTM>(P, p, q, st);
+    store_neuron<float, kTM, kRec>(P, p, q, st);
     if (P.nspk && nsp) P.nspk[p] += nsp;
   }
   // the launch's spikes, added to the total once per warp
@@ -2193,6 +2303,7 @@ struct Prod {
   bool single = false;     // runs on the single-step kernel k_prod1
   struct Tiles *tiles = nullptr;  // runs on the tile kernels (large networks)
   uint32_t b1_blocks = 0;  // its blocks (one per SM at most)
+  uint32_t t1_tag = 0;     // steps it has listed
   unsigned long long *phase_buf = nullptr;  // phase clock counters (debug aid)
   bool wide = false;  // some block's posts span several tiles: eight NMDA edges in flight
   bool ltp = false;   // long-term plasticity: runs on k_prod_ltp
@@ -2364,6 +2475,15 @@ int tiles_solo_create(Prod *p, std::string &err);
 
 namespace {
 
+// The single-step kernel's instance.
+const void *single_kernel(const Params &P) {
+  const bool two = (P.live & 12u) == 0;  // neither ACh nor GluCl is live
+  if (P.plast == PL_TM) return two ? (const void *)k_prod1<true, 3> : (const void *)k_prod1<true, 15>;
+  return two ? (const void *)k_prod1<false, 3> : (const void *)k_prod1<false, 15>;
+}
+// Bytes of its lists with `slots` entries a block.
+size_t t1_bytes(const Prod *p, uint32_t slots) { return (size_t)2 * p->b1_blocks * slots * p->P.t1_w * sizeof(uint4); }
+
 int launch(Prod *p, uint32_t nsteps, bool want_bits, bool wantV, cudaStream_t st, uint64_t *launches,
            std::string &err, bool wantI = false, bool wantNS = false, bool wantGV = false) {
   int rc = ensure_buffers(p, nsteps, wantV, wantI, wantNS, err);
@@ -2408,13 +2528,21 @@ int launch(Prod *p, uint32_t nsteps, bool want_bits, bool wantV, cudaStream_t st
     }
     p->ev.push_back({a, b});
   }
-  // the single-step kernel's lists start empty (region entries are told
-  // apart by their step tag; a reset or a restored checkpoint moves the
-  // step counter back)
-  if (p->single && (cudaMemsetAsync(P.t1_cnt, 0, 16, st) != cudaSuccess ||
-                    cudaMemsetAsync(P.t1_list, 0, (size_t)2 * p->b1_blocks * P.t1_slots * 16 * P.t1_w, st) != cudaSuccess)) {
-    err = "memset";
-    return FS_ERR_CUDA;
+  // tags of the single-step kernel's lists count the steps listed, not the
+  // network's (a reset or a restored checkpoint moves those back): an entry of
+  // an earlier step never carries a later one's.  They start anew, with empty
+  // lists, before they wrap.
+  if (p->single) {
+    if (p->t1_tag > 0xffffffffu - nsteps - 1u) {
+      p->t1_tag = 0;
+      if (cudaMemsetAsync(P.t1_list, 0, t1_bytes(p, P.t1_reps * P.t1_slots), st) != cudaSuccess ||
+          cudaMemsetAsync(P.t1_ovf, 0, t1_bytes(p, kT1), st) != cudaSuccess) {
+        err = "memset";
+        return FS_ERR_CUDA;
+      }
+    }
+    P.t1_tag = p->t1_tag;
+    p->t1_tag += nsteps - 1;  // (the last step's spikes go into the ring)
   }
   const auto &evp = p->ev[p->ev_used];
   cudaEventRecord(evp.first, st);
@@ -2435,8 +2563,7 @@ int launch(Prod *p, uint32_t nsteps, bool want_bits, bool wantV, cudaStream_t st
     if (e == cudaSuccess)
       e = cudaLaunchCooperativeKernel(ltp_kernel(p), p->blocks, kThreads, args, smem, st);
   } else if (p->single) {
-    const void *k1 = P.plast == PL_TM ? (const void *)k_prod1<true> : (const void *)k_prod1<false>;
-    e = cudaLaunchCooperativeKernel(k1, p->b1_blocks, kT1, args, P.t1_smem, st);
+    e = cudaLaunchCooperativeKernel(single_kernel(P), p->b1_blocks, kT1, args, P.t1_smem, st);
   } else {
     e = cudaLaunchCooperativeKernel(prod_kernel(p), p->blocks, kThreads, args, smem, st);
   }
@@ -2601,9 +2728,9 @@ struct Single {
 };
 
 // Shared memory of k_prod1's tables for one block (the kernel's layout):
-// accumulators | x, s copies x2 (per slot) | class table | edge weights |
-// bitmap | group rows | edge slots | ranks | linear rows | slots of the
-// tracked neurons | classes (per slot).
+// accumulators | x, s copies x2 (per slot) | edge weights | edge slots | classes
+// (per slot) | class table | bitmap | group rows | ranks | linear rows | slots
+// of the tracked neurons.
 static size_t single_smem(uint32_t nlin, uint32_t ncls, const Blk1 &k) {
   const size_t ng = ((size_t)k.np + 3) / 4;
   return (size_t)std::max(1u, nlin) * kT1 * 8 + (size_t)k.nslot * 16 + 3 * (size_t)ncls * 4 + (size_t)k.ne * 4 +
@@ -3274,13 +3401,13 @@ static int prod_create_from(Prod **out, const fs_net_desc *d, const fs_run_opts 
       cudaGetDevice(&dev);
       cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
       cudaFuncAttributes fa{};
-      cudaFuncGetAttributes(&fa, (const void *)k_prod1<true>);
+      cudaFuncGetAttributes(&fa, (const void *)k_prod1<true, 15>);
       const int dyn_max = std::min<int>(200 * 1024, maxsm - (int)fa.sharedSizeBytes);
-      if ((int)S1.smem <= dyn_max &&
-          cudaFuncSetAttribute((const void *)k_prod1<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn_max) ==
-              cudaSuccess &&
-          cudaFuncSetAttribute((const void *)k_prod1<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn_max) ==
-              cudaSuccess) {
+      bool fits = (int)S1.smem <= dyn_max;
+      for (const void *k : {(const void *)k_prod1<false, 3>, (const void *)k_prod1<false, 15>,
+                            (const void *)k_prod1<true, 3>, (const void *)k_prod1<true, 15>})
+        fits = fits && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn_max) == cudaSuccess;
+      if (fits) {
         if ((rc = dup(p, (Blk1 **)&P.b1, S1.blk.data(), S1.blk.size(), st, err))) goto fail;
         UPU(t1_gid, S1.gid.data(), S1.gid.size());
         if ((rc = dup(p, (uint16_t **)&P.t1_lrow, S1.lrow.data(), S1.lrow.size(), st, err))) goto fail;
@@ -3294,15 +3421,15 @@ static int prod_create_from(Prod **out, const fs_net_desc *d, const fs_run_opts 
         if ((rc = dup(p, (uint16_t **)&P.t1_eidx, S1.eidx.data(), S1.eidx.size(), st, err))) goto fail;
         UPU(t1_bits, S1.bits.data(), S1.bits.size());
         if ((rc = dup(p, (uint16_t **)&P.t1_rank, S1.rank.data(), S1.rank.size(), st, err))) goto fail;
-        if ((rc = dup(p, &P.t1_cnt, (const uint32_t *)nullptr, 4, st, err))) goto fail;
-        P.t1_slots = std::min<uint32_t>(16, kT1F / (uint32_t)S1.blk.size());
+        P.t1_slots = std::min<uint32_t>(kSlots, kT1F / (uint32_t)S1.blk.size());
         // one 16-byte word per listed spike when no neuron projects onto two
         // linear receptors (its one c travels alone), else two
         P.t1_w = 1;
         for (uint32_t i = 0; i < n; i++)
           if (__builtin_popcount(proj[i] & 15u) > 1) P.t1_w = 2;
-        if ((rc = dup(p, &P.t1_list, (const uint4 *)nullptr, (size_t)2 * S1.blk.size() * P.t1_slots * 2, st, err)) ||
-            (rc = dup(p, &P.t1_ovf, (const uint4 *)nullptr, (size_t)4 * n, st, err)))
+        P.t1_reps = 32 / P.t1_slots;  // (one warp writes them)
+        if ((rc = dup(p, &P.t1_list, (const uint4 *)nullptr, (size_t)2 * P.t1_reps * S1.blk.size() * P.t1_slots * P.t1_w, st, err)) ||
+            (rc = dup(p, &P.t1_ovf, (const uint4 *)nullptr, (size_t)2 * S1.blk.size() * kT1 * P.t1_w, st, err)))
           goto fail;
         P.t1_ncls = (uint32_t)(S1.tab.size() / 3);
         P.t1_smem = S1.smem;
@@ -4163,10 +4290,9 @@ int prod_debug_drive(Prod *p, uint64_t t0, uint32_t nsteps, uint32_t first, uint
 }
 
 // Phase clock: per block, SM cycles spent in each phase of the persistent
-// kernels since it was switched on (k_prod1: 0 spike-list lookups, 1 NMDA
-// copies of listed spikes, 2 last deliveries and NMDA sums, 3 neuron steps
-// and spike lists, 6 thread 0's barrier wait, 4 the rest of the barrier,
-// 5 set-up; k_prod: 0 NMDA pull, 1 drive draws, 9 conductances, 2 membranes and
+// kernels since it was switched on (k_prod1: 0 wait for the other blocks' lists
+// and their look-ups, 2 deliveries and NMDA sums, 3 membranes and list entries,
+// 4 presynaptic state and the next step's drive, 5 set-up; k_prod: 0 NMDA pull, 1 drive draws, 9 conductances, 2 membranes and
 // presynaptic state, 3 history and pushes, 4 grid barrier).
 int prod_phase_clock(Prod *p, int enable, cudaStream_t st, std::string &err) {
   const uint32_t nb = std::max(p->blocks, p->b1_blocks);
