@@ -371,8 +371,15 @@ __device__ __forceinline__ void nmda_pull_f32(const Params &P, uint32_t p0, uint
 // kDense: s of step tb - 1 is read from s_pre itself (4 B a neuron, several of
 // a region's sources in one line) instead of the history (128 B a neuron: a
 // line per edge); for kernels that do not step any neuron between the start
-// and the end of a pull.  Four of a lane's edges are in flight.
-template <bool kMW, bool kDense, uint32_t KT>
+// and the end of a pull.  U of a lane's edges are in flight.  What bounds the
+// pull is two dependent L2 round trips per U edges (the edge's source and
+// weight, then s): with U = 4 and a post's ~84 edges over eight lanes that was
+// eight to twelve round trips for each of a warp's two or three groups of posts
+// (12,100 cycles a step of k_prod_ltp on the 20k connectome).  U = 12 takes most
+// posts at once, and the next group's sources and weights are read while the
+// gathers are under way: 9,000 cycles, 27.3 -> 24.5 us a step (U = 16: 25.1);
+// kernels with 64 registers (k_tile_pull) keep U = 4.
+template <bool kMW, bool kDense, uint32_t KT, uint32_t U>
 __device__ __forceinline__ void nmda_pull1_f32(const Params &P, uint32_t p0, uint32_t np, uint64_t tb,
                                                float (*gn)[KT], uint32_t wid, uint32_t lane) {
   const uint32_t nw = kThreads / 32;
@@ -384,29 +391,48 @@ __device__ __forceinline__ void nmda_pull1_f32(const Params &P, uint32_t p0, uin
   const float *sh = kDense ? (const float *)P.s_pre : (const float *)P.s_hist + ((uint32_t)(tb - 1u) & P.mask);
   const size_t stride = kDense ? 1u : kSH * P.slots;
   const uint32_t h = lane >> 3, l8 = lane & 7u;
+  auto bounds = [&](uint32_t q, uint32_t &b0, uint32_t &b1) {
+    b0 = q < np ? __ldg(P.in_row + p0 + q) : 0u;
+    b1 = q < np ? __ldg(P.in_row + p0 + q + 1) : 0u;
+  };
+  uint32_t pre[U];
+  float w[U];
+  auto edges = [&](uint32_t e, uint32_t b1) {
+#pragma unroll
+    for (uint32_t u = 0; u < U; u++) {
+      const bool ok = e + 8u * u < b1;
+      pre[u] = ok ? __ldg(P.in_code + e + 8u * u) & 0xffffffu : 0u;
+      w[u] = ok ? (kMW ? __ldcg(P.in_w + e + 8u * u) : __ldg(P.in_w + e + 8u * u)) : 0.0f;
+    }
+  };
+  uint32_t b0, b1, n0, n1;
+  bounds(wid * 4u + h, b0, b1);
+  edges(b0 + l8, b1);
   for (uint32_t q0 = wid * 4u; q0 < np; q0 += nw * 4u) {
-    const uint32_t q = q0 + h;
-    const bool has = q < np;
-    const uint32_t b0 = has ? __ldg(P.in_row + p0 + q) : 0u, b1 = has ? __ldg(P.in_row + p0 + q + 1) : 0u;
+    bounds(q0 + nw * 4u + h, n0, n1);
     float acc = 0.0f;
-    for (uint32_t e = b0 + l8; e < b1; e += 32) {
-      uint32_t pre[4];
-      float w[4], v[4];
+    for (uint32_t e = b0 + l8;;) {
+      float v[U], c[U];
 #pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const bool ok = e + 8u * u < b1;
-        pre[u] = ok ? __ldg(P.in_code + e + 8u * u) & 0xffffffu : 0u;
-        w[u] = ok ? (kMW ? __ldcg(P.in_w + e + 8u * u) : __ldg(P.in_w + e + 8u * u)) : 0.0f;
+      for (uint32_t u = 0; u < U; u++) {
+        v[u] = e + 8u * u < b1 ? __ldca(sh + pre[u] * stride) : 0.0f;
+        c[u] = w[u];
       }
+      const uint32_t at = e;
+      e += 8u * U;
+      // the lanes' next edges, or the next group's first ones
+      const bool more = __any_sync(fsd::kFull, e < b1);
+      edges(more ? e : n0 + l8, more ? b1 : n1);
 #pragma unroll
-      for (int u = 0; u < 4; u++) v[u] = e + 8u * u < b1 ? __ldca(sh + pre[u] * stride) : 0.0f;
-#pragma unroll
-      for (int u = 0; u < 4; u++)
-        if (e + 8u * u < b1) acc = __fmaf_rn(w[u], v[u], acc);
+      for (uint32_t u = 0; u < U; u++)
+        if (at + 8u * u < b1) acc = __fmaf_rn(c[u], v[u], acc);
+      if (!more) break;
     }
 #pragma unroll
     for (int o = 4; o; o >>= 1) acc += __shfl_xor_sync(fsd::kFull, acc, o);
-    if (l8 == 0 && has) gn[0][q] = acc;
+    if (l8 == 0 && q0 + h < np) gn[0][q0 + h] = acc;
+    b0 = n0;
+    b1 = n1;
   }
 }
 
@@ -1268,7 +1294,7 @@ __device__ __forceinline__ void tile_pull(const Params &P, uint32_t tp0, uint32_
                                           TileBufs<T, KT> &B) {
   const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   if constexpr (sizeof(T) == 4) {
-    if (P.dmax0) nmda_pull1_f32<false, false, KT>(P, tp0, np, P.t0 + bs, (float (*)[KT])B.gn, wid, lane);
+    if (P.dmax0) nmda_pull1_f32<false, false, KT, 4>(P, tp0, np, P.t0 + bs, (float (*)[KT])B.gn, wid, lane);
     else nmda_pull_f32<PU, KT>(P, tp0, np, P.t0 + bs, L, (float (*)[KT])B.gn, wid, lane);
   } else {
     nmda_pull<T, KT>(P, tp0, np, P.t0 + bs, L, B.gn, wid, lane);
@@ -1536,7 +1562,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1) k_prod_ltp(c
       for (uint32_t tp0 = B0; tp0 < B1; tp0 += kT) {
         const uint32_t np = min(kT, B1 - tp0);
         T(*gn)[kT] = (T(*)[kT])((T *)P.ltp_gn + tp0);
-        if constexpr (sizeof(T) == 4) nmda_pull1_f32<true, true, KT>(P, tp0, np, t, (float(*)[KT])gn, wid, lane);
+        if constexpr (sizeof(T) == 4) nmda_pull1_f32<true, true, KT, 12>(P, tp0, np, t, (float(*)[KT])gn, wid, lane);
         else nmda_pull1_f64<true>(P, tp0, np, (double *)gn[0], wid, lane);
       }
       pc.mark(0);
@@ -2257,7 +2283,7 @@ __global__ void __launch_bounds__(kThreads, U == 4 ? 4 : 2) k_tile_pull(const Pa
   const Params &P = Psh;
   const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   if constexpr (sizeof(T) == 4) {
-    if (P.dmax0) nmda_pull1_f32<false, true, TileW<T>::W>(P, tl.p0, tl.np, P.t0 + bs, (float (*)[TileW<T>::W])gn, wid, lane);
+    if (P.dmax0) nmda_pull1_f32<false, true, TileW<T>::W, 4>(P, tl.p0, tl.np, P.t0 + bs, (float (*)[TileW<T>::W])gn, wid, lane);
     else nmda_pull_f32<U, TileW<T>::W>(P, tl.p0, tl.np, P.t0 + bs, L, (float (*)[TileW<T>::W])gn, wid, lane);
   } else {
     if (P.dmax0) nmda_pull1_f64<false>(P, tl.p0, tl.np, (double *)gn[0], wid, lane);
