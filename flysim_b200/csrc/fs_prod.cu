@@ -57,6 +57,7 @@ using fsd::grid_sync;
 constexpr double kFix = 1099511627776.0;           // 2^40
 constexpr double kInvFix = 9.094947017729282e-13;  // 2^-40
 constexpr uint32_t kThreads = 256;
+constexpr uint32_t kThreads64 = 512;  // of k_prod in FP64 (see k_prod)
 constexpr uint32_t kTile = 256;  // post neurons advanced together (one per thread)
 constexpr uint32_t kLB = 16;     // steps per NMDA pull batch
 // posts per tile (FP64 tiles are half as wide so the per-tile buffers stay
@@ -454,12 +455,12 @@ __device__ __forceinline__ void nmda_pull1_f64(const Params &P, uint32_t p0, uin
   }
 }
 
-template <class T, uint32_t KT>
+template <class T, uint32_t KT, uint32_t NT = kThreads>
 __device__ __forceinline__ void nmda_pull(const Params &P, uint32_t p0, uint32_t np, uint64_t tb, uint32_t L,
                                           T (*gn)[KT], uint32_t wid, uint32_t lane) {
   const T *sh = (const T *)P.s_hist;
   const uint32_t S = P.slots, mask = P.mask;
-  const uint32_t nw = kThreads / 32;
+  const uint32_t nw = NT / 32;
   for (uint32_t q = wid; q < np; q += nw) {
     T acc[kLB];
 #pragma unroll
@@ -564,10 +565,10 @@ __device__ __forceinline__ uint32_t draw_one(const Params &P, uint32_t p, uint64
 
 // Draws of L steps for a tile, by all threads at once, off the neurons'
 // per-step dependency chain.
-template <class T, uint32_t KT>
+template <class T, uint32_t KT, uint32_t NT = kThreads>
 __device__ __forceinline__ void draw_inputs(const Params &P, uint32_t p0, uint32_t np, uint64_t tb, uint32_t L,
                                             uint8_t (*hits)[KT], T (*gauss)[KT]) {
-  for (uint32_t idx = threadIdx.x; idx < np * L; idx += kThreads) {
+  for (uint32_t idx = threadIdx.x; idx < np * L; idx += NT) {
     const uint32_t j = idx / np, q = idx - j * np;
     T gv = (T)0;
     hits[j][q] = (uint8_t)draw_one<T>(P, p0 + q, tb + j, gv);
@@ -1273,23 +1274,23 @@ __device__ __forceinline__ void tile_neurons(const Params &P, uint32_t p0, uint3
 
 // The s values of a batch of L steps (tile_neurons leaves them in gn) into the
 // history, by the whole block; FP32: the shifted rows.
-template <class T, uint32_t KT>
+template <class T, uint32_t KT, uint32_t NT>
 __device__ __forceinline__ void store_history(const Params &P, uint32_t p0, uint32_t np, uint64_t tb, uint32_t L,
                                               const T (*gn)[KT]) {
   // thread: step j of the batch, row k of neurons q, q + 16 / K, ... (a neuron
   // that projects on no NMDA receptor stores its zeros, which nothing reads)
   constexpr uint32_t K = sizeof(T) == 4 ? kSH : 1u;
-  static_assert(kLB == 16 && kThreads % (16 * K) == 0, "a thread's step and row are fixed");
+  static_assert(kLB == 16 && NT % (16 * K) == 0, "a thread's step and row are fixed");
   const uint32_t S = P.slots, j = threadIdx.x & 15u, k = (threadIdx.x >> 4) & (K - 1u);
   if (j >= L) return;
   const T *src = gn[j];
   T *dst = (T *)P.s_hist + ((size_t)p0 * K + k) * S + (((uint32_t)tb + j - k) & P.mask);
 #pragma unroll 4
-  for (uint32_t q = threadIdx.x / (16 * K); q < np; q += kThreads / (16 * K)) __stcg(dst + (size_t)q * K * S, src[q]);
+  for (uint32_t q = threadIdx.x / (16 * K); q < np; q += NT / (16 * K)) __stcg(dst + (size_t)q * K * S, src[q]);
 }
 
 // NMDA sums of L steps for a tile's posts into B.gn.
-template <class T, int PU, uint32_t KT>
+template <class T, int PU, uint32_t KT, uint32_t NT>
 __device__ __forceinline__ void tile_pull(const Params &P, uint32_t tp0, uint32_t np, uint32_t bs, uint32_t L,
                                           TileBufs<T, KT> &B) {
   const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -1297,16 +1298,16 @@ __device__ __forceinline__ void tile_pull(const Params &P, uint32_t tp0, uint32_
     if (P.dmax0) nmda_pull1_f32<false, false, KT, 4>(P, tp0, np, P.t0 + bs, (float (*)[KT])B.gn, wid, lane);
     else nmda_pull_f32<PU, KT>(P, tp0, np, P.t0 + bs, L, (float (*)[KT])B.gn, wid, lane);
   } else {
-    nmda_pull<T, KT>(P, tp0, np, P.t0 + bs, L, B.gn, wid, lane);
+    nmda_pull<T, KT, NT>(P, tp0, np, P.t0 + bs, L, B.gn, wid, lane);
   }
 }
 
 // Gap currents of step bs of a tile's posts (interval 1): g (V_other -
 // V_self) over V at the end of the previous step (none before the first).
-template <class T>
+template <class T, uint32_t NT = kThreads>
 __device__ __forceinline__ void tile_gap(const Params &P, uint32_t tp0, uint32_t np, uint32_t bs, T *gapI) {
   const uint64_t t = P.t0 + bs;
-  for (uint32_t q = threadIdx.x; q < np; q += kThreads) {
+  for (uint32_t q = threadIdx.x; q < np; q += NT) {
     T acc = (T)0;
     if (t > 0) {
       const T *vp = (const T *)P.Vg + (size_t)((t - 1u) & 1u) * P.n;
@@ -1333,18 +1334,18 @@ __device__ __forceinline__ void tile_gap(const Params &P, uint32_t tp0, uint32_t
 // state 280, history and pushes 290; with the barrier 4.06 -> 3.88 us a step.
 // The 200k network's tile kernels (more posts than threads to start with)
 // gain from the shorter inner loops: 34.2 -> 30.8 us a step.
-template <class T, uint32_t KT>
+template <class T, uint32_t KT, uint32_t NT = kThreads>
 __device__ __forceinline__ void tile_steps(const Params &P, uint32_t tp0, uint32_t np, uint32_t bs, uint32_t L,
                                            TileBufs<T, KT> &B, PhaseClock &pc, bool hist) {
   constexpr uint32_t kCap = TileBufs<T, KT>::kCap;
   const SpikeList<T> lst{&B.l_n, B.l_p, B.l_tm, B.l_c, kCap};
   const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const uint32_t items = cond_items<T>(P, np);
-  draw_inputs<T, KT>(P, tp0, np, P.t0 + bs, L, B.hits, B.gauss(P));
-  if (P.gap_row) tile_gap<T>(P, tp0, np, bs, B.gapI);
+  draw_inputs<T, KT, NT>(P, tp0, np, P.t0 + bs, L, B.hits, B.gauss(P));
+  if (P.gap_row) tile_gap<T, NT>(P, tp0, np, bs, B.gapI);
   __syncthreads();
   pc.mark(1);
-  for (uint32_t i = tid; i < items; i += kThreads) {
+  for (uint32_t i = tid; i < items; i += NT) {
     CondItem<T> I;
     cond_load<T>(P, tp0, np, bs, L, i, I);
     cond_steps<T, KT>(P, tp0, bs, L, I, B.gn, B.hits, B.lin());
@@ -1354,20 +1355,20 @@ __device__ __forceinline__ void tile_steps(const Params &P, uint32_t tp0, uint32
   tile_neurons<T, false, true, KT>(P, tp0, np, bs, L, B.gn, B.lin(), B.gauss(P), lst, B.gapI);
   __syncthreads();
   pc.mark(2);
-  if (hist) store_history<T, KT>(P, tp0, np, P.t0 + bs, L, B.gn);
+  if (hist) store_history<T, KT, NT>(P, tp0, np, P.t0 + bs, L, B.gn);
   // the batch's spikes: with fewer spikes than warps the whole block
   // walks each spike's out-edges (a hub's hundreds of edges in one or
   // two rounds); with more, one spike per warp, eight in flight
   const uint32_t nl = min(B.l_n, kCap);
-  if (nl < kThreads / 32) {
+  if (nl < NT / 32) {
     for (uint32_t k = 0; k < nl; k++) {
       T cj[4];
 #pragma unroll
       for (int r = 0; r < 4; r++) cj[r] = B.l_c[k][r];
-      push_spike<T>(P, B.l_p[k], B.l_tm[k], cj, tid, kThreads);
+      push_spike<T>(P, B.l_p[k], B.l_tm[k], cj, tid, NT);
     }
   } else {
-    for (uint32_t k = wid; k < nl; k += kThreads / 32) {
+    for (uint32_t k = wid; k < nl; k += NT / 32) {
       T cj[4];
 #pragma unroll
       for (int r = 0; r < 4; r++) cj[r] = B.l_c[k][r];
@@ -1382,7 +1383,7 @@ __device__ __forceinline__ void tile_steps(const Params &P, uint32_t tp0, uint32
 // The steps of one block: posts [B0, B1) of the network P, whose blocks
 // (nblk of them) meet at a barrier after every interval.  PU: NMDA edges in
 // flight per lane in the pull (results do not depend on it).
-template <class T, int PU, uint32_t KT>
+template <class T, int PU, uint32_t KT, uint32_t NT>
 __device__ __forceinline__ void prod_blocks(const Params &P, uint32_t B0, uint32_t B1, uint32_t nblk) {
   constexpr uint32_t kT = KT;
   extern __shared__ __align__(16) unsigned char smt[];
@@ -1399,9 +1400,9 @@ __device__ __forceinline__ void prod_blocks(const Params &P, uint32_t B0, uint32
       const uint32_t L = min(kLB, iv_end - bs);
       for (uint32_t tp0 = B0; tp0 < B1; tp0 += kT) {
         const uint32_t np = min(kT, B1 - tp0);
-        tile_pull<T, PU, KT>(P, tp0, np, bs, L, B);
+        tile_pull<T, PU, KT, NT>(P, tp0, np, bs, L, B);
         pc.mark(0);
-        tile_steps<T, KT>(P, tp0, np, bs, L, B, pc, P.in_row != nullptr);
+        tile_steps<T, KT, NT>(P, tp0, np, bs, L, B, pc, P.in_row != nullptr);
       }
     }
     s = iv_end;
@@ -1412,15 +1413,19 @@ __device__ __forceinline__ void prod_blocks(const Params &P, uint32_t B0, uint32
   }
 }
 
-// FP32: two blocks per SM (128 registers); FP64 runs one block per SM.  PU
+// FP32: two blocks per SM (128 registers); FP64 runs one block per SM, of 512
+// threads: its pull takes a warp per post and waits for its scattered loads
+// (5,000 neurons, 34 posts a block: 4,500 cycles a step with eight warps, 3,250
+// with sixteen; 4.57 -> 3.96 us a step).  PU
 // NMDA edges in flight per lane: four when a block's posts fit one tile
 // (20k connectome: 4.05 us per timestep against 4.71 with eight), eight when
 // they span several (250k network: 43.3 against 46.3 us); ring slots two
 // steps ahead (4.60 us with one).  Batches of small networks run eight edges
 // and one step ahead (their kernel has fewer registers to spare).
 template <class T, int PU, uint32_t KT>
-__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1) k_prod(const __grid_constant__ Params P) {
-  prod_blocks<T, PU, KT>(P, P.block_post[blockIdx.x], P.block_post[blockIdx.x + 1], gridDim.x);
+__global__ void __launch_bounds__(sizeof(T) == 4 ? kThreads : kThreads64, sizeof(T) == 4 ? 2 : 1)
+    k_prod(const __grid_constant__ Params P) {
+  prod_blocks<T, PU, KT, sizeof(T) == 4 ? kThreads : kThreads64>(P, P.block_post[blockIdx.x], P.block_post[blockIdx.x + 1], gridDim.x);
 }
 
 // ---- long-term plasticity (networks with LTP, delays 0) ---------------------
@@ -2426,6 +2431,7 @@ const void *prod_kernel(const Prod *p) {
   if (p->wide) return (const void *)k_prod<float, 8, 256>;
   return p->max_posts <= 128 ? (const void *)k_prod<float, 4, 128> : (const void *)k_prod<float, 4, 256>;
 }
+uint32_t prod_threads(const Prod *p) { return p->fp64 && !p->ltp ? kThreads64 : kThreads; }
 const void *ltp_kernel(const Prod *p) {
   if (p->fp64) return (const void *)k_prod_ltp<double, 128>;
   return p->max_posts <= 128 ? (const void *)k_prod_ltp<float, 128> : (const void *)k_prod_ltp<float, 256>;
@@ -2591,7 +2597,7 @@ int launch(Prod *p, uint32_t nsteps, bool want_bits, bool wantV, cudaStream_t st
   } else if (p->single) {
     e = cudaLaunchCooperativeKernel(single_kernel(P), p->b1_blocks, kT1, args, P.t1_smem, st);
   } else {
-    e = cudaLaunchCooperativeKernel(prod_kernel(p), p->blocks, kThreads, args, smem, st);
+    e = cudaLaunchCooperativeKernel(prod_kernel(p), p->blocks, prod_threads(p), args, smem, st);
   }
   cudaEventRecord(evp.second, st);
   if (e != cudaSuccess) {
@@ -3314,7 +3320,7 @@ static int prod_create_from(Prod **out, const fs_net_desc *d, const fs_run_opts 
                          : (p->fp64 ? (const void *)k_prod<double, 4, 128> : (const void *)k_prod<float, 4, 256>);
     // (at the largest shared memory a change of the drive can ask for)
     tile_attributes();
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kq, kThreads, p->fp64 ? tile_smem<double, 128>(kLiveAll) : tile_smem<float, 256>(kLiveAll));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kq, (int)(p->fp64 && !ltp ? kThreads64 : kThreads), p->fp64 ? tile_smem<double, 128>(kLiveAll) : tile_smem<float, 256>(kLiveAll));
   }
   if (occ < 1) occ = 1;
   int per_sm = std::min(occ, 4);
@@ -3738,7 +3744,7 @@ void prod_info(const Prod *p, ProdInfo *info) {
   info->slots = p->P.slots;
   info->interval = p->P.interval;
   info->blocks = p->single ? p->b1_blocks : p->blocks;
-  info->threads = p->single ? kT1 : kThreads;
+  info->threads = p->single ? kT1 : p->tiles ? kThreads : prod_threads(p);
   info->single_step = p->single ? 1 : 0;
   info->tiles = p->tiles ? 1 : 0;
   info->ltp = p->ltp ? 1 : 0;
