@@ -1623,7 +1623,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1) k_prod_ltp(c
 
 // ---- single-step persistent kernel (networks whose delays are all 0) -------
 // Every network in the reference's own format has no synaptic delays, so a
-// spike of step t acts in step t + 1 and every step ends at a grid barrier.
+// spike of step t acts in step t + 1: the blocks exchange their spikes every step.
 // k_prod1 keeps everything a block reads from other neurons in its own
 // shared memory, so the only traffic between blocks per step is the list of
 // the step's spikes:
@@ -1687,11 +1687,11 @@ __device__ __forceinline__ int find_tracked(const uint32_t *bits, const uint16_t
   return (int)rank[w] + __popc(word & ((1u << b) - 1u));
 }
 
-// Deliveries of a pass of listed spikes onto a block (k_prod1): warp w of
+// Deliveries of the listed spikes onto a block (k_prod1): warp w of
 // nw takes listed spikes w, w + nw, ... and walks the spike's synapse row
 // onto the block's posts, adding w * c (receptor gain applied) as 2^-40
 // fixed point into the per-post accumulators.
-constexpr uint32_t kDelW = 4;  // warps that deliver the last pass
+constexpr uint32_t kDelW = 4;  // warps that deliver in a block without helpers
 __device__ __forceinline__ void deliver_listed(const Params &P, const Blk1 &me, uint32_t nf, const uint32_t *f_j,
                                                const float (*f_c)[4], const uint16_t *lrow, long long *acc,
                                                uint32_t w, uint32_t lane, uint32_t nw) {
