@@ -848,11 +848,13 @@ __device__ __forceinline__ bool step_membrane(const Params &P, const NeuronPar<T
     }
     st.V = fma_t<T>(q.df, v, mul_t(q.ef, I));
     if (P.outI && own) {  // kept only while requested (code/EqsGnl2.cpp:196-206)
-      P.Irep[p] = (float)((live & 1u) ? mul_t(g[FS_AMPA], q.vrev[FS_AMPA] - v) : (T)0);
-      P.Irep[(size_t)n + p] = (float)((live & 2u) ? mul_t(g[FS_GABA], q.vrev[FS_GABA] - v) : (T)0);
+      // (a dead receptor's current is 0 with the driving force's sign, which
+      // output files print)
+      P.Irep[p] = (float)mul_t((live & 1u) ? g[FS_AMPA] : (T)0, q.vrev[FS_AMPA] - v);
+      P.Irep[(size_t)n + p] = (float)mul_t((live & 2u) ? g[FS_GABA] : (T)0, q.vrev[FS_GABA] - v);
       P.Irep[(size_t)FS_NMDA * n + p] = (float)Ir2;
-      P.Irep[(size_t)FS_ACH * n + p] = (float)((live & 4u) ? mul_t(g[FS_ACH], q.vrev[FS_ACH] - v) : (T)0);
-      P.Irep[(size_t)FS_GCL * n + p] = (float)((live & 8u) ? mul_t(g[FS_GCL], q.vrev[FS_GCL] - v) : (T)0);
+      P.Irep[(size_t)FS_ACH * n + p] = (float)mul_t((live & 4u) ? g[FS_ACH] : (T)0, q.vrev[FS_ACH] - v);
+      P.Irep[(size_t)FS_GCL * n + p] = (float)mul_t((live & 8u) ? g[FS_GCL] : (T)0, q.vrev[FS_GCL] - v);
     }
     if (st.V > q.vth) {
       ns |= FS_NS_FIRE;
