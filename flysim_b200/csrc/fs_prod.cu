@@ -2045,6 +2045,11 @@ __global__ void __launch_bounds__(kT1, 1) k_prod1(const __grid_constant__ Params
     next_grp = grp0;
     gave_up = 0;
   }
+  // a launch of one step exchanges no lists, whose wait otherwise keeps an
+  // owner's new x_pre and s_pre (stored at the end) behind every block's read
+  // of the old ones (the copies above)
+  unsigned long long target = 0;
+  if (P.nsteps == 1 && !grid_sync(P.bar, P.err, gridDim.x, target)) return;
   __syncthreads();
   pc.mark(5);
   bool ok = true;
