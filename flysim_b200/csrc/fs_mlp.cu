@@ -28,6 +28,7 @@
 #include <random>
 #include <string>
 #include <thread>
+#include <utility>
 #include <vector>
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -1396,6 +1397,7 @@ struct Mlp {
   float *Zo = nullptr, *T = nullptr, *loss = nullptr, *xs = nullptr, *ts = nullptr;
   int *ctr = nullptr, *err = nullptr;
   FwdLayer *fl = nullptr;  // k_forward's layers
+  cudaEvent_t fwd0 = nullptr;  // start of a forward()
   bool pooled = false;     // counted by the lane pool
   // k_train: its blocked buffers and tiles (lazily), grid barrier
   std::vector<TrainLayer> tl;
@@ -1462,6 +1464,7 @@ void destroy(Mlp *m) {
   if (m->order) cudaFreeHost(m->order);
   for (cudaEvent_t x : m->ev)
     if (x) cudaEventDestroy(x);
+  if (m->fwd0) cudaEventDestroy(m->fwd0);
   if (m->st) cudaStreamDestroy(m->st);
   if (m->pooled) lane_pool().leave();
   delete m;
@@ -1486,9 +1489,10 @@ int create(const uint32_t *dims, uint32_t nd, int device, uint64_t seed, Mlp **o
   m->device = device;
   cudaError_t e = cudaSetDevice(device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&m->st, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaEventCreate(&m->fwd0);
   if (e != cudaSuccess) {
     err = std::string("mlp: ") + cudaGetErrorString(e);
-    delete m;
+    destroy(m);
     return FS_ERR_CUDA;
   }
   if (!gemm_attr_set) {
@@ -1719,8 +1723,10 @@ int grad(Mlp *m, const float *x, const float *t, int rows, float *g, float *loss
 }
 
 // Rows [r0, r0 + n) of a call through lane a (n <= kChunk); host copies into
-// and out of the pinned buffers by the calling thread.
-cudaError_t forward_rows(Mlp *m, FwdLane &a, const float *x, float *y, uint64_t r0, int n, double &ms) {
+// and out of the pinned buffers by the calling thread.  ran: when its kernel
+// ran, in ms after Mlp::fwd0.
+cudaError_t forward_rows(Mlp *m, FwdLane &a, const float *x, float *y, uint64_t r0, int n,
+                         std::pair<float, float> &ran) {
   const int di = m->dims[0], no = m->dims[m->L];
   const size_t bx = (size_t)n * di * 4, by = (size_t)n * no * 4, oy = (bx + 255) / 256 * 256;
   std::memcpy(a.host, x + r0 * di, bx);
@@ -1740,10 +1746,20 @@ cudaError_t forward_rows(Mlp *m, FwdLane &a, const float *x, float *y, uint64_t 
   if (e == cudaSuccess) e = cudaStreamSynchronize(a.st);
   if (e != cudaSuccess) return e;
   std::memcpy(y + r0 * no, a.host + oy, by);
-  float t = 0;
-  cudaEventElapsedTime(&t, a.e0, a.e1);
-  ms += t;
-  return cudaSuccess;
+  e = cudaEventElapsedTime(&ran.first, m->fwd0, a.e0);
+  if (e == cudaSuccess) e = cudaEventElapsedTime(&ran.second, m->fwd0, a.e1);
+  return e;
+}
+
+// Milliseconds that at least one of the intervals covers.
+double covered(std::vector<std::pair<float, float>> &v) {
+  std::sort(v.begin(), v.end());
+  double sum = 0.0, end = 0.0;
+  for (const auto &p : v) {
+    sum += std::max(0.0, (double)p.second - std::max((double)p.first, end));
+    end = std::max(end, (double)p.second);
+  }
+  return sum;
 }
 
 // Calls of more than one chunk run on several lanes, each with a host thread
@@ -1757,16 +1773,17 @@ int forward(Mlp *m, const float *x, uint64_t rows, float *y, double *device_ms, 
   cudaError_t e = cudaFuncSetAttribute(k_forward<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem<16>);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_forward<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem<64>);
+  if (e == cudaSuccess) e = cudaEventRecord(m->fwd0, m->st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(m->st);  // weights and parameters are in place
   std::atomic<uint64_t> next{0};
-  std::vector<double> ms(lanes, 0.0);
+  std::vector<std::pair<float, float>> ran(chunks);
   std::vector<cudaError_t> res(lanes, cudaSuccess);
   auto work = [&](size_t w) {
     FwdLane a;
     cudaError_t r = cudaSetDevice(m->device);
     if (r == cudaSuccess) r = lane_pool().take(m->device, cap, a);
     for (uint64_t c; r == cudaSuccess && (c = next.fetch_add(1)) < chunks;)
-      r = forward_rows(m, a, x, y, c * kChunk, (int)std::min<uint64_t>(kChunk, rows - c * kChunk), ms[w]);
+      r = forward_rows(m, a, x, y, c * kChunk, (int)std::min<uint64_t>(kChunk, rows - c * kChunk), ran[c]);
     lane_pool().give(a);
     res[w] = r;
   };
@@ -1779,16 +1796,13 @@ int forward(Mlp *m, const float *x, uint64_t rows, float *y, double *device_ms, 
     work(0);
     for (std::thread &q : th) q.join();
   }
-  double total = 0.0;
-  for (size_t w = 0; w < lanes; w++) {
-    total += ms[w];
+  for (size_t w = 0; w < lanes; w++)
     if (e == cudaSuccess) e = res[w];
-  }
   if (e != cudaSuccess) {
     err = std::string("mlp forward: ") + cudaGetErrorString(e);
     return e == cudaErrorMemoryAllocation ? FS_ERR_NOMEM : FS_ERR_CUDA;
   }
-  if (device_ms) *device_ms = total;
+  if (device_ms) *device_ms = covered(ran);  // (the lanes' kernels overlap and wait for each other)
   return check(m, err);
 }
 

@@ -508,7 +508,8 @@ int fs_mlp_destroy(fs_mlp *m);
 uint64_t fs_mlp_param_count(const fs_mlp *m);
 int fs_mlp_get_params(fs_mlp *m, float *params);
 int fs_mlp_set_params(fs_mlp *m, const float *params);
-/* y[rows x outputs] = network(x[rows x inputs]); host arrays. */
+/* y[rows x outputs] = network(x[rows x inputs]); host arrays.  device_ms (or
+ * NULL): the time in which kernels of the call ran, without the transfers. */
 int fs_mlp_forward(fs_mlp *m, const float *x, uint64_t rows, float *y, double *device_ms);
 /* Gradients of the loss over one batch (rows a multiple of 16, <= 256),
  * targets t[rows x outputs]; no update. */
