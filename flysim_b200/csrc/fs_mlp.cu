@@ -1318,6 +1318,17 @@ void free_lane(FwdLane &a) {
   a = FwdLane();
 }
 
+// Bytes of a lane for chunks of `need` bytes, of a network whose full chunks
+// take `full`: rounded up, so that calls of growing size soon find their lane
+// (a buffer of exactly the call's size made every larger call wait for a new
+// one).  4 MB hold a full chunk of the surrogate.
+size_t lane_bytes(size_t need, size_t full) {
+  const size_t page = 2u << 20;
+  size_t cap = 4u << 20;
+  while (cap < need) cap *= 2;
+  return (std::min(cap, full) + page - 1) / page * page;
+}
+
 // Idle lanes, shared by the networks of the process (a new network's first
 // call would otherwise wait for page-locked memory); at most kLanes are kept,
 // and none once the last network is destroyed.
@@ -1769,7 +1780,7 @@ int forward(Mlp *m, const float *x, uint64_t rows, float *y, double *device_ms, 
   const uint64_t chunks = (rows + kChunk - 1) / kChunk, per = std::min<uint64_t>(rows, kChunk);
   const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
   const size_t lanes = (size_t)std::max<uint64_t>(1, std::min<uint64_t>({(uint64_t)kLanes, chunks, (uint64_t)hw}));
-  const size_t cap = (size_t)per * (m->dims[0] + m->dims[m->L]) * 4 + 256;
+  const size_t row = (size_t)(m->dims[0] + m->dims[m->L]) * 4, cap = lane_bytes(per * row + 256, kChunk * row + 256);
   cudaError_t e = cudaFuncSetAttribute(k_forward<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem<16>);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_forward<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem<64>);

@@ -1,0 +1,21 @@
+"""The page-locked and device buffers that inference keeps between calls."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def test_calls_of_growing_size_share_a_lane(built):
+    # 14.3 to 16.8 MB a call: at most two sizes of lane (16 and 18 MB), not one
+    # for each of the twelve calls (six kept: 90 MB)
+    import torch
+    net = built.Mlp([256, 256], seed=1)
+    try:
+        x = np.zeros((8192, 256), np.float32)
+        net.forward(x[:16])
+        free = torch.cuda.mem_get_info()[0]
+        for rows in np.linspace(7000, 8192, 12).astype(int):
+            net.forward(x[:rows])
+        assert free - torch.cuda.mem_get_info()[0] <= 48 << 20
+    finally:
+        net.close()
