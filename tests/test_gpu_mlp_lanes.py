@@ -19,3 +19,21 @@ def test_calls_of_growing_size_share_a_lane(built):
         assert free - torch.cuda.mem_get_info()[0] <= 48 << 20
     finally:
         net.close()
+
+
+def test_a_first_call_of_a_few_chunks_makes_one_lane(built):
+    # five chunks: one lane of 18 MB, not five (a lane takes as long to make as
+    # three chunks to run); later calls make more
+    import torch
+    net = built.Mlp([256, 256], seed=1)
+    try:
+        x = np.zeros((8192 * 5, 256), np.float32)
+        net.grad(x[:16], x[:16])
+        free = torch.cuda.mem_get_info()[0]
+        net.forward(x)
+        assert free - torch.cuda.mem_get_info()[0] <= 40 << 20
+        for _ in range(12):
+            net.forward(x)
+        assert free - torch.cuda.mem_get_info()[0] >= 60 << 20
+    finally:
+        net.close()
