@@ -1840,6 +1840,7 @@ int forward(Mlp *m, const float *x, uint64_t rows, float *y, double *device_ms, 
     e = make_lane(m->device, cap, a);
     if (e == cudaSuccess) lane.push_back(a);
   }
+  if (!lane.empty()) e = cudaSuccess;  // a lane that cannot be made is done without
   const size_t lanes = lane.size();
   std::atomic<uint64_t> next{0};
   std::vector<cudaError_t> res(lanes, cudaSuccess);
@@ -1849,7 +1850,7 @@ int forward(Mlp *m, const float *x, uint64_t rows, float *y, double *device_ms, 
       r = forward_rows(m, lane[w], x, y, c * kChunk, (int)std::min<uint64_t>(kChunk, rows - c * kChunk), ran[c]);
     res[w] = r;
   };
-  if (e == cudaSuccess) {
+  if (lanes) {
     std::vector<std::thread> th;
     try {
       for (size_t w = 1; w < lanes; w++) th.emplace_back(work, w);

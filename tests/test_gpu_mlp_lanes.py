@@ -37,3 +37,22 @@ def test_a_first_call_of_a_few_chunks_makes_one_lane(built):
         assert free - torch.cuda.mem_get_info()[0] >= 60 << 20
     finally:
         net.close()
+
+
+def test_a_lane_that_cannot_be_made_is_done_without(built):
+    # room for three or four more lanes of 4 MB where the call wants five
+    import torch
+    net = built.Mlp([64, 2], seed=1)
+    fill = None
+    try:
+        x = np.random.default_rng(0).uniform(-1, 1, (8192 * 100, 64)).astype(np.float32)
+        want = net.forward(x[:8192])
+        free = torch.cuda.mem_get_info()[0]
+        fill = torch.empty((free - (14 << 20)) // 2097152 * 2097152, dtype=torch.uint8, device="cuda")
+        y = net.forward(x)
+        np.testing.assert_array_equal(y[:8192], want)
+        np.testing.assert_array_equal(net.forward(x[-8192:]), y[-8192:])
+    finally:
+        del fill
+        torch.cuda.empty_cache()
+        net.close()
