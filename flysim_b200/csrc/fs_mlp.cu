@@ -1460,7 +1460,7 @@ struct Mlp {
   float *xall = nullptr, *tall = nullptr, *eloss = nullptr;
   int *perm = nullptr;
   int *order = nullptr;  // pinned: the orders of two epochs
-  cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};  // order copied (2), device time
+  cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};  // start and end of the last even and odd epoch
   uint64_t cap_rows = 0;
   uint32_t cap_epochs = 0;
   std::vector<void *> allocs;
@@ -2016,29 +2016,38 @@ int train(Mlp *m, const float *x, const float *t, uint64_t rows, uint32_t epochs
     return e == cudaSuccess;
   };
   if (epochs) ok(cudaMemsetAsync(m->eloss, 0, (size_t)epochs * 4, m->st));
-  ok(cudaEventRecord(m->ev[2], m->st));
+  double ms = 0.0;
+  auto epoch_time = [&](uint32_t ep) {  // of an epoch that has ended
+    float t = 0;
+    if (ok(cudaEventElapsedTime(&t, m->ev[ep & 1u], m->ev[2 + (ep & 1u)]))) ms += t;
+  };
   for (uint32_t ep = 0; ep < epochs && e == cudaSuccess; ep++) {
     // the host draws an epoch's order while the device runs the last one
     int *order = m->order + (ep & 1u) * m->cap_rows;
-    if (ep >= 2 && !ok(cudaEventSynchronize(m->ev[ep & 1u]))) break;
+    if (ep >= 2) {
+      if (!ok(cudaEventSynchronize(m->ev[2 + (ep & 1u)]))) break;
+      epoch_time(ep - 2);
+    }
     std::iota(order, order + rows, 0);
     std::shuffle(order, order + rows, gen);
     ok(cudaMemcpyAsync(m->perm, order, (size_t)steps * kBatch * 4, cudaMemcpyHostToDevice, m->st));
-    ok(cudaEventRecord(m->ev[ep & 1u], m->st));
     if (exec) {
       ok(cudaMemsetAsync(m->ctr, 0, 4, m->st));  // batch index (the Adam count in ctr[1] runs on)
       ok(cudaMemsetAsync(m->loss, 0, 4, m->st));
+      ok(cudaEventRecord(m->ev[ep & 1u], m->st));
       for (int s = 0; s < steps && e == cudaSuccess; s++) ok(cudaGraphLaunch(exec, m->st));
+      ok(cudaEventRecord(m->ev[2 + (ep & 1u)], m->st));
       ok(cudaMemcpyAsync(m->eloss + ep, m->loss, 4, cudaMemcpyDeviceToDevice, m->st));
     } else {
       a.loss = m->eloss + ep;
       void *args[] = {&a};
       ok(cudaMemsetAsync(m->bar, 0, 8, m->st));
+      ok(cudaEventRecord(m->ev[ep & 1u], m->st));
       if (e == cudaSuccess)
         ok(cudaLaunchCooperativeKernel((const void *)k_train, kRowCtas + m->tiles, kTrThreads, args, kTrainSmem, m->st));
+      ok(cudaEventRecord(m->ev[2 + (ep & 1u)], m->st));
     }
   }
-  ok(cudaEventRecord(m->ev[3], m->st));
   for (int l = 0; l < m->L; l++) {  // the BF16 copies that inference and grad() read
     const int n = m->pd[l] * m->pd[l + 1];
     k_refresh<<<(n + 255) / 256, 256, 0, m->st>>>(m->W[l], m->pd[l + 1], m->pd[l], m->Wb[l], m->Wt[l], m->Wk[l]);
@@ -2051,8 +2060,8 @@ int train(Mlp *m, const float *x, const float *t, uint64_t rows, uint32_t epochs
     err = std::string("mlp train: ") + cudaGetErrorString(e);
     rc = FS_ERR_CUDA;
   }
-  float ms = 0;
-  if (!rc) cudaEventElapsedTime(&ms, m->ev[2], m->ev[3]);
+  if (!rc)
+    for (uint32_t ep = epochs > 2 ? epochs - 2 : 0; ep < epochs; ep++) epoch_time(ep);
   if (epoch_loss)
     for (uint32_t ep = 0; ep < epochs && !rc; ep++) epoch_loss[ep] = el[ep] / (float)steps;
   if (device_ms) *device_ms = ms;

@@ -515,7 +515,9 @@ int fs_mlp_forward(fs_mlp *m, const float *x, uint64_t rows, float *y, double *d
  * targets t[rows x outputs]; no update. */
 int fs_mlp_grad(fs_mlp *m, const float *x, const float *t, uint32_t rows, float *grads, float *loss);
 /* Adam, batches of 256 rows in a fresh shuffle per epoch (rows beyond a
- * multiple of 256 are left out of that epoch); epoch_loss[epochs] or NULL. */
+ * multiple of 256 are left out of that epoch); epoch_loss[epochs] or NULL;
+ * device_ms (or NULL): the time of the epochs' kernels, without the waits for
+ * an epoch's order. */
 int fs_mlp_train(fs_mlp *m, const float *x, const float *t, uint64_t rows, uint32_t epochs, float lr,
                  uint64_t seed, float *epoch_loss, double *device_ms);
 /* One tensor-core GEMM for checks: c[m x n] = a[m x k] . b[n x k]^T (+ bias,

@@ -22,9 +22,27 @@ def test_forward_of_overlapping_lanes(built):
             t = time.perf_counter()
             _, ms = net.forward(x, with_time=True)
             wall = 1e3 * (time.perf_counter() - t)
-            assert 0.3 * wall < ms <= wall, (ms, wall)
+            assert ms <= wall, (ms, wall)
         _, one = net.forward(x[:8192], with_time=True)
         # 18 chunks of the same work, at most two at a time on the SMs
         assert 0.5 * 18 * one <= ms <= 1.5 * 18 * one, (ms, one)
+    finally:
+        net.close()
+
+
+def test_training_without_the_hosts_part(built):
+    # a small network on many rows: drawing an epoch's order of 2,000,000 rows
+    # takes the host tens of ms; the first epoch's, which nothing hides, is not
+    # in device_ms, so one epoch takes what each of four more adds
+    rows = 2_000_000
+    rng = np.random.default_rng(1)
+    x = rng.uniform(-1, 1, (rows, 1)).astype(np.float32)
+    t = np.stack([x[:, 0], x[:, 0] > 0], 1).astype(np.float32)
+    net = built.Mlp([1, 2], seed=2)
+    try:
+        net.train(x, t, epochs=1)
+        one = net.train(x, t, epochs=1)[1]
+        each = (net.train(x, t, epochs=5)[1] - one) / 4
+        assert abs(one - each) <= 0.03 * each + 1.0, (one, each)
     finally:
         net.close()
