@@ -1458,8 +1458,9 @@ struct Mlp {
   // the training set on the device, kept (grown) across calls: fit() trains in
   // rounds on the same rows
   float *xall = nullptr, *tall = nullptr, *eloss = nullptr;
-  int *perm = nullptr;
-  int *order = nullptr;  // pinned: the orders of two epochs
+  int *perm = nullptr;           // the orders of two epochs
+  cudaStream_t order_st = nullptr;  // copies an epoch's order while the last one runs
+  cudaEvent_t order_ev = nullptr;   // it is there
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};  // start and end of the last even and odd epoch
   uint64_t cap_rows = 0;
   uint32_t cap_epochs = 0;
@@ -1511,8 +1512,10 @@ void destroy(Mlp *m) {
   if (!m) return;
   cudaSetDevice(m->device);
   if (m->st) cudaStreamSynchronize(m->st);
+  if (m->order_st) cudaStreamSynchronize(m->order_st);
   for (void *p : m->allocs) cudaFree(p);
-  if (m->order) cudaFreeHost(m->order);
+  if (m->order_st) cudaStreamDestroy(m->order_st);
+  if (m->order_ev) cudaEventDestroy(m->order_ev);
   for (cudaEvent_t x : m->ev)
     if (x) cudaEventDestroy(x);
   if (m->fwd0) cudaEventDestroy(m->fwd0);
@@ -1886,21 +1889,37 @@ int ensure_train(Mlp *m, std::string &err) {
     m->tiles = -1;
     return FS_OK;
   }
+  // the blocked buffers are parts of one allocation (a dozen of their own took
+  // longer than a small first call)
   std::vector<TrainLayer> tl(m->L);
-  int rc = FS_OK;
-  for (int l = 0; l < m->L && !rc; l++) {
-    TrainLayer &y = tl[l];
-    y.in = m->pd[l];
-    y.out = m->pd[l + 1];
+  bf16 *buf = nullptr;
+  size_t total = 0;
+  for (int pass = 0; pass < 2; pass++) {
+    size_t at = 0;
     const auto up = [](int v, int k) { return (size_t)((v + k - 1) / k); };
-    y.Wk = m->Wk[l];
-    if ((rc = mal(m, &y.Wt, up(y.in, 128) * up(y.out, 64) * (kChunkB / 2), err)) ||
-        (rc = mal(m, &y.HT, up(y.in, kTileN) * kTileN * kBatch, err)) ||
-        (rc = mal(m, &y.dZT, up(y.out, 128) * 128 * kBatch, err)))
-      break;
-    y.W = m->W[l]; y.mW = m->mW[l]; y.vW = m->vW[l];
-    y.b = m->b[l]; y.mb = m->mb[l]; y.vb = m->vb[l];
+    const auto part = [&](size_t n) {
+      bf16 *p = buf ? buf + at : nullptr;
+      at += (n + 127) / 128 * 128;
+      return p;
+    };
+    for (int l = 0; l < m->L; l++) {
+      TrainLayer &y = tl[l];
+      y.in = m->pd[l];
+      y.out = m->pd[l + 1];
+      y.Wk = m->Wk[l];
+      y.Wt = part(up(y.in, 128) * up(y.out, 64) * (kChunkB / 2));
+      y.HT = part(up(y.in, kTileN) * kTileN * kBatch);
+      y.dZT = part(up(y.out, 128) * 128 * kBatch);
+      y.W = m->W[l]; y.mW = m->mW[l]; y.vW = m->vW[l];
+      y.b = m->b[l]; y.mb = m->mb[l]; y.vb = m->vb[l];
+    }
+    total = at;
+    if (pass == 0) {
+      int rc = mal(m, &buf, total, err);
+      if (rc) return rc;
+    }
   }
+  int rc = FS_OK;
   if (!rc) rc = mal(m, &m->tile, tile.size(), err);
   if (!rc) rc = mal(m, &m->bar, 64, err);
   if (rc) return rc;
@@ -1941,7 +1960,7 @@ int capture_step(Mlp *m, const float *xall, const float *tall, const int *perm, 
   return rc;
 }
 
-// Device and pinned buffers for `rows` training rows and `epochs` epochs.
+// Device buffers for `rows` training rows and `epochs` epochs.
 int ensure_rows(Mlp *m, uint64_t rows, uint32_t epochs, std::string &err) {
   int rc = FS_OK;
   if (rows > m->cap_rows) {
@@ -1951,15 +1970,13 @@ int ensure_rows(Mlp *m, uint64_t rows, uint32_t epochs, std::string &err) {
     release(m, m->perm);
     m->xall = m->tall = nullptr;
     m->perm = nullptr;
-    if (m->order) cudaFreeHost(m->order);
-    m->order = nullptr;
     if ((rc = mal(m, &m->xall, rows * m->dims[0], err)) || (rc = mal(m, &m->tall, rows * m->dims[m->L], err)) ||
-        (rc = mal(m, &m->perm, rows, err)))
+        (rc = mal(m, &m->perm, 2 * rows, err)))
       return rc;
-    if (cudaMallocHost((void **)&m->order, 2 * rows * sizeof(int)) != cudaSuccess) {
-      m->order = nullptr;
-      err = "mlp train: pinned host memory";
-      return FS_ERR_NOMEM;
+    // (their zero fill, before another stream writes perm)
+    if (cudaStreamSynchronize(m->st) != cudaSuccess) {
+      err = "mlp train: buffers";
+      return FS_ERR_CUDA;
     }
     m->cap_rows = rows;
   }
@@ -1970,12 +1987,17 @@ int ensure_rows(Mlp *m, uint64_t rows, uint32_t epochs, std::string &err) {
     if ((rc = mal(m, &m->eloss, epochs, err))) return rc;
     m->cap_epochs = epochs;
   }
-  for (cudaEvent_t &e : m->ev)
-    if (!e && cudaEventCreate(&e) != cudaSuccess) {
-      e = nullptr;
-      err = "mlp train: event create";
-      return FS_ERR_CUDA;
-    }
+  cudaError_t e = cudaSuccess;
+  for (cudaEvent_t &x : m->ev)
+    if (!x && e == cudaSuccess) e = cudaEventCreate(&x);
+  if (epochs > 1) {
+    if (!m->order_st && e == cudaSuccess) e = cudaStreamCreateWithFlags(&m->order_st, cudaStreamNonBlocking);
+    if (!m->order_ev && e == cudaSuccess) e = cudaEventCreateWithFlags(&m->order_ev, cudaEventDisableTiming);
+  }
+  if (e != cudaSuccess) {
+    err = std::string("mlp train: ") + cudaGetErrorString(e);
+    return FS_ERR_CUDA;
+  }
   return FS_OK;
 }
 
@@ -2003,7 +2025,6 @@ int train(Mlp *m, const float *x, const float *t, uint64_t rows, uint32_t epochs
   a.tiles = m->tiles;
   a.x = m->xall;
   a.t = m->tall;
-  a.perm = m->perm;
   a.tile = m->tile;
   a.lr = lr;
   a.ctr = m->ctr;
@@ -2021,16 +2042,26 @@ int train(Mlp *m, const float *x, const float *t, uint64_t rows, uint32_t epochs
     float t = 0;
     if (ok(cudaEventElapsedTime(&t, m->ev[ep & 1u], m->ev[2 + (ep & 1u)]))) ms += t;
   };
+  std::vector<int> order(rows);
   for (uint32_t ep = 0; ep < epochs && e == cudaSuccess; ep++) {
-    // the host draws an epoch's order while the device runs the last one
-    int *order = m->order + (ep & 1u) * m->cap_rows;
+    // the host draws an epoch's order, and copies it on a stream of its own,
+    // while the device runs the last one (pageable memory, staged by the copy:
+    // page-locking its room cost a network's first call 2 ms); the captured step
+    // has one place for it, behind the last epoch
     if (ep >= 2) {
       if (!ok(cudaEventSynchronize(m->ev[2 + (ep & 1u)]))) break;
       epoch_time(ep - 2);
     }
-    std::iota(order, order + rows, 0);
-    std::shuffle(order, order + rows, gen);
-    ok(cudaMemcpyAsync(m->perm, order, (size_t)steps * kBatch * 4, cudaMemcpyHostToDevice, m->st));
+    std::iota(order.begin(), order.end(), 0);
+    std::shuffle(order.begin(), order.end(), gen);
+    const bool apart = !exec && epochs > 1;
+    a.perm = m->perm + (apart ? (ep & 1u) * m->cap_rows : 0);
+    const cudaStream_t cs = apart ? m->order_st : m->st;
+    ok(cudaMemcpyAsync((void *)a.perm, order.data(), (size_t)steps * kBatch * 4, cudaMemcpyHostToDevice, cs));
+    if (apart) {
+      ok(cudaEventRecord(m->order_ev, cs));
+      ok(cudaStreamWaitEvent(m->st, m->order_ev, 0));
+    }
     if (exec) {
       ok(cudaMemsetAsync(m->ctr, 0, 4, m->st));  // batch index (the Adam count in ctr[1] runs on)
       ok(cudaMemsetAsync(m->loss, 0, 4, m->st));
