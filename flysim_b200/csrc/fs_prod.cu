@@ -252,6 +252,27 @@ __device__ __forceinline__ float comp4(const float4 &q, int k) {
   return k == 0 ? q.x : k == 1 ? q.y : k == 2 ? q.z : q.w;
 }
 
+// The pull's loads, in the order written: the windows (L1 may serve them, see
+// above) before the next edges.  Left to the compiler the order changed with the
+// code around the pull, and the pull with it (20,000 neurons: 3,150 to 3,480
+// cycles a step).
+__device__ __forceinline__ float4 ld_window(const float4 *p, bool ok) {
+  float4 v;
+  asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %5, 0;\n mov.f32 %0, 0f00000000;\n mov.f32 %1, 0f00000000;\n"
+               " mov.f32 %2, 0f00000000;\n mov.f32 %3, 0f00000000;\n @q ld.global.ca.v4.f32 {%0, %1, %2, %3}, [%4];\n}"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "l"(p), "r"((uint32_t)ok)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ uint32_t ld_edge(const uint32_t *p, bool ok) {
+  uint32_t v;
+  asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %2, 0;\n mov.u32 %0, 0;\n @q ld.global.nc.u32 %0, [%1];\n}"
+               : "=r"(v)
+               : "l"(p), "r"((uint32_t)ok));
+  return v;
+}
+
 // Lanes work in groups that each take one edge, lane k of a group loading
 // vector k of the edge's window (steps 4k..4k+3), so one warp load covers a
 // group's worth of edges whose vectors share a cache line per edge (about
@@ -266,7 +287,11 @@ __device__ __forceinline__ float comp4(const float4 &q, int k) {
 // combined in a fixed tree (g + 5 onto g, then g + 3, g + 2 and g + 1) and
 // quads by an xor butterfly over the eight groups.  The group size depends
 // on the network's interval alone, so the sums depend on neither U, the
-// block plan, the kernel nor the length of a batch.
+// block plan, the kernel nor the length of a batch.  The row bounds are read two
+// posts ahead: a post's first edges wait for them, and many posts have edges
+// for one round only.  Cycles a step, 20,000 / 60,000 neurons: 3,360 / 7,050
+// -> 2,880 / 5,970 (3,150 / 6,450 as the code before the batches' three passes
+// happened to be compiled).
 template <int U, uint32_t KT>
 __device__ __forceinline__ void nmda_pull_f32(const Params &P, uint32_t p0, uint32_t np, uint64_t tb, uint32_t L,
                                               float (*gn)[KT], uint32_t wid, uint32_t lane) {
@@ -285,23 +310,22 @@ __device__ __forceinline__ void nmda_pull_f32(const Params &P, uint32_t p0, uint
 #pragma unroll
     for (int u = 0; u < U; u++) {
       const uint32_t eu = base + g + G * u;
-      code[u] = gv && eu < end ? __ldg(P.in_code + eu) : 0u;
-      w[u] = gv && eu < end ? __ldg(P.in_w + eu) : 0.0f;
+      code[u] = ld_edge(P.in_code + eu, gv && eu < end);
+      w[u] = __uint_as_float(ld_edge((const uint32_t *)P.in_w + eu, gv && eu < end));
     }
   };
-  uint32_t q = wid, b0 = 0, b1 = 0;
-  if (P.in_row && q < np) {
-    b0 = __ldg(P.in_row + p0 + q);
-    b1 = __ldg(P.in_row + p0 + q + 1);
-    fetch(b0, b1);
-  }
+  auto bounds = [&](uint32_t i, uint32_t &lo, uint32_t &hi) {
+    const bool ok = P.in_row && i < np;
+    lo = ok ? __ldg(P.in_row + p0 + i) : 0u;
+    hi = ok ? __ldg(P.in_row + p0 + i + 1) : 0u;
+  };
+  uint32_t q = wid, b0, b1, n0, n1;
+  bounds(q, b0, b1);
+  bounds(q + nw, n0, n1);
+  fetch(b0, b1);
   for (; q < np; q += nw) {
-    const uint32_t qn = q + nw;
-    uint32_t n0 = 0, n1 = 0;
-    if (P.in_row && qn < np) {
-      n0 = __ldg(P.in_row + p0 + qn);
-      n1 = __ldg(P.in_row + p0 + qn + 1);
-    }
+    uint32_t m0, m1;
+    bounds(q + 2 * nw, m0, m1);
     float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     const uint32_t nch = (b1 - b0 + CH - 1) / CH;
     for (uint32_t c = 0; c < nch; c++) {
@@ -313,13 +337,13 @@ __device__ __forceinline__ void nmda_pull_f32(const Params &P, uint32_t p0, uint
         const uint32_t pre = code[u] & 0xffffffu, d = code[u] >> 24;
         const uint32_t a = (uint32_t)(tb - 1u - d) & mask;
         const float4 *row = sh + ((size_t)pre * kSH + (a & 3u)) * S4;
-        v[u] = ok ? __ldca(row + (((a >> 2) + k) & qmask)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[u] = ld_window(row + (((a >> 2) + k) & qmask), ok);
       }
       float wc[U];
 #pragma unroll
       for (int u = 0; u < U; u++) wc[u] = w[u];
-      if (c + 1 < nch) fetch(b0 + (c + 1) * CH, b1);
-      else if (qn < np) fetch(n0, n1);
+      const bool more = c + 1 < nch;
+      fetch(more ? b0 + (c + 1) * CH : n0, more ? b1 : n1);
 #pragma unroll
       for (int u = 0; u < U; u++) {
         acc[0] += wc[u] * v[u].x;
@@ -328,7 +352,7 @@ __device__ __forceinline__ void nmda_pull_f32(const Params &P, uint32_t p0, uint
         acc[3] += wc[u] * v[u].w;
       }
     }
-    if (nch == 0 && qn < np) fetch(n0, n1);
+    if (nch == 0) fetch(n0, n1);
     if (tri) {
       // g + 5 onto g (g < 5), g + 3 onto g (g < 2), then g + 2 and g + 1
       // onto g = 0: lane k ends with its four steps' sums
@@ -358,6 +382,8 @@ __device__ __forceinline__ void nmda_pull_f32(const Params &P, uint32_t p0, uint
     }
     b0 = n0;
     b1 = n1;
+    n0 = m0;
+    n1 = m1;
   }
 }
 
