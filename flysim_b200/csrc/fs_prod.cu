@@ -1195,6 +1195,26 @@ __device__ __forceinline__ void pre_batch(const Params &P, const NeuronPar<T> &N
   }
 }
 
+// A thread's neuron.  Batches of one step (kOne: networks of interval 1) load it
+// with their first conductance item before the drive draws: one wait for
+// memory instead of three a step (45,000 neurons without delays, us a step: 25.4
+// -> 22.8; 100,000: 38.7 -> 34.0).
+template <class T>
+struct TileNeuron {
+  NeuronPar<T> N;
+  NeuronState<T> st;
+};
+template <class T>
+__device__ __forceinline__ void load_one(const Params &P, uint32_t p0, uint32_t np, uint32_t sb, uint32_t items,
+                                         TileNeuron<T> &I, CondItem<T> &C) {
+  const uint32_t q = threadIdx.x, p = p0 + q;
+  if (q < np) {
+    load_membrane<T>(P, p, I.N, I.st);
+    load_pre<T>(P, p, I.N, I.st);
+  }
+  if (q < items) cond_load<T>(P, p0, np, sb, 1, q, C);
+}
+
 // Membrane and presynaptic state of the batch, a thread per neuron: the
 // membrane's L steps first (the spikes as a bit mask), then the presynaptic
 // part with the spike outputs and the list of spikes that the block pushes at
@@ -1202,19 +1222,20 @@ __device__ __forceinline__ void pre_batch(const Params &P, const NeuronPar<T> &N
 // until the interval's end; past the list's room a thread pushes its spike
 // itself).  kKeepS: the s values of the batch are left in gn for
 // store_history, with whom to store them for in nm.
-template <class T, bool kLTP, bool kKeepS, uint32_t KT>
+template <class T, bool kLTP, bool kKeepS, bool kOne, uint32_t KT>
 __device__ __forceinline__ void tile_neurons(const Params &P, uint32_t p0, uint32_t np, uint32_t sb, uint32_t L,
                                              T (*gn)[KT], const T (*gl)[kLB][KT],
-                                             const T (*gauss)[KT], const SpikeList<T> &lst, const T *gapI, uint8_t *nm) {
+                                             const T (*gauss)[KT], const SpikeList<T> &lst, const T *gapI, uint8_t *nm,
+                                             TileNeuron<T> &I) {
   const uint32_t n = P.n, q = threadIdx.x;
   if (q >= np) return;
   const uint32_t p = p0 + q;
-  NeuronPar<T> N;
-  NeuronState<T> st;
-  load_membrane<T>(P, p, N, st);
-  if (kLTP) load_pre<T>(P, p, N, st);  // one step: its latency would not hide
+  NeuronPar<T> &N = I.N;
+  NeuronState<T> &st = I.st;
   LtpTrace<T> lt;
-  if constexpr (kLTP) {
+  if (!kOne) load_membrane<T>(P, p, N, st);
+  if constexpr (kLTP) {  // (loaded as early as kOne's: 16.4 -> 16.7 us a step at 20,000 neurons)
+    load_pre<T>(P, p, N, st);  // one step: its latency would not hide
     lt.lp = ((float *)P.ltp_lp)[p];
     lt.clp = P.ltp_clp[p];
     lt.dflp = __ldg(P.ltp_dflp + p);
@@ -1235,7 +1256,7 @@ __device__ __forceinline__ void tile_neurons(const Params &P, uint32_t p0, uint3
   }
   store_membrane<T>(P, p, st);
   if (P.gap_row) ((T *)P.Vg)[(size_t)((P.t0 + sb) & 1u) * n + p] = st.V;
-  if (!kLTP) load_pre<T>(P, p, N, st);  // (held through the membranes' steps, its registers cost more)
+  if (!kOne && !kLTP) load_pre<T>(P, p, N, st);  // (held through the membranes' steps, its registers cost more)
   if (kKeepS) nm[q] = (N.pj >> FS_NMDA) & 1u;
   float tm[3] = {0.0f, 0.0f, 0.0f};
   if (N.pj & kPjTM) {
@@ -1376,25 +1397,27 @@ __device__ __forceinline__ void tile_gap(const Params &P, uint32_t tp0, uint32_t
 // state 280, history and pushes 290; with the barrier 4.06 -> 3.88 us a step.
 // The 200k network's tile kernels (more posts than threads to start with)
 // gain from the shorter inner loops: 34.2 -> 30.8 us a step.
-template <class T, uint32_t KT, uint32_t NT = kThreads>
+template <class T, uint32_t KT, bool kOne = false, uint32_t NT = kThreads>
 __device__ __forceinline__ void tile_steps(const Params &P, uint32_t tp0, uint32_t np, uint32_t bs, uint32_t L,
                                            TileBufs<T, KT> &B, PhaseClock &pc, bool hist) {
   constexpr uint32_t kCap = TileBufs<T, KT>::kCap;
   const SpikeList<T> lst{&B.l_n, B.l_p, B.l_tm, B.l_c, kCap};
   const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const uint32_t items = cond_items<T>(P, np);
+  TileNeuron<T> I;
+  CondItem<T> C;
+  if (kOne) load_one<T>(P, tp0, np, bs, items, I, C);
   draw_inputs<T, KT, NT>(P, tp0, np, P.t0 + bs, L, B.hits, B.gauss(P));
   if (P.gap_row) tile_gap<T, NT>(P, tp0, np, bs, B.gapI);
   __syncthreads();
   pc.mark(1);
   for (uint32_t i = tid; i < items; i += NT) {
-    CondItem<T> I;
-    cond_load<T>(P, tp0, np, bs, L, i, I);
-    cond_steps<T, KT>(P, tp0, bs, L, I, B.gn, B.hits, B.lin());
+    if (!kOne || i != tid) cond_load<T>(P, tp0, np, bs, L, i, C);
+    cond_steps<T, KT>(P, tp0, bs, L, C, B.gn, B.hits, B.lin());
   }
   __syncthreads();
   pc.mark(9);
-  tile_neurons<T, false, true, KT>(P, tp0, np, bs, L, B.gn, B.lin(), B.gauss(P), lst, B.gapI, B.nm);
+  tile_neurons<T, false, true, kOne, KT>(P, tp0, np, bs, L, B.gn, B.lin(), B.gauss(P), lst, B.gapI, B.nm, I);
   __syncthreads();
   pc.mark(2);
   if (hist) store_history<T, KT, NT>(P, tp0, np, P.t0 + bs, L, B.gn, B.nm);
@@ -1425,7 +1448,7 @@ __device__ __forceinline__ void tile_steps(const Params &P, uint32_t tp0, uint32
 // The steps of one block: posts [B0, B1) of the network P, whose blocks
 // (nblk of them) meet at a barrier after every interval.  PU: NMDA edges in
 // flight per lane in the pull (results do not depend on it).
-template <class T, int PU, uint32_t KT, uint32_t NT>
+template <class T, int PU, uint32_t KT, bool kOne, uint32_t NT>
 __device__ __forceinline__ void prod_blocks(const Params &P, uint32_t B0, uint32_t B1, uint32_t nblk) {
   constexpr uint32_t kT = KT;
   extern __shared__ __align__(16) unsigned char smt[];
@@ -1439,12 +1462,12 @@ __device__ __forceinline__ void prod_blocks(const Params &P, uint32_t B0, uint32
   while (s < P.nsteps) {
     const uint32_t iv_end = min(P.nsteps, s + P.interval);
     for (uint32_t bs = s; bs < iv_end; bs += kLB) {
-      const uint32_t L = min(kLB, iv_end - bs);
+      const uint32_t L = kOne ? 1u : min(kLB, iv_end - bs);
       for (uint32_t tp0 = B0; tp0 < B1; tp0 += kT) {
         const uint32_t np = min(kT, B1 - tp0);
         tile_pull<T, PU, KT, NT>(P, tp0, np, bs, L, B);
         pc.mark(0);
-        tile_steps<T, KT, NT>(P, tp0, np, bs, L, B, pc, P.in_row != nullptr);
+        tile_steps<T, KT, kOne, NT>(P, tp0, np, bs, L, B, pc, P.in_row != nullptr);
       }
     }
     s = iv_end;
@@ -1464,10 +1487,11 @@ __device__ __forceinline__ void prod_blocks(const Params &P, uint32_t B0, uint32
 // they span several (250k network: 43.3 against 46.3 us); ring slots two
 // steps ahead (4.60 us with one).  Batches of small networks run eight edges
 // and one step ahead (their kernel has fewer registers to spare).
-template <class T, int PU, uint32_t KT>
+template <class T, int PU, uint32_t KT, bool kOne = false>
 __global__ void __launch_bounds__(sizeof(T) == 4 ? kThreads : kThreads64, sizeof(T) == 4 ? 2 : 1)
     k_prod(const __grid_constant__ Params P) {
-  prod_blocks<T, PU, KT, sizeof(T) == 4 ? kThreads : kThreads64>(P, P.block_post[blockIdx.x], P.block_post[blockIdx.x + 1], gridDim.x);
+  prod_blocks<T, PU, KT, kOne, sizeof(T) == 4 ? kThreads : kThreads64>(P, P.block_post[blockIdx.x],
+                                                                     P.block_post[blockIdx.x + 1], gridDim.x);
 }
 
 // ---- long-term plasticity (networks with LTP, delays 0) ---------------------
@@ -1654,7 +1678,8 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1) k_prod_ltp(c
         cond_steps<T, KT>(P, tp0, s, 1, I, gn, B.hits, B.lin());
       }
       __syncthreads();
-      tile_neurons<T, true, false, KT>(P, tp0, np, s, 1, gn, B.lin(), B.gauss(P), lst, B.gapI, B.nm);
+      TileNeuron<T> I;
+      tile_neurons<T, true, false, false, KT>(P, tp0, np, s, 1, gn, B.lin(), B.gauss(P), lst, B.gapI, B.nm, I);
       __syncthreads();
       pc.mark(2);
     }
@@ -2475,6 +2500,10 @@ constexpr uint32_t kLiveAll = 0x11f0fu;
 // flight where blocks span several tiles.
 const void *prod_kernel(const Prod *p) {
   if (p->fp64) return p->max_posts <= 64 ? (const void *)k_prod<double, 4, 64> : (const void *)k_prod<double, 4, 128>;
+  if (p->P.interval == 1) {
+    if (p->wide) return (const void *)k_prod<float, 8, 256, true>;
+    return p->max_posts <= 128 ? (const void *)k_prod<float, 4, 128, true> : (const void *)k_prod<float, 4, 256, true>;
+  }
   if (p->wide) return (const void *)k_prod<float, 8, 256>;
   return p->max_posts <= 128 ? (const void *)k_prod<float, 4, 128> : (const void *)k_prod<float, 4, 256>;
 }
@@ -2494,7 +2523,9 @@ size_t prod_smem(const Prod *p, uint32_t live) {
 void tile_attributes() {
   const int f = (int)tile_smem<float, 256>(kLiveAll), d = (int)tile_smem<double, 128>(kLiveAll);
   for (const void *k : {(const void *)k_prod<float, 4, 128>, (const void *)k_prod<float, 4, 256>,
-                        (const void *)k_prod<float, 8, 256>, (const void *)k_prod_ltp<float, 128>,
+                        (const void *)k_prod<float, 8, 256>, (const void *)k_prod<float, 4, 128, true>,
+                        (const void *)k_prod<float, 4, 256, true>, (const void *)k_prod<float, 8, 256, true>,
+                        (const void *)k_prod_ltp<float, 128>,
                         (const void *)k_prod_ltp<float, 256>, (const void *)k_tile_step<float>})
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, f);
   for (const void *k : {(const void *)k_prod<double, 4, 64>, (const void *)k_prod<double, 4, 128>,
