@@ -42,6 +42,7 @@ struct fs_handle {
   uint32_t gpar = 0;             // parity of the group gates' next buffer (kept across resets, like the gates)
   uint32_t *drawoff = nullptr, *injoff = nullptr;
   uint32_t jcong = 0;
+  bool tables = false;  // counted among the users of the device's ExpTables
   // batch buffers
   uint32_t *spikebits = nullptr, *counts = nullptr, *offsets = nullptr, *idx = nullptr;
   uint64_t batch_cap = 0;  // steps the batch buffers hold
@@ -111,6 +112,73 @@ std::string lib_dir() {
     if (s != std::string::npos) return p.substr(0, s);
   }
   return ".";
+}
+
+// The expf and logf exception tables of a device, hashed: 8 MB that every
+// reference-order handle on it reads, made by the first and freed with the last
+// (a copy a handle made each create 0.7 ms longer).
+struct ExpTables {
+  int device = 0;
+  uint32_t users = 0;
+  uint4 *mem = nullptr;  // expf's table, then logf's
+};
+std::mutex g_tables_mu;
+std::vector<ExpTables> &exp_tables() {
+  static std::vector<ExpTables> *v = new std::vector<ExpTables>();  // (handles may outlive static objects)
+  return *v;
+}
+constexpr size_t kTabWords = fsd::kHashBytes / sizeof(uint4);
+
+int take_tables(fs_handle *h) {
+  std::lock_guard<std::mutex> lock(g_tables_mu);
+  ExpTables *t = nullptr;
+  for (ExpTables &x : exp_tables())
+    if (x.device == h->device) t = &x;
+  if (!t) {
+    std::vector<uint32_t> keys[2];
+    std::vector<float> vals[2];
+    const std::string dir = lib_dir();
+    if (!fsh::read_table(dir + "/expf_glibc.bin", keys[0], vals[0]) ||
+        !fsh::read_table(dir + "/logf_glibc.bin", keys[1], vals[1]))
+      return set_err(h, FS_ERR_IO, "missing " + dir + "/expf_glibc.bin or logf_glibc.bin (run the build)");
+    struct Buf {  // freed on every way out unless handed over
+      void *p = nullptr;
+      ~Buf() {
+        if (p) cudaFree(p);
+      }
+    } mem;
+    // (the sorted lists lie behind the tables: one allocation, 0.4 ms each)
+    CK(cudaMalloc(&mem.p, 2 * fsd::kHashBytes + 8 * (keys[0].size() + keys[1].size())));
+    for (int f = 0; f < 2; f++) {
+      const size_t n = keys[f].size();
+      uint32_t *dk = (uint32_t *)((uint4 *)mem.p + 2 * kTabWords) + (f ? 2 * keys[0].size() : 0);
+      float *dv = (float *)(dk + n);
+      CK(cudaMemcpyAsync(dk, keys[f].data(), n * 4, cudaMemcpyHostToDevice, h->st));
+      CK(cudaMemcpyAsync(dv, vals[f].data(), n * 4, cudaMemcpyHostToDevice, h->st));
+      CK(fsd::hash_fill(dk, dv, (uint32_t)n, (uint4 *)mem.p + f * kTabWords, h->st));
+    }
+    CK(cudaStreamSynchronize(h->st));
+    exp_tables().push_back(ExpTables{h->device, 0, (uint4 *)mem.p});
+    mem.p = nullptr;
+    t = &exp_tables().back();
+  }
+  t->users++;
+  h->tables = true;
+  h->cd.expf_tab = t->mem;
+  h->cd.logf_tab = t->mem + kTabWords;
+  return FS_OK;
+}
+void give_tables(fs_handle *h) {
+  if (!h->tables) return;
+  std::lock_guard<std::mutex> lock(g_tables_mu);
+  std::vector<ExpTables> &v = exp_tables();
+  for (size_t i = 0; i < v.size(); i++)
+    if (v[i].device == h->device && --v[i].users == 0) {
+      cudaFree(v[i].mem);
+      v.erase(v.begin() + (ptrdiff_t)i);
+      break;
+    }
+  h->tables = false;
 }
 
 // Ziggurat tables (Burkardt's r4_nor_setup, code/StiExt.h:321-351) and the
@@ -368,26 +436,7 @@ int create_compat(fs_handle *h, const fs_net_desc *d) {
     for (int k = 0; k < fsd::CS_N; k++) c.nst[k] = st[k] ? (uint32_t *)st[k] : c.nst[k - 1] + n;
   }
   if ((rc = zeros(h, &h->mt_state, 624)) || (rc = zeros(h, &h->mt_pos, 1))) return rc;
-  // exception tables
-  std::vector<uint32_t> ek, lk;
-  std::vector<float> ev, lv;
-  const std::string dir = lib_dir();
-  if (!fsh::read_table(dir + "/expf_glibc.bin", ek, ev) || !fsh::read_table(dir + "/logf_glibc.bin", lk, lv))
-    return set_err(h, FS_ERR_IO, "missing " + dir + "/expf_glibc.bin or logf_glibc.bin (run the build)");
-  {
-    uint32_t *dk = nullptr;
-    float *dv = nullptr;
-    for (int f = 0; f < 2; f++) {
-      const std::vector<uint32_t> &keys = f ? lk : ek;
-      const std::vector<float> &vals = f ? lv : ev;
-      uint4 *tab = nullptr;
-      if ((rc = upload(h, &dk, keys.data(), keys.size())) || (rc = upload(h, &dv, vals.data(), vals.size())) ||
-          (rc = dalloc(h, &tab, fsd::kHashBytes / sizeof(uint4))))
-        return rc;
-      CK(fsd::hash_fill(dk, dv, (uint32_t)keys.size(), tab, h->st));
-      (f ? c.logf_tab : c.expf_tab) = tab;
-    }
-  }
+  if ((rc = take_tables(h))) return rc;
   uint32_t kn[128], ja[32], jc[32];
   float fn[128], wn[128];
   host_tables(kn, fn, wn, ja, jc);
@@ -559,6 +608,7 @@ int fs_destroy(fs_handle *h) {
   if (h->st) cudaStreamSynchronize(h->st);
   if (h->prod) fsp::prod_destroy(h->prod);
   for (void *p : h->allocs) cudaFree(p);
+  give_tables(h);
   if (h->ev0) cudaEventDestroy(h->ev0);
   if (h->ev1) cudaEventDestroy(h->ev1);
   if (h->st) cudaStreamDestroy(h->st);
