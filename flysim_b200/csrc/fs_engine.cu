@@ -523,9 +523,13 @@ int compat_batch(fs_handle *h, uint32_t nsteps, fs_step_out *out, uint64_t *writ
   return FS_OK;
 }
 
-// steps per batch for compat: bounded by the spike buffers
-uint32_t compat_batch_steps(fs_handle *h, uint32_t left) {
-  const uint64_t lim = std::min<uint64_t>(h->chunk, std::max<uint64_t>(1, (64ull << 20) / std::max<uint32_t>(1, h->n)));
+// Steps per batch for compat: bounded by the spike buffers, and with per-step
+// outputs, which the device holds for the whole batch, to 64 M random draws (the
+// draws' own buffer was the bound while a batch's were made beforehand).
+uint32_t compat_batch_steps(fs_handle *h, const fs_step_out *out, uint32_t left) {
+  const bool outputs = out && (out->V || out->Irep || out->nstate || out->gv_n);
+  const uint64_t per = std::max<uint32_t>({1u, h->n, outputs ? h->cd.draws_per_step : 0u});
+  const uint64_t lim = std::min<uint64_t>(h->chunk, std::max<uint64_t>(1, (64ull << 20) / per));
   return (uint32_t)std::min<uint64_t>(lim, left);
 }
 
@@ -677,7 +681,7 @@ int fs_step(fs_handle *h, uint32_t nsteps, fs_step_out *out) {
   if (h->mode == FS_MODE_COMPAT) {
     uint32_t done = 0;
     while (done < nsteps) {
-      const uint32_t b = compat_batch_steps(h, nsteps - done);
+      const uint32_t b = compat_batch_steps(h, out, nsteps - done);
       rc = compat_batch(h, b, out, &written, done);
       if (rc) return rc;
       done += b;
@@ -707,7 +711,7 @@ int fs_run(fs_handle *h, uint32_t nsteps) {
     uint32_t done = 0;
     uint64_t written = 0;
     while (done < nsteps) {
-      const uint32_t b = compat_batch_steps(h, nsteps - done);
+      const uint32_t b = compat_batch_steps(h, nullptr, nsteps - done);
       rc = compat_batch(h, b, nullptr, &written, done);
       if (rc) return rc;
       done += b;
