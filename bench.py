@@ -45,6 +45,27 @@ METRIC = "simulated seconds per wall second (20k-neuron connectome network)"
 UNIT = "sim-s/wall-s"
 
 
+# Counters of the persistent kernels' phase clock, by kernel (a lap counts from
+# the start of its phase; the others add up to a step).
+PHASES = {
+    "single_step": {0: "list wait and lookups", 2: "deliveries+nmda sums", 3: "membranes and list",
+                    4: "presynaptic state and next drive", 5: "set-up",
+                    10: "sums: warp 0 deliveries issued (lap)", 11: "sums: warp 0 out of posts (lap)",
+                    13: "membranes and list: warp 0 stepped (lap)"},
+    "interval": {0: "nmda pull", 1: "drive draws", 9: "conductances", 2: "membranes and presynaptic state",
+                 3: "history and pushes", 4: "barrier"},
+    "ltp": {0: "nmda pull", 5: "pushes", 6: "barrier after pushes", 7: "ltp rules", 1: "drive draws",
+            2: "neuron steps", 4: "barrier after steps"},
+}
+
+
+def phase_line(eng, steps):
+    """Mean and largest SM cycles per timestep of each phase over the blocks."""
+    ph = eng.phase_times().astype(np.float64) / steps
+    return {nm: {"mean": round(float(ph[:, k].mean()), 1), "max": round(float(ph[:, k].max()), 1)}
+            for k, nm in PHASES.get(eng.layout()["kernel"], {}).items()}
+
+
 def _env_int(k, d):
     try:
         return int(os.environ.get(k, d))
@@ -338,13 +359,8 @@ def run_compat(args, rank):
             eng.run(args.profile_steps)
             eng.sync()
             line = {"profile_steps": args.profile_steps, "stats": eng.stats(), "layout": eng.layout()}
-            if args.phase_clock and eng.layout()["kernel"] == "ltp":
-                ph = eng.phase_times().astype(np.float64) / args.profile_steps
-                names = {0: "nmda pull", 1: "drive draws", 2: "neuron steps", 4: "barrier after steps",
-                         5: "pushes", 6: "barrier after pushes", 7: "ltp rules"}
-                line["cycles_per_timestep"] = {nm: {"mean": round(float(ph[:, k].mean()), 1),
-                                                    "max": round(float(ph[:, k].max()), 1)}
-                                               for k, nm in names.items()}
+            if args.phase_clock:
+                line["cycles_per_timestep"] = phase_line(eng, args.profile_steps)
             print(json.dumps(line))
             eng.close()
             m.close()
@@ -490,16 +506,7 @@ def main():
         eng.sync()
         line = {"profile_steps": args.profile_steps, "stats": eng.stats(), "layout": eng.layout()}
         if args.phase_clock:
-            ph = eng.phase_times().astype(np.float64) / args.profile_steps
-            names = (["list wait and lookups", "-", "deliveries+nmda sums", "membranes and list",
-                      "presynaptic state and next drive", "set-up", "-", "-", "-", "-",
-                      "sums: warp 0 deliveries issued (lap)", "sums: warp 0 out of posts (lap)", "-",
-                      "membranes and list: warp 0 stepped (lap)"]
-                     if eng.layout()["kernel"] == "single_step" else
-                     ["nmda pull", "drive draws", "neuron steps", "pushes", "barrier"])
-            line["cycles_per_timestep"] = {nm: {"mean": round(float(ph[:, k].mean()), 1),
-                                                "max": round(float(ph[:, k].max()), 1)}
-                                           for k, nm in enumerate(names) if nm != "-"}
+            line["cycles_per_timestep"] = phase_line(eng, args.profile_steps)
         print(json.dumps(line))
         return 0
 

@@ -737,7 +737,7 @@ struct MtBlock {
 // is kept by step parity, so the owners' next (A) does not disturb it and one
 // barrier a step suffices.  Records are read and written by their post's
 // block only.  A block
-// with one tile (up to ~37,000 neurons) keeps its neurons in shared memory for
+// with one tile (up to 28,352 neurons: 443 blocks of 64) keeps its neurons in shared memory for
 // the launch; with more it loads and stores them every step.
 //
 // A step moves every record once through L2 (17 B a linear, 25 B an NMDA
@@ -747,7 +747,7 @@ struct MtBlock {
 // of its own.
 // Measured: 20,000 neurons with 4.1 M records 106 -> 42 us a step, now bounded by
 // the random stream (160 blocks of 624 words a step, about 480 cycles each
-// next to three other blocks of its SM); the two-population network of 1,000
+// next to two other blocks of its SM); the two-population network of 1,000
 // neurons 30 -> 9.7 us, latencies one after the other (activation 5,700
 // cycles, barrier 3,500, terms 4,500, ordered sums 3,800).  Three blocks an SM:
 // four spill (64 registers), and the spills and the tile leave L1 too little.

@@ -202,7 +202,7 @@ __device__ __forceinline__ unsigned long long *ring_at(const Params &P, int ri, 
 
 // Loads of the NMDA s history may be served by L1 (ld.global.ca): a block
 // reads only slots written in earlier intervals, and every interval ends
-// with the grid barrier above, whose fences (release before the arrival,
+// with a grid barrier (grid_sync), whose fences (release before the arrival,
 // acquire after the wait, then bar.sync) order those writes before the
 // reads in the PTX memory model; the vector windows of one edge and the
 // edges of different posts that share a presynaptic neuron then hit L1.
@@ -1041,6 +1041,9 @@ __device__ __forceinline__ void gv_write(const Params &P, uint32_t p, uint32_t s
 template <class T, uint32_t KT>
 struct TileBufs {
   static constexpr uint32_t kT = KT;
+  // listed spikes of a batch: one of each neuron of the widest tile and some more
+  // (a second one in 16 steps of 0.1 ms needs a refractory period below 1.6 ms);
+  // past it a thread pushes its spike itself
   static constexpr uint32_t kCap = sizeof(T) == 4 ? 320 : 192;
   T gn[kLB][kT];
   T gapI[kT];
@@ -1484,9 +1487,8 @@ __device__ __forceinline__ void prod_blocks(const Params &P, uint32_t B0, uint32
 // with sixteen; 4.57 -> 3.96 us a step).  PU
 // NMDA edges in flight per lane: four when a block's posts fit one tile
 // (20k connectome: 4.05 us per timestep against 4.71 with eight), eight when
-// they span several (250k network: 43.3 against 46.3 us); ring slots two
-// steps ahead (4.60 us with one).  Batches of small networks run eight edges
-// and one step ahead (their kernel has fewer registers to spare).
+// they span several (250k network: 43.3 against 46.3 us); both by the kernel
+// before the batches' three passes.  kOne: networks of interval 1.
 template <class T, int PU, uint32_t KT, bool kOne = false>
 __global__ void __launch_bounds__(sizeof(T) == 4 ? kThreads : kThreads64, sizeof(T) == 4 ? 2 : 1)
     k_prod(const __grid_constant__ Params P) {
@@ -1739,7 +1741,11 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1) k_prod_ltp(c
 constexpr uint32_t kT1 = 512;   // threads of k_prod1 (= max posts per block)
 constexpr uint32_t kT1F = 512;  // list entries of a step's blocks
 constexpr uint32_t kSlots = 2;  // (three: a third more lines to poll; one: 64 % of the 20k connectome's steps overflow)
-constexpr uint32_t kInline = 8;  // spikes beyond a region that the thread of its entry reads itself
+// Spikes beyond a region that the thread of its entry reads itself, one L2 round
+// trip after the other while the others poll; more take the block's pass with its
+// four barriers.  (A block of 500 posts at 20 Hz has one spike a step; the line
+// between the two was not tuned.)
+constexpr uint32_t kInline = 8;
 
 // Tracked index of neuron id in a block (or -1): bit id of the block's
 // bitmap (words [w0, w0 + nwd) of the id space) says whether it is
@@ -1788,7 +1794,8 @@ __device__ __forceinline__ void st_entry(uint4 *p, uint32_t x, uint32_t y, uint3
                "l"((unsigned long long)x | (unsigned long long)y << 32),
                "l"((unsigned long long)z | (unsigned long long)w << 32) : "memory");
 }
-// Waits until entry e (W words) carries the tag; false: the wait's limit ran out or
+// Waits until entry e (W words) carries the tag; false: the wait's limit ran out
+// (2^22 polls of an L2 round trip, some seconds: the other block is gone) or
 // another block gave up.  b is the second word (W = 2).
 __device__ __forceinline__ bool await_entry(const uint4 *e, uint32_t W, uint32_t tag, uint4 &a, uint4 &b, int *err) {
   for (uint32_t spins = 0;;) {
@@ -3410,6 +3417,8 @@ static int prod_create_from(Prod **out, const fs_net_desc *d, const fs_run_opts 
   block_post[0] = 0;
   {
     // cost of a post: its NMDA in-edges (pull) plus a fixed update cost
+    // (24 edges' worth: measured with the kernel before the batches' three passes,
+    // not refitted since; results do not depend on the cut)
     const double upd = 24.0;
     const double total = (double)nnm_e + upd * n;
     double acc = 0;

@@ -323,14 +323,16 @@ int fs_debug_single_step_plan(const fs_net_desc *desc, uint32_t sm_count, uint64
  * the reference).  fs_debug_phase_clock(h, 1) zeroes and switches on
  * per-block counters of SM cycles per phase, 0 switches them off;
  * fs_debug_phase_times copies up to cap counters, [blocks][16], and the
- * block count.  Phases: single-step kernel 0 spike-list lookups, 1 NMDA
- * copies of listed spikes, 2 last deliveries and NMDA sums, 3 neuron steps,
- * 6 thread 0's wait at the grid barrier, 4 the rest of the barrier (the
- * other warps' drive draws and NMDA copies), 5 set-up, and laps inside a
- * phase (cycles from its start): 8 the list's entry count loaded, 9 the
- * look-ups done, 10 warp 0's deliveries issued, 11 warp 0 out of posts to
- * sum, 12 thread 0's list entries loaded, 13 warp 0's neuron steps done; interval kernel 0 NMDA pull, 1 drive draws, 2 neuron steps,
- * 3 pushes, 4 grid barrier.  The tile kernels have no phase clock. */
+ * block count.  Phases, as a block's thread 0 passes them.  Single-step kernel:
+ * 0 wait for the other blocks' lists and their look-ups, 2 deliveries and NMDA
+ * sums, 3 membranes and list entries, 4 presynaptic state and the next step's
+ * drive, 5 set-up, and laps (cycles from the start of their phase) 10 warp 0's
+ * deliveries issued, 11 warp 0 out of posts to sum, 13 warp 0's membranes done.
+ * Interval kernel: 0 NMDA pull, 1 drive draws, 9 conductances, 2 membranes and
+ * presynaptic state, 3 history and pushes, 4 grid barrier.  Long-term plasticity
+ * kernel: 0 NMDA pull, 5 pushes, 6 barrier after them, 7 rules, 1 drive draws, 2
+ * conductances and neurons, 4 barrier after them.  The tile and reference-order
+ * kernels have no phase clock. */
 int fs_debug_phase_clock(fs_handle *h, int enable);
 int fs_debug_phase_times(fs_handle *h, uint64_t *out, uint32_t cap, uint32_t *blocks);
 /* Failure detection on the host side: stores into the handle's device error
