@@ -1609,9 +1609,9 @@ int grad(Mlp *m, const float *x, const float *t, int rows, float *g, float *loss
 
 // Rows [r0, r0 + n) of a call through lane a (n <= kChunk); host copies into
 // and out of the pinned buffers by the calling thread.  ran: when its kernel
-// ran, in ms after Mlp::fwd0.
+// ran, in ms after the event `from` (null: from its own start on).
 cudaError_t forward_rows(Mlp *m, FwdLane &a, const float *x, float *y, uint64_t r0, int n,
-                         std::pair<float, float> &ran) {
+                         cudaEvent_t from, std::pair<float, float> &ran) {
   const int di = m->dims[0], no = m->dims[m->L];
   const size_t bx = (size_t)n * di * 4, by = (size_t)n * no * 4, oy = (bx + 255) / 256 * 256;
   std::memcpy(a.host, x + r0 * di, bx);
@@ -1631,9 +1631,15 @@ cudaError_t forward_rows(Mlp *m, FwdLane &a, const float *x, float *y, uint64_t 
   if (e == cudaSuccess) e = cudaStreamSynchronize(a.st);
   if (e != cudaSuccess) return e;
   std::memcpy(y + r0 * no, a.host + oy, by);
-  e = cudaEventElapsedTime(&ran.first, m->fwd0, a.e0);
-  if (e == cudaSuccess) e = cudaEventElapsedTime(&ran.second, m->fwd0, a.e1);
+  if (from) e = cudaEventElapsedTime(&ran.first, from, a.e0);
+  if (e == cudaSuccess) e = cudaEventElapsedTime(&ran.second, from ? from : a.e0, a.e1);
   return e;
+}
+
+double total(const std::vector<std::pair<float, float>> &v) {
+  double sum = 0.0;
+  for (const auto &p : v) sum += p.second;
+  return sum;
 }
 
 // Milliseconds that at least one of the intervals covers.
@@ -1658,7 +1664,9 @@ int forward(Mlp *m, const float *x, uint64_t rows, float *y, double *device_ms, 
   cudaError_t e = cudaFuncSetAttribute(k_forward<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem<16>);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_forward<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem<64>);
-  if (e == cudaSuccess) e = cudaEventRecord(m->fwd0, m->st);
+  // (one lane's kernels follow each other: no common start is needed, whose
+  // record and queries took 8 us of a call of 2,000 rows)
+  if (e == cudaSuccess && want > 1) e = cudaEventRecord(m->fwd0, m->st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(m->st);  // weights and parameters are in place
   if (e != cudaSuccess) {
     err = std::string("mlp forward: ") + cudaGetErrorString(e);
@@ -1681,7 +1689,8 @@ int forward(Mlp *m, const float *x, uint64_t rows, float *y, double *device_ms, 
   auto work = [&](size_t w) {
     cudaError_t r = cudaSetDevice(m->device);
     for (uint64_t c; r == cudaSuccess && (c = next.fetch_add(1)) < chunks;)
-      r = forward_rows(m, lane[w], x, y, c * kChunk, (int)std::min<uint64_t>(kChunk, rows - c * kChunk), ran[c]);
+      r = forward_rows(m, lane[w], x, y, c * kChunk, (int)std::min<uint64_t>(kChunk, rows - c * kChunk),
+                       want > 1 ? m->fwd0 : nullptr, ran[c]);
     res[w] = r;
   };
   if (lanes) {
@@ -1701,7 +1710,9 @@ int forward(Mlp *m, const float *x, uint64_t rows, float *y, double *device_ms, 
     err = std::string("mlp forward: ") + cudaGetErrorString(e);
     return e == cudaErrorMemoryAllocation ? FS_ERR_NOMEM : FS_ERR_CUDA;
   }
-  if (device_ms) *device_ms = covered(ran);  // (the lanes' kernels overlap and wait for each other)
+  // (the lanes' kernels overlap and wait for each other; want = 1: one chunk at most,
+  // or one host thread)
+  if (device_ms) *device_ms = want > 1 ? covered(ran) : total(ran);
   return check(m, err);
 }
 
