@@ -206,7 +206,10 @@ __global__ void __launch_bounds__(kThreads) k_gemm_tn(const __grid_constant__ Ge
         mma_bf16(tmem, ad, bd, id, sl > 0 ? 1u : 0u);
       }
     }
-    if (!loads_ok && g.err) atomicExch(g.err, 4);
+    if (!loads_ok) {
+      if (g.err) atomicExch(g.err, 4);
+      for (int c = 0; c < nch; c++) mbar_wait(smem_u32(mbar + 1 + c), 0);  // no copy outlives the CTA
+    }
   }
   if (tid == 0)
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
@@ -540,6 +543,12 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_
                "l"(src), "r"(bytes), "r"(bar)
                : "memory");
 }
+// Waits (bounded) for the ring's copies in flight, so that a CTA that leaves after
+// a wait gave up leaves none behind: slot, ph: the issuing thread's next slot and
+// its round's parity (a slot never filled passes at once).
+__device__ __forceinline__ void drain_ring(const uint64_t *full, int slots, uint32_t slot, uint32_t ph) {
+  for (uint32_t c = 0; c < (uint32_t)slots; c++) mbar_wait(smem_u32(full + c), c < slot ? ph : ph ^ 1u);
+}
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
@@ -591,6 +600,9 @@ __device__ __forceinline__ void train_rows(const TrainArgs &g, uint8_t *smem, Tr
       const float v = c < g.din ? __ldg(g.x + (size_t)B.src[s & 1][r] * g.din + c) : 0.0f;
       Hs[(c >> 3) * (kHsBox / 2) + r * 8 + (c & 7)] = __float2bfloat16_rn(v);
     }
+  };
+  auto leave = [&]() {
+    if (warp == 8 && lane == 0) drain_ring(B.full, kRing, slot, ph);
   };
   rows_of(0);
   __syncthreads();
@@ -778,10 +790,10 @@ __device__ __forceinline__ void train_rows(const TrainArgs &g, uint8_t *smem, Tr
       }
     }
     if (!ok) B.fail = 1;
-    if (!fsd::grid_sync(g.bar, g.err, gridDim.x, target)) return;  // activations and gradients are out
+    if (!fsd::grid_sync(g.bar, g.err, gridDim.x, target)) return leave();  // activations and gradients are out
     if (B.fail) {
       if (tid == 0) atomicExch(g.err, 6);
-      return;
+      return leave();
     }
     if (s + 1 < g.steps) {  // while the tiles update
       rows_of(s + 1);
@@ -909,7 +921,10 @@ __device__ __forceinline__ void train_tile(const TrainArgs &g, uint8_t *smem, Tr
         for (int k = 0; k < kC; k++) adam_update(w[k], m[k], v[k], __uint_as_float(a[k]), g.lr, c1, c2);
       publish();
     }
-    if (!ok) B.fail = 1;
+    if (!ok) {
+      B.fail = 1;
+      if (warp == 9) drain_ring(B.full, 4, 4, ph);  // (its copies in flight; the copying lane does not wait)
+    }
     if (!fsd::grid_sync(g.bar, g.err, gridDim.x, target)) return;
     if (B.fail) {
       if (tid == 0) atomicExch(g.err, 6);
@@ -1008,7 +1023,7 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_forward(const FwdLayer *gl, i
   bool ok = true;
   auto layer = [&](int l) { return l < kFwdCached ? sl[l] : gl[l]; };
   if (warp == 8) {
-    if (lane == 0)
+    if (lane == 0) {
       for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x)
         for (int l = 0; l < L && ok; l++) {
           const FwdLayer Y = layer(l);
@@ -1025,6 +1040,8 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_forward(const FwdLayer *gl, i
             if (++slot == kRing) slot = 0, ph ^= 1u;
           }
         }
+      drain_ring(B.full, kRing, slot, ph);
+    }
   } else if (warp == 9) {
     const uint64_t ra = sdesc(smem_u32(smem), 2048, 128);
     const uint64_t rx = sdesc(smem_u32(Xs), kBox, 128), rh = sdesc(smem_u32(Hs), kBox, 128);
