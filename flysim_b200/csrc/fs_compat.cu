@@ -13,7 +13,7 @@
 //                   memory, then added by one thread per (post, receptor) in the
 //                   reference's order; LTP (code/EqsGnl2.cpp:1005-1044) rewrites a
 //                   record's weight right after its term
-//     mt_block      the std::mt19937 output stream the reference draws from, on a
+//     MtBlock       the std::mt19937 output stream the reference draws from, on a
 //                   block of its own, one step ahead
 //   k_count / k_write   ordered spike-list compaction (ballot bitmaps, block prefix)
 #include <cstdint>
@@ -85,6 +85,18 @@ cudaError_t hash_fill(const uint32_t *keys, const float *vals, uint32_t n, uint4
     e = cudaGetLastError();
   }
   return e;
+}
+
+// A warp per post.
+__global__ void __launch_bounds__(256) k_fill_loc(const uint32_t *row, const uint8_t *in_tile, uint32_t n, uint8_t *loc) {
+  const uint32_t p = blockIdx.x * 8u + (threadIdx.x >> 5);
+  if (p >= n) return;
+  const uint8_t v = in_tile[p];
+  for (uint32_t e = row[p] + (threadIdx.x & 31u), e1 = row[p + 1]; e < e1; e += 32) loc[e] = v;
+}
+cudaError_t fill_loc(const uint32_t *row, const uint8_t *in_tile, uint32_t n, uint8_t *loc, cudaStream_t st) {
+  k_fill_loc<<<(n + 7) / 8, 256, 0, st>>>(row, in_tile, n, loc);
+  return cudaGetLastError();
 }
 
 // Every expf exception lies within 0.0017 float ulp of a rounding boundary

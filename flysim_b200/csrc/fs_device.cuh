@@ -114,6 +114,8 @@ cudaError_t spikes_compact(const uint32_t *bits, uint32_t nsteps, uint32_t words
 constexpr uint32_t kHashBits = 17, kHashEmpty = 0xffffffffu;
 constexpr size_t kHashBytes = (size_t)32 << kHashBits;
 cudaError_t hash_fill(const uint32_t *keys, const float *vals, uint32_t n, uint4 *tab, cudaStream_t st);
+// loc[e] = in_tile[p] for the records e of post p (row: records by post)
+cudaError_t fill_loc(const uint32_t *row, const uint8_t *in_tile, uint32_t n, uint8_t *loc, cudaStream_t st);
 // test hooks
 cudaError_t expf_ref_eval(const float *x, float *y, uint64_t k, const uint32_t *keys, const float *vals,
                           uint32_t nk, const uint4 *tab, cudaStream_t st);

@@ -296,18 +296,20 @@ int compat_tiles(fs_handle *h, const fs_net_desc *d) {
   if (rc) return rc;
   h->cblocks = std::min(res, T);
   // a record's post, counted from its tile's first
-  std::vector<uint8_t> in_tile(n), loc;
+  std::vector<uint8_t> in_tile(n);
   for (uint32_t t = 0; t < T; t++)
     for (uint32_t i = cut[t]; i < cut[t + 1]; i++) in_tile[i] = (uint8_t)(i - cut[t]);
+  // (one allocation: each takes 0.3 ms)
+  uint8_t *mem = nullptr;
+  if ((rc = dalloc(h, &mem, (size_t)n + h->cd.rec_off[FS_NREC]))) return rc;
+  CK(cudaMemcpyAsync(mem, in_tile.data(), n, cudaMemcpyHostToDevice, h->st));
   for (int r = 0; r < FS_NREC; r++) {
-    const fs_rec_layout &L = d->compat->rec[r];
     fsd::RecDev &R = h->cd.R[r];
     R.rloc = nullptr;
     if (!R.rrow) continue;
-    loc.assign(L.n_recs, 0);
-    for (uint32_t i = 0; i < n; i++)
-      std::fill(loc.begin() + L.rec_rowptr[i], loc.begin() + L.rec_rowptr[i + 1], in_tile[i]);
-    if ((rc = upload(h, (uint8_t **)&R.rloc, loc.data(), loc.size()))) return rc;
+    uint8_t *loc = mem + n + h->cd.rec_off[r];
+    CK(fsd::fill_loc(R.rrow, mem, n, loc, h->st));
+    R.rloc = loc;
   }
   CK(cudaStreamSynchronize(h->st));
   return FS_OK;
